@@ -444,8 +444,12 @@ void march_plasma(Ctx& c, double s0, double s1) {
         G3D_CUDA(cudaMemsetAsync(P.bcnt.p, 0, sizeof(int), c.stream));
         G3D_CUDA(cudaMemsetAsync(P.rhol.p, 0, P.rhol.n * sizeof(double), c.stream));
         // front: half-cell N-2 predicted with its value of level s0; the front slice solved with it
-        launch_slice_prologue(c, N - 1, N - 2, 0, 0);
-        launch_march_slice(c, D, N - 1);
+        if (fh) {
+            launch_slice_prologue(c, N - 1, N - 2, 0, 0);
+            launch_march_slice_fh(c, D, N - 1);
+        } else {
+            launch_front(c, D);
+        }
         real_fields_slice(c, N - 1, N - 2, true, rec_fld ? long(passes) * (N - 1) + passes - 1 : -1);
         if (rec && !rec_fld) launch_record_fields(c, N - 1, passes - 1);
 
@@ -462,11 +466,13 @@ void march_plasma(Ctx& c, double s0, double s1) {
         sa.ext = c.ext;
         const long nl = long(c.nx) + c.ny;
         for (int n = nhi; n >= c.a; --n) {
-            // sin, si0 <- pin; the prediction of half-cell n-1 from its level s0; the slice saved for the passes
-            // (for the half-cells below the first, fused into the correction of the half-cell above)
-            if (n == nhi) launch_slice_prologue(c, n, n >= 1 ? n - 1 : -1, 1, passes > 1 ? 1 : 0);
+            // free-hand y: sin, si0 <- pin; the prediction of half-cell n-1 from its level s0; the slice saved for the
+            // passes (for the half-cells below the first, fused into the correction of the half-cell above). Fourier y
+            // keeps jk the beam's until the half-cell is final (k_pass_cols) and needs neither.
+            if (fh && n == nhi) launch_slice_prologue(c, n, n >= 1 ? n - 1 : -1, 1, passes > 1 ? 1 : 0);
             const double wex = (n >= 1 && n + 1 <= N - 2 && have_dl)
                                    ? (cen[size_t(n)] - cen[size_t(n - 1)]) / (cen[size_t(n + 1)] - cen[size_t(n)]) : 0.0;
+            const double q = D * c.wlo_h[size_t(n + 1)];          // the correction's factor
             if (rec && !rec_x) launch_record_particles(c, n);
             for (int pass = 0; pass < passes; ++pass) {
                 if (fh) launch_pass_prologue(c, n, pass > 0 ? 1 : 0);
@@ -481,20 +487,20 @@ void march_plasma(Ctx& c, double s0, double s1) {
                 if (ionz && pass + 1 == passes) launch_born_append(c);
                 if (!fh) {                     // rows of the current's spectra; columns, march and field columns fused
                     launch_stream_spectra_rows(c);
-                    launch_pass_cols(c, D, n, extrap ? 1 : 0, wex, pass > 0 ? 1 : 0);
+                    launch_pass_cols(c, D, n, extrap ? 1 : 0, wex, q, pass + 1 == passes);
                     real_fields_slice(c, n, pass + 1 < passes ? n : n - 1, false, rec_fld ? long(passes) * n + pass : -1);
                     if (rec && !rec_fld) launch_record_fields(c, n, pass);
                 } else {
                     launch_stream_spectra(c);
                     launch_replace_pred(c, n, extrap ? 1 : 0, wex);
-                    launch_march_slice(c, D, n);
+                    launch_march_slice_fh(c, D, n);
                     real_fields_slice(c, n, pass + 1 < passes ? n : n - 1);
                 }
             }
             // half-cell n is final: correct R at slice n+1, keep the change and the current
-            const double q = D * c.wlo_h[size_t(n + 1)];
-            if (n - 1 >= c.a) launch_correct_prologue(c, n, q, n + 1 < c.b ? 1 : 0, n - 1 >= 1 ? n - 2 : -1, passes > 1 ? 1 : 0);
-            else launch_correct(c, n, q, n + 1 < c.b ? 1 : 0);
+            // (Fourier y: in the last pass's k_pass_cols)
+            if (fh && n - 1 >= c.a) launch_correct_prologue(c, n, q, n + 1 < c.b ? 1 : 0, n - 1 >= 1 ? n - 2 : -1, passes > 1 ? 1 : 0);
+            else if (fh) launch_correct(c, n, q, n + 1 < c.b ? 1 : 0);
             have_dl = true;
         }
         if (rec) launch_record_particles(c, -1);         // the states after the last half-cell
@@ -548,9 +554,9 @@ void march_plasma(Ctx& c, double s0, double s1) {
         keep.insert(keep.end(), add.begin(), add.end());
         set_particles(c, keep.data(), long(keep.size()));
     }
-    // the sponge damps R - R_b with the bound field of the beam list only: jkz -= js0z
-    if (c.mixed) launch_axpy_fc(c, c.mx.jkz.p, P.js0z.p, -1.0, size_t(c.ns + 1) * c.nkh);
-    else launch_axpy_c(c, c.jkz.p, P.js0z.p, -1.0, size_t(c.ns + 1) * c.nkh);
+    // the sponge damps R - R_b with the bound field of the beam list only: free-hand y, jkz -= js0z (on Fourier y the
+    // march leaves jkz the beam's)
+    if (!c.yf) launch_axpy_c(c, c.jkz.p, P.js0z.p, -1.0, size_t(c.ns + 1) * c.nkh);
 }
 
 // The beam particles that became slower than vz_min stream in the current march (collect_restreaming,

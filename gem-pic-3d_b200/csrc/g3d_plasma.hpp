@@ -227,12 +227,11 @@ void launch_stream_spectra(Ctx& c);
 // Fourier y: the rows of the streaming current's spectra, then the fused column work of a pass (the current's
 // y transforms and filters, the replace and march of slice n, the y transforms of slice n's fields into W)
 void launch_stream_spectra_rows(Ctx& c);
-void launch_pass_cols(Ctx& c, double D, int n, int extrap, double w, int restore);
-void launch_replace(Ctx& c, int m, cpx* old, const cpx* nw);
+void launch_front(Ctx& c, double D);
+void launch_pass_cols(Ctx& c, double D, int n, int extrap, double w, double q, bool last);
 void launch_replace_pred(Ctx& c, int n, int extrap, double w);
 void launch_correct(Ctx& c, int n, double q, int own);
 void launch_correct_prologue(Ctx& c, int n, double q, int own, int pred_m, int backup);
-void launch_march_slice(Ctx& c, double D, int n);
 void launch_born_append(Ctx& c);
 // number of particles with alive == state among n (n_dev: the count on the device instead, when not null)
 long count_state(Ctx& c, const int32_t* alive, long n, const long* n_dev, int state);

@@ -281,6 +281,7 @@ __global__ void __launch_bounds__(NY) k_adjp_pass_cols(Geo g, AdjPlasmaPtrs a, c
     cpx* tl[6];
 #pragma unroll
     for (int k = 0; k < 6; ++k) tl[k] = reinterpret_cast<cpx*>(smp) + k * Tile::size;
+    cpx* const stw = reinterpret_cast<cpx*>(smp) + 6 * Tile::size;
     const int kxi = blockIdx.x, j = threadIdx.x;
     const long i = long(j) * g.H + kxi;
     for (long e = long(blockIdx.x) * NY + j; e < nzero; e += long(gridDim.x) * NY) {
@@ -293,10 +294,11 @@ __global__ void __launch_bounds__(NY) k_adjp_pass_cols(Geo g, AdjPlasmaPtrs a, c
     const cpx* Win[6] = {W0, W1, W2, W3, W4, W5};
 #pragma unroll
     for (int k = 0; k < 6; ++k) tl[k][Tile::at(j, 0)] = Win[k][i];
+    stage_twiddles<NY>(stw, g.twy, j, NY);
     __syncthreads();
     {
         cpx* const ls_[2] = {tl[2 * grp], tl[2 * grp + 1]};
-        fft_lines_some<NY, 2>(ls_, RowAddr{0}, tt, g.twy, act);
+        fft_lines_slice<NY, 2>(ls_, RowAddr{0}, tt, stw, act);
     }
     __syncthreads();
     const cpx lsl[6] = {tl[0][Tile::at(j, 0)], tl[1][Tile::at(j, 0)], tl[4][Tile::at(j, 0)], tl[5][Tile::at(j, 0)],
@@ -313,7 +315,7 @@ __global__ void __launch_bounds__(NY) k_adjp_pass_cols(Geo g, AdjPlasmaPtrs a, c
     __syncthreads();
     {
         cpx* const ls_[1] = {tl[grp]};
-        fft_lines_some<NY, 1>(ls_, RowAddr{0}, tt, g.twy, act);
+        fft_lines_slice<NY, 1>(ls_, RowAddr{0}, tt, stw, act);
     }
     __syncthreads();
     T0[i] = conj(tl[0][Tile::at(j, 0)]);
@@ -324,7 +326,7 @@ template <int NY>
 static void adjp_pass_cols(Ctx& c, const AdjPlasmaPtrs& a, const AdjPlasmaWs& w, int n, double D, double q, int last, int first,
                            int multi, int extrap, double wex, double* zero_a, double* zero_b, bool keep0, double a2) {
     using Tile = ColTile<NY, 1>;
-    const size_t smem = 6 * Tile::size * sizeof(cpx);
+    const size_t smem = (6 * Tile::size + NY) * sizeof(cpx);
     smem_attr(reinterpret_cast<const void*>(k_adjp_pass_cols<NY>), smem);
     k_adjp_pass_cols<NY><<<unsigned(c.H), NY, smem, c.stream>>>(c.geo(), a, w.Wsc[0], w.Wsc[1], w.Wsc[2], w.Wsc[3], w.Wsc[4], w.Wsc[5],
                                                                w.Tsc[0], w.Tsc[1], w.Tsc[2], n, D, q, last, first, multi, extrap, wex,

@@ -69,19 +69,23 @@ __global__ void k_adj_seed(PartsDev P, long np, double W, double* __restrict__ l
 // rows: per row of slice l, Lambda_R = (lEx + lBy)/2 + i (lEy - lBx)/2, Lambda_L = (lEx - lBy)/2 + i (lEy + lBx)/2,
 // Lambda_E = lEz + i lBz; their forward transforms times 1/nk, folded onto the half rows of the two fields of
 // each pair: lA(k) = z(k) + conj z(nx-k), lB(k) = -i z(k) + i conj z(nx-k) (mirror terms for 0 < k < nx/2)
-template <int NX>
-__global__ void __launch_bounds__(ANT) k_adj_rf_rows(Geo g, const double* __restrict__ lF, cpx* __restrict__ W0, cpx* __restrict__ W1,
+// ONE: the launch for a single slice (the plasma march's transpose), one row per CTA and a thread per point, as the
+// forward's k_rf_row_slice (k_slice_rows.cuh)
+template <int NX, bool ONE>
+constexpr int adj_row_threads() { return ONE ? slice_row_threads<NX>() : ANT; }
+template <int NX, bool ONE = false>
+__global__ void __launch_bounds__(adj_row_threads<NX, ONE>()) k_adj_rf_rows(Geo g, const double* __restrict__ lF, cpx* __restrict__ W0, cpx* __restrict__ W1,
                                                     cpx* __restrict__ W2, cpx* __restrict__ W3, cpx* __restrict__ W4,
                                                     cpx* __restrict__ W5, long fpl) {
     using S = FftShape<NX>;
-    constexpr int LPC = ANT / S::T, RS = row_stride<NX>(), H = NX / 2 + 1;
+    constexpr int NTH = adj_row_threads<NX, ONE>(), LPC = ONE ? 1 : NTH / S::T, RS = row_stride<NX>(), H = NX / 2 + 1;
     extern __shared__ cpx sm[];
     cpx* a0 = sm;
     cpx* a1 = sm + LPC * RS;
     cpx* a2 = sm + 2 * LPC * RS;
     const int l = blockIdx.y, r0 = blockIdx.x * LPC, tid = threadIdx.x;
     const long fbase = long(l) * g.nk;
-    for (int e = tid; e < LPC * NX; e += ANT) {
+    for (int e = tid; e < LPC * NX; e += NTH) {
         const int rr = e / NX, p = e - rr * NX, row = r0 + rr;
         double f[6] = {0, 0, 0, 0, 0, 0};
         if (row < g.ny) {
@@ -93,15 +97,20 @@ __global__ void __launch_bounds__(ANT) k_adj_rf_rows(Geo g, const double* __rest
         a1[q] = C(0.5 * (f[0] - f[4]), 0.5 * (f[1] + f[3]));
         a2[q] = C(f[2], f[5]);
     }
+    if constexpr (ONE) stage_twiddles<NX>(sm + 3 * RS, g.twx, tid, NTH);
     __syncthreads();
     const int r = tid / S::T, t = tid - r * S::T;
-    {
+    if constexpr (ONE) {                               // the three lines side by side
+        cpx* const ls_[1] = {r < 3 ? sm + r * RS : sm};
+        fft_lines_slice<NX, 1>(ls_, RowAddr{0}, t, sm + 3 * RS, r < 3);
+        __syncthreads();
+    } else {
         decltype(a0) const ls_[3] = {a0, a1, a2};
         fft_lines<NX, 3>(ls_, RowAddr{r * RS}, t, g.twx);
     }
     const double s = 1.0 / double(g.nk);
     const long base = long(l) * g.nkh;
-    for (int e = tid; e < LPC * H; e += ANT) {
+    for (int e = tid; e < LPC * H; e += NTH) {
         const int rr = e / H, kx = e - rr * H, row = r0 + rr;
         if (row >= g.ny) continue;
         const bool mirror = kx > 0 && kx < NX / 2;
@@ -356,22 +365,22 @@ __global__ void __launch_bounds__(ACW * FftShape<NY>::T) k_adj_cur_cols(Geo g, c
 // rows: the transposed Hermitian split (lz(k) = (lTX + i lTY)/2, lz(nx-k) = (conj lTX + i conj lTY)/2; at
 // k = 0, nx/2: Re lTX + i Re lTY) and the unnormalised inverse transform along x: Re -> lv_x, Im -> lv_y; j_z
 // from lTZ (zero above nx/2), real part -> lv_z. Out: V [3][ns+1][ny][nx].
-template <int NX>
-__global__ void __launch_bounds__(ANT) k_adj_cur_rows(Geo g, const cpx* __restrict__ TX, const cpx* __restrict__ TY,
+template <int NX, bool ONE = false>
+__global__ void __launch_bounds__(adj_row_threads<NX, ONE>()) k_adj_cur_rows(Geo g, const cpx* __restrict__ TX, const cpx* __restrict__ TY,
                                                      const cpx* __restrict__ TZ, double* __restrict__ V, long vpl) {
     using S = FftShape<NX>;
-    constexpr int LPC = ANT / S::T, RS = row_stride<NX>(), H = NX / 2 + 1;
+    constexpr int NTH = adj_row_threads<NX, ONE>(), LPC = ONE ? 1 : NTH / S::T, RS = row_stride<NX>(), H = NX / 2 + 1;
     extern __shared__ cpx sm[];
     cpx* a0 = sm;
     cpx* a1 = sm + LPC * RS;
     const int tid = threadIdx.x, r0 = blockIdx.x * LPC, hk = blockIdx.y;
     const long base = long(hk) * g.nkh;
-    for (int e = tid; e < LPC * NX; e += ANT) {                 // zero the rows (the mirror halves are added)
+    for (int e = tid; e < LPC * NX; e += NTH) {                 // zero the rows (the mirror halves are added)
         const int rr = e / NX, p = e - rr * NX;
         a0[rr * RS + p + (p >> 3)] = C(0); a1[rr * RS + p + (p >> 3)] = C(0);
     }
     __syncthreads();
-    for (int e = tid; e < LPC * H; e += ANT) {
+    for (int e = tid; e < LPC * H; e += NTH) {
         const int rr = e / H, kx = e - rr * H, row = r0 + rr;
         if (row >= g.ny) continue;
         const long o = base + long(row) * H + kx;
@@ -386,14 +395,19 @@ __global__ void __launch_bounds__(ANT) k_adj_cur_rows(Geo g, const cpx* __restri
         a0[rr * RS + kx + (kx >> 3)] = conj(zk);
         a1[rr * RS + kx + (kx >> 3)] = conj(TZ[o]);
     }
+    if constexpr (ONE) stage_twiddles<NX>(sm + 2 * RS, g.twx, tid, NTH);
     __syncthreads();
     const int r = tid / S::T, t = tid - r * S::T;
-    {
+    if constexpr (ONE) {
+        cpx* const ls_[1] = {r < 2 ? sm + r * RS : sm};
+        fft_lines_slice<NX, 1>(ls_, RowAddr{0}, t, sm + 2 * RS, r < 2);
+        __syncthreads();
+    } else {
         decltype(a0) const ls_[2] = {a0, a1};
         fft_lines<NX, 2>(ls_, RowAddr{r * RS}, t, g.twx);
     }
     const long nk = g.nk;
-    for (int e = tid; e < LPC * NX; e += ANT) {
+    for (int e = tid; e < LPC * NX; e += NTH) {
         const int rr = e / NX, p = e - rr * NX, row = r0 + rr;
         if (row >= g.ny) continue;
         const cpx u = conj(a0[rr * RS + p + (p >> 3)]), w = conj(a1[rr * RS + p + (p >> 3)]);
@@ -949,11 +963,10 @@ void launch_adj_real_fields(Ctx& c, const double* lF, cpx* const* W, cpx* const*
 // fpl) assigned to the slice's spectrum adjoints lsl = {Rx, Ry, Ez, Bz, Lx, Ly} (one plane each); W: 6 planes of scratch
 template <int NX>
 static void adj_rf_rows_slice(Ctx& c, const double* lF, long fpl, cpx* const* W) {
-    constexpr int LPC = ANT / FftShape<NX>::T;
-    const size_t smem = size_t(3) * LPC * row_stride<NX>() * sizeof(cpx);
-    allow_smem(k_adj_rf_rows<NX>, smem);
-    k_adj_rf_rows<NX><<<dim3(unsigned((c.ny + LPC - 1) / LPC), 1u), ANT, smem, c.stream>>>(c.geo(), lF, W[0], W[1], W[2], W[3],
-                                                                                          W[4], W[5], fpl);
+    const size_t smem = (size_t(3) * row_stride<NX>() + NX) * sizeof(cpx);
+    auto kern = k_adj_rf_rows<NX, true>;
+    allow_smem(kern, smem);
+    kern<<<dim3(unsigned(c.ny), 1u), adj_row_threads<NX, true>(), smem, c.stream>>>(c.geo(), lF, W[0], W[1], W[2], W[3], W[4], W[5], fpl);
     c.check_launch("k_adj_rf_rows");
 }
 template <int NY>
@@ -982,10 +995,10 @@ static void adj_ss_cols(Ctx& c, cpx* const* ljsn, cpx* const* T, bool keep0, dou
 }
 template <int NX>
 static void adj_ss_rows(Ctx& c, cpx* const* T, double* lJ) {
-    constexpr int LPC = ANT / FftShape<NX>::T;
-    const size_t smem = size_t(2) * LPC * row_stride<NX>() * sizeof(cpx);
-    allow_smem(k_adj_cur_rows<NX>, smem);
-    k_adj_cur_rows<NX><<<dim3(unsigned((c.ny + LPC - 1) / LPC), 1u), ANT, smem, c.stream>>>(c.geo(), T[0], T[1], T[2], lJ, long(c.nk));
+    const size_t smem = (size_t(2) * row_stride<NX>() + NX) * sizeof(cpx);
+    auto kern = k_adj_cur_rows<NX, true>;
+    allow_smem(kern, smem);
+    kern<<<dim3(unsigned(c.ny), 1u), adj_row_threads<NX, true>(), smem, c.stream>>>(c.geo(), T[0], T[1], T[2], lJ, long(c.nk));
     c.check_launch("k_adj_cur_rows");
 }
 void launch_adj_rf_rows_slice(Ctx& c, const double* lF, long fpl, cpx* const* W) {

@@ -179,11 +179,23 @@ __device__ __forceinline__ void fft_lines(T* const* sm, const Addr& A, int t, co
     for (int s = 0; s < S::NR8; ++s) { fft_pass_multi<N, 8, NL>(sm, A, t, L, tw); L *= 8; }
 }
 
-// The same transform in a CTA that has more threads than it needs: only the threads with act (t < FftShape<N>::T
-// per line set) load, compute and store; every thread of the CTA takes part in the barriers. For kernels with one
-// thread per mode of a column around the transform.
+// The transforms of one slice of the plasma march, in kernels with one row or column per CTA and more threads than the
+// transform needs: only the threads with act (t < FftShape<N>::T per line set) load, compute and store. A line's threads
+// lie in one warp when T <= 32 (T is a power of two and the lines' threads are consecutive), so its passes meet at warp
+// barriers and the CTA's barriers stay outside; every thread of the CTA calls it all the same. The twiddles come from a
+// copy of the table in shared memory (stage_twiddles): such a kernel starts with a cold L1, and each pass would wait for
+// them from L2.
+template <int N>
+__device__ __forceinline__ void slice_sync() {
+    if constexpr (FftShape<N>::T <= 32) __syncwarp();
+    else __syncthreads();
+}
+template <int N, class T>
+__device__ __forceinline__ void stage_twiddles(T* sm, const T* __restrict__ tw, int tid, int nthr) {
+    for (int k = tid; k < N; k += nthr) sm[k] = __ldg(tw + k);
+}
 template <int N, int R, int NL, class Addr, class T>
-__device__ __forceinline__ void fft_pass_multi_some(T* const* sm, const Addr& A, int t, int L, const T* __restrict__ tw, bool act) {
+__device__ __forceinline__ void fft_pass_slice(T* const* sm, const Addr& A, int t, int L, const T* tw, bool act) {
     constexpr int E = FftShape<N>::E, TT = FftShape<N>::T, BPT = E / R;
     const int m = N / (L * R);
     T v[NL][E];
@@ -200,7 +212,7 @@ __device__ __forceinline__ void fft_pass_multi_some(T* const* sm, const Addr& A,
             if (L > 1) {
 #pragma unroll
                 for (int q = 1; q < R; ++q) {
-                    const T w = __ldg(&tw[q * k * m]);
+                    const T w = tw[q * k * m];
 #pragma unroll
                     for (int l = 0; l < NL; ++l) v[l][u * R + q] = v[l][u * R + q] * w;
                 }
@@ -209,7 +221,7 @@ __device__ __forceinline__ void fft_pass_multi_some(T* const* sm, const Addr& A,
             for (int l = 0; l < NL; ++l) dft<R>(&v[l][u * R]);
         }
     }
-    __syncthreads();
+    slice_sync<N>();
     if (act) {
 #pragma unroll
         for (int u = 0; u < BPT; ++u) {
@@ -222,19 +234,23 @@ __device__ __forceinline__ void fft_pass_multi_some(T* const* sm, const Addr& A,
             }
         }
     }
-    __syncthreads();
+    slice_sync<N>();
 }
 template <int N, int NL, class Addr, class T>
-__device__ __forceinline__ void fft_lines_some(T* const* sm, const Addr& A, int t, const T* __restrict__ tw, bool act) {
+__device__ __forceinline__ void fft_lines_slice(T* const* sm, const Addr& A, int t, const T* tw, bool act) {
     using S = FftShape<N>;
     int L = 1;
-    if constexpr (S::P3) { fft_pass_multi_some<N, 3, NL>(sm, A, t, L, tw, act); L *= 3; }
-    if constexpr (S::REM > 1) { fft_pass_multi_some<N, S::REM, NL>(sm, A, t, L, tw, act); L *= S::REM; }
+    if constexpr (S::P3) { fft_pass_slice<N, 3, NL>(sm, A, t, L, tw, act); L *= 3; }
+    if constexpr (S::REM > 1) { fft_pass_slice<N, S::REM, NL>(sm, A, t, L, tw, act); L *= S::REM; }
 #pragma unroll
-    for (int s = 0; s < S::NR4; ++s) { fft_pass_multi_some<N, 4, NL>(sm, A, t, L, tw, act); L *= 4; }
+    for (int s = 0; s < S::NR4; ++s) { fft_pass_slice<N, 4, NL>(sm, A, t, L, tw, act); L *= 4; }
 #pragma unroll
-    for (int s = 0; s < S::NR8; ++s) { fft_pass_multi_some<N, 8, NL>(sm, A, t, L, tw, act); L *= 8; }
+    for (int s = 0; s < S::NR8; ++s) { fft_pass_slice<N, 8, NL>(sm, A, t, L, tw, act); L *= 8; }
 }
+// Threads of a CTA that works on one row of N points of one slice: a thread per point, at least two warps (an N of 8 has
+// three lines of one thread each, the shortest the others, and the rest load and store), at most 256.
+template <int N>
+constexpr int slice_row_threads() { return N < 64 ? 64 : (N > 256 ? 256 : N); }
 
 // Shared-memory addressing of a row line: one padding slot per 8 values keeps the strided
 // Stockham accesses free of bank conflicts.

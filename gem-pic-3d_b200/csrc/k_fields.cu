@@ -18,6 +18,7 @@
 #include "k_fft.cuh"
 #include "k_dispatch.cuh"
 #include "k_tma.cuh"
+#include "k_slice_rows.cuh"
 
 namespace g3d {
 
@@ -385,38 +386,22 @@ __global__ void __launch_bounds__(8 * FftShape<NY>::T) k_rf_cols_tma(Geo g, cons
 }
 
 // ---------------------------------------------------------------- real fields: rows (inverse x, F)
-// XM (exact fields with midpoint fields, FP64 Fourier y): the midpoint fields from the FP64 values of both slices
-// (Fd), so that the streaming push of the exact forward gathers unrounded fields like the beam push does
-template <int NX, bool XM = false>
+// (one slice of the plasma march: k_rf_row_slice, k_slice_rows.cuh)
+template <int NX>
 __global__ void __launch_bounds__(NT) k_rf_rows(Geo g, const cpx* __restrict__ W0, const cpx* __restrict__ W1,
                                                const cpx* __restrict__ W2, const cpx* __restrict__ W3,
-                                               const cpx* __restrict__ W4, const cpx* __restrict__ W5, float* __restrict__ F, int l0,
-                                               double* __restrict__ Fd, FmidOut fm) {
+                                               const cpx* __restrict__ W4, const cpx* __restrict__ W5, float* __restrict__ F,
+                                               double* __restrict__ Fd) {
     using S = FftShape<NX>;
     constexpr int LPC = NT / S::T, RS = row_stride<NX>(), H = NX / 2 + 1;
     extern __shared__ cpx sm[];
     cpx* a0 = sm;
     cpx* a1 = sm + LPC * RS;
     cpx* a2 = sm + 2 * LPC * RS;
-    const int l = l0 + blockIdx.y, r0 = blockIdx.x * LPC, tid = threadIdx.x;
+    const int l = blockIdx.y, r0 = blockIdx.x * LPC, tid = threadIdx.x;
     const long base = long(l) * g.nkh;
     const long fpl = long(g.ns + 2) * g.nk, fbase = long(l) * g.nk;
     constexpr int EO = (LPC * NX + NT - 1) / NT;                    // output elements of a thread
-    float oth[XM ? 1 : EO][6];                                      // the midpoint fields' other slice
-    double othd[XM ? EO : 1][6];
-    if (fm.out) {
-    #pragma unroll
-        for (int u_ = 0; u_ < EO; ++u_) {
-            const int e = tid + u_ * NT, rr = e / NX, p = e - rr * NX, row = r0 + rr;
-            if (e >= LPC * NX || row >= g.ny) continue;
-            if constexpr (XM) {
-#pragma unroll
-                for (int comp = 0; comp < 6; ++comp) othd[u_][comp] = Fd[comp * fpl + long(fm.other) * g.nk + long(row) * NX + p];
-            } else {
-                fmid_load(fm, F, fpl, g.nk, long(row) * NX + p, oth[u_]);
-            }
-        }
-    }
     #pragma unroll
     for (int u_ = 0; u_ < (LPC * H + NT - 1) / NT; ++u_) {      // unrolled: the loads of all elements in flight
         const int e = tid + u_ * NT;
@@ -453,20 +438,6 @@ __global__ void __launch_bounds__(NT) k_rf_rows(Geo g, const cpx* __restrict__ W
                              float(0.5 * (l2 - r2)), float(0.5 * (r1 - l1)), float(z3.y)};  // B_x, B_y, B_z
 #pragma unroll
         for (int comp = 0; comp < 6; ++comp) F[comp * fpl + idx] = fv[comp];
-        if constexpr (XM) {
-            const double dv[6] = {0.5 * (r1 + l1), 0.5 * (r2 + l2), z3.x, 0.5 * (l2 - r2), 0.5 * (r1 - l1), z3.y};
-            if (fm.rec_f) {                            // the adjoint's record of the slice
-                double* R = *fm.rec_f + fm.rec_off + long(row) * NX + p;
-#pragma unroll
-                for (int comp = 0; comp < 6; ++comp) R[comp * g.nk] = dv[comp];
-            }
-            double2* o = reinterpret_cast<double2*>(fm.out) + 3 * (long(row) * NX + p);
-            o[0] = make_double2(0.5 * (dv[0] + othd[u_][0]), 0.5 * (dv[1] + othd[u_][1]));
-            o[1] = make_double2(0.5 * (dv[2] + othd[u_][2]), 0.5 * (dv[3] + othd[u_][3]));
-            o[2] = make_double2(0.5 * (dv[4] + othd[u_][4]), 0.5 * (dv[5] + othd[u_][5]));
-        } else if (fm.out) {
-            fmid_store(fm, long(row) * NX + p, fv, oth[u_]);
-        }
         if (Fd) {                                      // exact fields: the same values before the rounding
             Fd[0 * fpl + idx] = 0.5 * (r1 + l1); Fd[1 * fpl + idx] = 0.5 * (r2 + l2);
             Fd[3 * fpl + idx] = 0.5 * (l2 - r2); Fd[4 * fpl + idx] = 0.5 * (r1 - l1);
@@ -580,47 +551,39 @@ static void rf_cols(Ctx& c, int l0, int nl) {
     rf_cols_w<NY, CW>(c, l0, nl);
 }
 template <int NX>
-static void rf_rows(Ctx& c, int l0, int nl, FmidOut fm = FmidOut()) {
+static void rf_rows(Ctx& c, const cpx* W0, const cpx* W1, const cpx* W2, const cpx* W3, const cpx* W4, const cpx* W5) {
     constexpr int LPC = NT / FftShape<NX>::T;
     const size_t smem = size_t(3) * LPC * row_stride<NX>() * sizeof(cpx);
-    const int tok = c.prof_begin(nl == 1 ? "real_rows_slice" : "real_rows");
-    const dim3 grid(unsigned((c.ny + LPC - 1) / LPC), unsigned(nl));
-    if (c.Fd.p && fm.out && !fm.f32 && !fm.fh) {       // exact fields: unrounded midpoint fields
-        allow_smem(k_rf_rows<NX, true>, smem);
-        k_rf_rows<NX, true><<<grid, NT, smem, c.stream>>>(c.geo(), c.W[0].p, c.W[1].p, c.W[2].p, c.W[3].p, c.W[4].p, c.W[5].p, c.F.p,
-                                                          l0, c.Fd.p, fm);
-    } else {
-        allow_smem(k_rf_rows<NX>, smem);
-        k_rf_rows<NX><<<grid, NT, smem, c.stream>>>(c.geo(), c.W[0].p, c.W[1].p, c.W[2].p, c.W[3].p, c.W[4].p, c.W[5].p, c.F.p, l0,
-                                                    c.Fd.p, fm);
-    }
+    allow_smem(k_rf_rows<NX>, smem);
+    const int tok = c.prof_begin("real_rows");
+    k_rf_rows<NX><<<dim3(unsigned((c.ny + LPC - 1) / LPC), unsigned(c.ns)), NT, smem, c.stream>>>(c.geo(), W0, W1, W2, W3, W4, W5, c.F.p,
+                                                                                                  c.Fd.p);
     c.check_launch("k_rf_rows");
     c.prof_end(tok);
 }
 void launch_real_fields(Ctx& c) {
     G3D_DISPATCH_N(c.ny, NY, rf_cols<NY>(c, 0, c.ns));
-    G3D_DISPATCH_N(c.nx, NX, rf_rows<NX>(c, 0, c.ns));
+    G3D_DISPATCH_N(c.nx, NX, rf_rows<NX>(c, c.W[0].p, c.W[1].p, c.W[2].p, c.W[3].p, c.W[4].p, c.W[5].p));
 }
 // free-hand y: the spectra are already real in y; one inverse transform along x per row of R, L and E_z + i B_z
-template <int NX>
-static void rf_rows_direct(Ctx& c, int l0, int nl, FmidOut fm = FmidOut()) {
-    constexpr int LPC = NT / FftShape<NX>::T;
-    const size_t smem = size_t(3) * LPC * row_stride<NX>() * sizeof(cpx);
-    allow_smem(k_rf_rows<NX>, smem);
-    const int tok = c.prof_begin(nl == 1 ? "real_rows_slice" : "real_rows");
-    k_rf_rows<NX><<<dim3(unsigned((c.ny + LPC - 1) / LPC), unsigned(nl)), NT, smem, c.stream>>>(
-        c.geo(), c.Rx.p, c.Ry.p, c.Lx.p, c.Ly.p, c.Ez.p, c.Bz.p, c.F.p, l0, c.Fd.p, fm);
-    c.check_launch("k_rf_rows");
-    c.prof_end(tok);
+void launch_real_fields_fh(Ctx& c) {
+    G3D_DISPATCH_N(c.nx, NX, rf_rows<NX>(c, c.Rx.p, c.Ry.p, c.Lx.p, c.Ly.p, c.Ez.p, c.Bz.p));
 }
-void launch_real_fields_fh(Ctx& c) { G3D_DISPATCH_N(c.nx, NX, rf_rows_direct<NX>(c, 0, c.ns)); }
-void launch_real_fields_slice_fh(Ctx& c, int l, FmidOut fm) { G3D_DISPATCH_N(c.nx, NX, rf_rows_direct<NX>(c, l, 1, fm)); }
+void launch_real_fields_slice_fh(Ctx& c, int l, FmidOut fm) {
+    G3D_DISPATCH_N(c.nx, NX, (rf_row_slice<NX, cpx, false>(c, c.twx.p, c.Rx.p, c.Ry.p, c.Lx.p, c.Ly.p, c.Ez.p, c.Bz.p, l, l, c.Fd.p, fm)));
+}
 // the sponge's row pass alone (inverse x, mask, forward x) on W0, W1: the free-hand y sponge
 void launch_sp_rows(Ctx& c) { G3D_DISPATCH_N(c.nx, NX, sp_rows<NX>(c)); }
-// E and B of one slice (plane l) in real space (Simulation::real_fields_slice, src/sim_plasma.cpp:200-220)
+// E and B of one slice (plane l) in real space (Simulation::real_fields_slice, src/sim_plasma.cpp:200-220). cols: the
+// columns too (into plane l of W); else they are in plane 0 of W, where k_pass_cols left them
 void launch_real_fields_slice(Ctx& c, int l, FmidOut fm, bool cols) {
     if (cols) G3D_DISPATCH_N(c.ny, NY, rf_cols<NY>(c, l, 1));
-    G3D_DISPATCH_N(c.nx, NX, rf_rows<NX>(c, l, 1, fm));
+    const cpx* W[6] = {c.W[0].p, c.W[1].p, c.W[2].p, c.W[3].p, c.W[4].p, c.W[5].p};
+    const int lw = cols ? l : 0;
+    if (c.Fd.p && fm.out && !fm.f32 && !fm.fh)         // exact fields: unrounded midpoint fields
+        G3D_DISPATCH_N(c.nx, NX, (rf_row_slice<NX, cpx, true>(c, c.twx.p, W[0], W[1], W[2], W[3], W[4], W[5], l, lw, c.Fd.p, fm)))
+    else
+        G3D_DISPATCH_N(c.nx, NX, (rf_row_slice<NX, cpx, false>(c, c.twx.p, W[0], W[1], W[2], W[3], W[4], W[5], l, lw, c.Fd.p, fm)))
 }
 
 // ---------------------------------------------------------------- half <-> full spectrum layouts

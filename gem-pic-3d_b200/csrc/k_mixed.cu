@@ -13,6 +13,7 @@
 #include "g3d_ctx.hpp"
 #include "k_fft.cuh"
 #include "k_dispatch.cuh"
+#include "k_slice_rows.cuh"
 
 namespace g3d {
 
@@ -401,24 +402,16 @@ template <int NX>
 __global__ void __launch_bounds__(NT) k_rf_rows_f(Geo g, const cpxf* __restrict__ tw, const cpxf* __restrict__ W0,
                                                  const cpxf* __restrict__ W1, const cpxf* __restrict__ W2,
                                                  const cpxf* __restrict__ W3, const cpxf* __restrict__ W4,
-                                                 const cpxf* __restrict__ W5, float* __restrict__ F, int l0, FmidOut fm) {
+                                                 const cpxf* __restrict__ W5, float* __restrict__ F) {
     using S = FftShape<NX>;
     constexpr int LPC = NT / S::T, RS = row_stride<NX>(), H = NX / 2 + 1;
     extern __shared__ cpxf smf[];
     cpxf* a[3] = {smf, smf + LPC * RS, smf + 2 * LPC * RS};
-    const int l = l0 + blockIdx.y, r0 = blockIdx.x * LPC, tid = threadIdx.x;
+    const int l = blockIdx.y, r0 = blockIdx.x * LPC, tid = threadIdx.x;
     const long base = long(l) * g.nkh;
     const cpxf* in[6] = {W0, W1, W2, W3, W4, W5};
     const long fpl = long(g.ns + 2) * g.nk, fbase = long(l) * g.nk;
     constexpr int EO = (LPC * NX + NT - 1) / NT;                    // output elements of a thread
-    float oth[EO][6];                                               // the midpoint fields' other slice
-    if (fm.out) {
-    #pragma unroll
-        for (int u_ = 0; u_ < EO; ++u_) {
-            const int e = tid + u_ * NT, rr = e / NX, p = e - rr * NX, row = r0 + rr;
-            if (e < LPC * NX && row < g.ny) fmid_load(fm, F, fpl, g.nk, long(row) * NX + p, oth[u_]);
-        }
-    }
     #pragma unroll
     for (int u_ = 0; u_ < (LPC * H + NT - 1) / NT; ++u_) {
         const int e = tid + u_ * NT;
@@ -448,12 +441,6 @@ __global__ void __launch_bounds__(NT) k_rf_rows_f(Geo g, const cpxf* __restrict_
                              0.5f * (z2.y - z1.y), 0.5f * (z1.x - z2.x), z3.y};     // B_x, B_y, B_z
 #pragma unroll
         for (int comp = 0; comp < 6; ++comp) F[comp * fpl + idx] = fv[comp];
-        if (fm.out) fmid_store(fm, long(row) * NX + p, fv, oth[u_]);
-        if (fm.rec_f) {                                // the adjoint's record of the slice (widened)
-            double* R = *fm.rec_f + fm.rec_off + long(row) * NX + p;
-#pragma unroll
-            for (int comp = 0; comp < 6; ++comp) R[comp * g.nk] = double(fv[comp]);
-        }
     }
 }
 
@@ -483,10 +470,6 @@ __global__ void k_rotate_f(Geo g, cpxf* __restrict__ p, long n, double sx, doubl
         const double ph = g.kxs[i % g.H] * sx + (nys ? g.kys[i / g.H] * sy : 0.0);
         p[idx] = to_f(to_d(p[idx]) * C(cos(ph), sin(ph)));
     }
-}
-__global__ void k_axpy_fc(cpxf* __restrict__ y, const cpx* __restrict__ x, double a, long n) {
-    for (long i = long(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += long(gridDim.x) * blockDim.x)
-        y[i] = to_f(to_d(y[i]) + a * x[i]);
 }
 __global__ void k_copy_f(cpxf* __restrict__ y, const cpxf* __restrict__ x, long n) {
     for (long i = long(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += long(gridDim.x) * blockDim.x) y[i] = x[i];
@@ -598,25 +581,28 @@ static void rf_cols_f(Ctx& c, int l0, int nl) {
     else rf_cols_fw<NY, CW>(c, l0, nl);
 }
 template <int NX>
-static void rf_rows_f(Ctx& c, int l0, int nl, FmidOut fm = FmidOut()) {
+static void rf_rows_f(Ctx& c) {
     constexpr int LPC = NT / FftShape<NX>::T;
     const size_t smem = size_t(3) * LPC * row_stride<NX>() * sizeof(cpxf);
     allow_smem(k_rf_rows_f<NX>, smem);
-    const int tok = c.prof_begin(nl == 1 ? "real_rows_slice" : "real_rows");
+    const int tok = c.prof_begin("real_rows");
     auto& m = c.mx;
-    k_rf_rows_f<NX><<<dim3(unsigned((c.ny + LPC - 1) / LPC), unsigned(nl)), NT, smem, c.stream>>>(
-        c.geo(), m.twx.p, m.W[0].p, m.W[1].p, m.W[2].p, m.W[3].p, m.W[4].p, m.W[5].p, c.F.p, l0, fm);
+    k_rf_rows_f<NX><<<dim3(unsigned((c.ny + LPC - 1) / LPC), unsigned(c.ns)), NT, smem, c.stream>>>(
+        c.geo(), m.twx.p, m.W[0].p, m.W[1].p, m.W[2].p, m.W[3].p, m.W[4].p, m.W[5].p, c.F.p);
     c.check_launch("k_rf_rows_f");
     c.prof_end(tok);
 }
 void launch_real_fields_f(Ctx& c) {
     G3D_DISPATCH_N(c.ny, NY, rf_cols_f<NY>(c, 0, c.ns));
-    G3D_DISPATCH_N(c.nx, NX, rf_rows_f<NX>(c, 0, c.ns));
+    G3D_DISPATCH_N(c.nx, NX, rf_rows_f<NX>(c));
 }
-// E and B of one slice (plane l) of the mixed form (the real fields of one slice of the plasma march)
+// E and B of one slice (plane l) of the mixed form (the real fields of one slice of the plasma march); cols: the columns
+// too (into plane l of W); else they are in plane 0 of W, where k_pass_cols left them
 void launch_real_fields_slice_f(Ctx& c, int l, FmidOut fm, bool cols) {
     if (cols) G3D_DISPATCH_N(c.ny, NY, rf_cols_f<NY>(c, l, 1));
-    G3D_DISPATCH_N(c.nx, NX, rf_rows_f<NX>(c, l, 1, fm));
+    auto& m = c.mx;
+    G3D_DISPATCH_N(c.nx, NX, (rf_row_slice<NX, cpxf, false>(c, m.twx.p, m.W[0].p, m.W[1].p, m.W[2].p, m.W[3].p, m.W[4].p, m.W[5].p, l,
+                                                            cols ? l : 0, nullptr, fm)));
 }
 void launch_half_to_full_f(Ctx& c, const cpxf* half, cpx* full, long planes) {
     k_half_to_full_f<<<ew_blocks(planes * c.nk), 256, 0, c.stream>>>(c.geo(), half, full, planes);
@@ -630,11 +616,6 @@ void launch_rotate_f(Ctx& c, cpxf* p, size_t n, double sx, double sy, int nys) {
     if (!n) return;
     k_rotate_f<<<ew_blocks(long(n)), 256, 0, c.stream>>>(c.geo(), p, long(n), sx, sy, nys);
     c.check_launch("k_rotate_f");
-}
-void launch_axpy_fc(Ctx& c, cpxf* y, const cpx* x, double a, size_t n) {
-    if (!n) return;
-    k_axpy_fc<<<ew_blocks(long(n)), 256, 0, c.stream>>>(y, x, a, long(n));
-    c.check_launch("k_axpy_fc");
 }
 void launch_copy_f(Ctx& c, cpxf* y, const cpxf* x, size_t n) {
     if (!n) return;

@@ -7,19 +7,18 @@
 //                  Boris pushes (a third when the particle is trapped inside the half-cell), TSC deposit of its
 //                  current and charge into the real planes jsr (stream_deposit, :33-64), ADK ionization of the ions
 //                  with the counter-based random numbers (ionize, :80-101; ionization.hpp:25-46)
-//   k_ss_rows/cols the spectra of jsr: FFT of jx + i jy and jz of one plane, the k-filters, the smoothing
-//                  1 / (1 + a^2 k_perp^2) (stream_spectra, src/sim_plasma.cpp:94-157) -> jsn (half spectrum)
-//   k_replace_pred replace the streaming part of jk(n) by jsn and, with the extrapolating predictor, of jk(n-1) by
-//                  js0(n-1) + d + w (d - dl), d = jsn - js0(n) (sim_plasma.cpp:339-351)
-//   k_march_slice  the march of the modes of slice n (march_point, src/sim_kernels.hpp:173-210)
-//   real fields of slice n: the column and row kernels of k_fields.cu on one plane
-// On the Fourier y grid the column transform of the spectra, the replace and prediction, the slice march and the
-// column transforms of the real fields are one kernel per k_x column (k_pass_cols), between k_ss_rows and the
-// rows kernel of the real fields.
+//   k_ss_rows      the spectra of jsr along x: FFT of jx + i jy and jz of one plane (stream_spectra,
+//                  src/sim_plasma.cpp:94-157)
+//   k_pass_cols    Fourier y: per k_x column the rest of the spectra (FFT along y, the k-filters, the smoothing
+//                  1 / (1 + a^2 k_perp^2)), the prediction js0(n-1) + d + w (d - dl), d = js - js0(n), of half-cell n-1
+//                  (sim_plasma.cpp:339-351), the march of slice n (march_point, src/sim_kernels.hpp:173-210), the
+//                  transforms along y of its real fields and, in the last pass, the half-cell's correction (:381-403)
+//   k_rf_row_slice the real fields' transforms along x (k_slice_rows.cuh), with the midpoint fields of the next gather
+// On the free-hand y grid the parts of k_pass_cols are kernels of their own (k_ss_lines_fh, k_replace_pred, the line
+// march, k_correct).
 // A pass before the last (the predictor) deposits, transforms and marches like the last one but leaves the
 // particles unchanged (StreamArgs::dry), so every pass starts from the same particle state without a copy.
-// After the passes: k_correct (R of slice n+1 corrected for the prediction it used; dl, js0 updated,
-// sim_plasma.cpp:381-403) and k_born_append (the freed electrons join the march).
+// After the passes: k_born_append (the freed electrons join the march).
 #include <type_traits>
 #include <cub/device/device_scan.cuh>
 #include "g3d_plasma.hpp"
@@ -657,27 +656,30 @@ static void stream_launch(Ctx& c, const StreamArgs& a, unsigned blocks) {
 }
 
 // ---------------------------------------------------------------- spectra of the streaming current
-// rows: per row, FFT along x of jx + i jy (split) and of jz -> three half rows in T0..T2
+// rows: per row, FFT along x of jx + i jy (split) and of jz -> three half rows in T0..T2. One CTA per row, a thread per
+// point, the two lines side by side on threads of their own (k_slice_rows.cuh says why; four rows a CTA of 128 threads
+// before: per launch with the events' ~5 us 8.4 -> 6.4 us at 64 x 64 FP64, 8.5 -> 6.4 us at 32 x 32 mixed, 8.8 -> 8.5 us
+// at 256 x 256 mixed).
 template <int NX, class JT>
-__global__ void __launch_bounds__(128) k_ss_rows(Geo g, JT* __restrict__ J, cpx* __restrict__ T0, cpx* __restrict__ T1,
-                                                cpx* __restrict__ T2, int clear, int* __restrict__ bcnt) {
+__global__ void __launch_bounds__(slice_row_threads<NX>()) k_ss_rows(Geo g, JT* __restrict__ J, cpx* __restrict__ T0, cpx* __restrict__ T1,
+                                                                    cpx* __restrict__ T2, int clear, int* __restrict__ bcnt) {
     using S = FftShape<NX>;
-    constexpr int LPC = 128 / S::T, RS = row_stride<NX>(), H = NX / 2 + 1;
+    constexpr int NTH = slice_row_threads<NX>(), RS = row_stride<NX>(), H = NX / 2 + 1, EPT = (NX + NTH - 1) / NTH;
     extern __shared__ cpx sm[];
     cpx* a0 = sm;
-    cpx* a1 = sm + LPC * RS;
-    const int tid = threadIdx.x, r0 = blockIdx.x * LPC;
-    const long nk = g.nk;
+    cpx* a1 = sm + RS;
+    cpx* stw = sm + 2 * RS;
+    const int tid = threadIdx.x, row = blockIdx.x;
+    const long nk = g.nk, k0 = long(row) * NX;
     // every load first, then the clears for the next pass's deposit, then shared memory: a clear between two loads
     // would keep the second waiting for the first (the compiler cannot move a load above a store it may alias)
-    constexpr int EPT = LPC * NX / 128;
     double jx[EPT], jy[EPT], jz[EPT];
 #pragma unroll
     for (int u = 0; u < EPT; ++u) {
-        const int e = tid + u * 128, rr = e / NX, p = e - rr * NX, row = r0 + rr;
+        const int p = tid + u * NTH;
         jx[u] = jy[u] = jz[u] = 0;
-        if (row < g.ny) {
-            const long i = long(row) * NX + p;
+        if (p < NX) {
+            const long i = k0 + p;
             if constexpr (std::is_same<JT, float4>::value) {            // interleaved per point (FP32, Fourier y)
                 const float4 v = J[i];
                 jx[u] = v.x; jy[u] = v.y; jz[u] = v.z;
@@ -686,39 +688,40 @@ __global__ void __launch_bounds__(128) k_ss_rows(Geo g, JT* __restrict__ J, cpx*
             }
         }
     }
+    stage_twiddles<NX>(stw, g.twx, tid, NTH);
     if (clear) {
 #pragma unroll
         for (int u = 0; u < EPT; ++u) {
-            const int e = tid + u * 128, rr = e / NX, p = e - rr * NX, row = r0 + rr;
-            if (row >= g.ny) continue;
-            const long i = long(row) * NX + p;
+            const int p = tid + u * NTH;
+            if (p >= NX) continue;
+            const long i = k0 + p;
             if constexpr (std::is_same<JT, float4>::value) J[i] = make_float4(0.f, 0.f, 0.f, 0.f);
             else { J[i] = JT(0); J[nk + i] = JT(0); J[2 * nk + i] = JT(0); }
         }
     }
 #pragma unroll
     for (int u = 0; u < EPT; ++u) {
-        const int e = tid + u * 128, rr = e / NX, p = e - rr * NX;
-        a0[rr * RS + p + (p >> 3)] = C(jx[u], jy[u]);
-        a1[rr * RS + p + (p >> 3)] = C(jz[u], 0.0);
+        const int p = tid + u * NTH;
+        if (p >= NX) continue;
+        a0[p + (p >> 3)] = C(jx[u], jy[u]);
+        a1[p + (p >> 3)] = C(jz[u], 0.0);
     }
     if (bcnt && blockIdx.x == 0 && tid == 0) *bcnt = 0;          // the freed electrons of the next pass
     __syncthreads();
-    const int r = tid / S::T, t = tid - r * S::T;
     {
-        decltype(a0) const ls_[2] = {a0, a1};
-        fft_lines<NX, 2>(ls_, RowAddr{r * RS}, t, g.twx);
+        const int grp = tid / S::T;
+        cpx* const ls_[1] = {grp == 0 ? a0 : a1};
+        fft_lines_slice<NX, 1>(ls_, RowAddr{0}, tid % S::T, stw, grp < 2);
     }
-    for (int e = tid; e < LPC * H; e += 128) {
-        const int rr = e / H, kx = e - rr * H, row = r0 + rr;
-        if (row >= g.ny) continue;
+    __syncthreads();
+    for (int kx = tid; kx < H; kx += NTH) {
         const int km = (NX - kx) % NX;
-        const cpx z = a0[rr * RS + kx + (kx >> 3)], zm = conj(a0[rr * RS + km + (km >> 3)]);
+        const cpx z = a0[kx + (kx >> 3)], zm = conj(a0[km + (km >> 3)]);
         const cpx d = z - zm;
         const long o = long(row) * H + kx;
         T0[o] = 0.5 * (z + zm);
         T1[o] = 0.5 * C(d.y, -d.x);
-        T2[o] = a1[rr * RS + kx + (kx >> 3)];
+        T2[o] = a1[kx + (kx >> 3)];
     }
 }
 // columns: FFT along y, filters and smoothing -> jsn (3 half planes)
@@ -769,17 +772,6 @@ __global__ void __launch_bounds__(CW * FftShape<NY>::T) k_ss_cols(Geo g, const c
 }
 
 // ---------------------------------------------------------------- elementwise steps of the half-cell
-// jk(m) += nw - old; old <- nw (the `replace` of sim_plasma.cpp:257-264), three half planes
-template <class T>
-__global__ void k_replace(T* __restrict__ jx, T* __restrict__ jy, T* __restrict__ jz, cpx* __restrict__ old,
-                          const cpx* __restrict__ nw, long nkh) {
-    for (long i = long(blockIdx.x) * blockDim.x + threadIdx.x; i < nkh; i += long(gridDim.x) * blockDim.x) {
-        jx[i] = narrow<T>(widen(jx[i]) + nw[i] - old[i]);
-        jy[i] = narrow<T>(widen(jy[i]) + nw[nkh + i] - old[nkh + i]);
-        jz[i] = narrow<T>(widen(jz[i]) + nw[2 * nkh + i] - old[2 * nkh + i]);
-        old[i] = nw[i]; old[nkh + i] = nw[nkh + i]; old[2 * nkh + i] = nw[2 * nkh + i];
-    }
-}
 // after a pass: replace the streaming part of jk(n) by jsn (old = sin); with the extrapolating predictor and
 // n >= 1 the prediction of half-cell n-1: tmp = js0(n-1) + d + w (d - dl), d = jsn - js0(n); replace(n-1, pin, tmp)
 template <class T>
@@ -826,171 +818,183 @@ __global__ void k_correct(PlasmaPtrs p, cpx* __restrict__ Rx, cpx* __restrict__ 
     for (long i = long(blockIdx.x) * blockDim.x + threadIdx.x; i < p.nkh; i += long(gridDim.x) * blockDim.x)
         correct_mode(p, Rx, Ry, n, q, own, i);
 }
-// the march of slice n, one mode (march_point, sim_kernels.hpp:173-210, one rank: b = N, no boundary slice). The
-// current pointers carry no __restrict__: the fused kernel below writes jk just before.
-template <class T>
-__device__ __forceinline__ void march_slice_mode(const Geo& g, cpx* Rx, cpx* Ry, T* Ez, T* Bz, T* Lx, T* Ly, const T* j0x,
-                                                 const T* j0y, const T* jkx, const T* jky, const T* jkz, double D, int n, long i) {
-    const long nk = g.nkh;
-    const int kxi = int(i % g.H), j = int(i / g.H);
-    const double kx = g.kxd[kxi], ky = g.kyd[j], k2 = kx * kx + ky * ky, wl = g.wlo[n], wu = g.whi[n];
-    const long o = long(n - g.a) * nk + i, od = o, ou = o + nk;
-    const cpx Jx = wl * (widen(j0x[od]) + widen(jkx[od])) + wu * (widen(j0x[ou]) + widen(jkx[ou]));
-    const cpx Jy = wl * (widen(j0y[od]) + widen(jky[od])) + wu * (widen(j0y[ou]) + widen(jky[ou]));
-    const cpx ez = widen(Ez[o]), bz = widen(Bz[o]);
-    const cpx Rsx = Rx[o] + D * (ik(kx, ez) + ik(ky, bz)) - D * Jx;
-    const cpx Rsy = Ry[o] + D * (ik(ky, ez) - ik(kx, bz)) - D * Jy;
-    if (n == g.N - 1) {
-        Rx[o] = Rsx; Ry[o] = Rsy;
-        Ez[o] = narrow<T>(C(0)); Bz[o] = narrow<T>(C(0)); Lx[o] = narrow<T>(C(0)); Ly[o] = narrow<T>(C(0));
-        return;
-    }
-    const long pp = o + nk;
-    const cpx pRx = Rx[pp], pRy = Ry[pp], pEz = widen(Ez[pp]), pBz = widen(Bz[pp]), pLx = widen(Lx[pp]), pLy = widen(Ly[pp]);
-    const double h = g.hcg[n + 2];
-    const cpx upx = widen(jkx[ou]), upy = widen(jky[ou]), upz = widen(jkz[ou]);
-    const cpx Lsx = pLx - 0.25 * h * (ik(kx, pEz) - ik(ky, pBz)) - 0.5 * h * upx;
-    const cpx Lsy = pLy - 0.25 * h * (ik(kx, pBz) + ik(ky, pEz)) - 0.5 * h * upy;
-    const cpx Cp = 0.5 * (ik(kx, pRy + pLy) - ik(ky, pRx + pLx));
-    const cpx Qp = -0.5 * ik(kx, pRx - pLx) + 0.5 * ik(ky, pLy - pRy);
-    const cpx SB = ik(kx, Rsy) + ik(kx, Lsy) - ik(ky, Rsx) - ik(ky, Lsx);
-    const cpx SE = -ik(kx, Rsx) + ik(kx, Lsx) + ik(ky, Lsy) - ik(ky, Rsy);
-    const double den = 1 + 0.25 * h * (D + 0.25 * h) * k2;
-    const cpx Bzn = (pBz - 0.5 * h * Cp - 0.25 * h * SB) / den;
-    const cpx Ezn = (pEz - 0.5 * h * Qp - 0.25 * h * SE - h * upz) / den;
-    Ez[o] = narrow<T>(Ezn); Bz[o] = narrow<T>(Bzn);
-    Rx[o] = Rsx + D * (ik(kx, Ezn) + ik(ky, Bzn)); Ry[o] = Rsy + D * (ik(ky, Ezn) - ik(kx, Bzn));
-    Lx[o] = narrow<T>(Lsx - 0.25 * h * (ik(kx, Ezn) - ik(ky, Bzn)));
-    Ly[o] = narrow<T>(Lsy - 0.25 * h * (ik(kx, Bzn) + ik(ky, Ezn)));
-}
-template <class T>
-__global__ void __launch_bounds__(128) k_march_slice(Geo g, cpx* Rx, cpx* Ry, T* Ez, T* Bz, T* Lx, T* Ly, const T* j0x, const T* j0y,
-                                                    const T* jkx, const T* jky, const T* jkz, double D, int n) {
-    const long i = long(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < g.nkh) march_slice_mode<T>(g, Rx, Ry, Ez, Bz, Lx, Ly, j0x, j0y, jkx, jky, jkz, D, n, i);
-}
 // ---------------------------------------------------------------- one pass's column work, fused (Fourier y)
-// k_pass_cols: one CTA per k_x column, one thread per k_y (per mode). (1) Each thread loads what the march of its
-// mode reads (the loads of the replace and march below; they are in flight during the transform). (2) The y
-// transforms of the streaming current's three row spectra, the filters and the smoothing (k_ss_cols) -> jsn. (3)
-// Per mode the replace and the march of slice n (replace_pred_mode + march_slice_mode in one). (4) The inverse y transforms of slice n's new
-// R, L, E_z, B_z from shared memory (k_rf_cols, or k_rf_cols_f in FP32 for the mixed form) -> W, which the rows
-// kernel of the real fields takes. One launch and one pass over the spectra instead of three. The transforms
-// run on three groups of FftShape<NY>::T threads (a line or a line pair each); all threads take the barriers.
-template <int NY, class T, class WT>
+// The front slice N-1 of a step (half-cell N-2 predicted with its current of level s0, src/sim_plasma.cpp:236-262): its
+// march (L = E_z = B_z = 0) with the beam's jk plus that prediction, which is kept as the prediction slice N-1 was
+// solved with (pin; k_pass_cols' correction of half-cell N-2 reads it).
+template <class T>
+__global__ void k_front(PlasmaPtrs p, Geo g, cpx* __restrict__ Rx, cpx* __restrict__ Ry, T* __restrict__ Ez, T* __restrict__ Bz,
+                        T* __restrict__ Lx, T* __restrict__ Ly, const T* __restrict__ j0x, const T* __restrict__ j0y, double D) {
+    const long nk = g.nkh;
+    const int n = g.N - 1;
+    const T* jkx = static_cast<const T*>(p.jkx);
+    const T* jky = static_cast<const T*>(p.jky);
+    const double wl = g.wlo[n], wu = g.whi[n];
+    for (long i = long(blockIdx.x) * blockDim.x + threadIdx.x; i < nk; i += long(gridDim.x) * blockDim.x) {
+        const double kx = g.kxd[int(i % g.H)], ky = g.kyd[int(i / g.H)];
+        const long o = long(n - g.a) * nk + i, ou = o + nk;
+        const cpx tx = p.js0x[o], ty = p.js0y[o];                 // half-cell N-2 is plane N-1
+        const cpx ez = widen(Ez[o]), bz = widen(Bz[o]), rx = Rx[o], ry = Ry[o];
+        const cpx Jx = wl * (widen(j0x[o]) + (widen(jkx[o]) + tx)) + wu * (widen(j0x[ou]) + widen(jkx[ou]));
+        const cpx Jy = wl * (widen(j0y[o]) + (widen(jky[o]) + ty)) + wu * (widen(j0y[ou]) + widen(jky[ou]));
+        Rx[o] = rx + D * (ik(kx, ez) + ik(ky, bz)) - D * Jx;
+        Ry[o] = ry + D * (ik(ky, ez) - ik(kx, bz)) - D * Jy;
+        Ez[o] = narrow<T>(C(0)); Bz[o] = narrow<T>(C(0)); Lx[o] = narrow<T>(C(0)); Ly[o] = narrow<T>(C(0));
+        p.pin[i] = tx; p.pin[nk + i] = ty;
+    }
+}
+// k_pass_cols: one CTA per k_x column, one thread per k_y (per mode), all of a pass's work between the rows of the
+// current's spectra and the rows of the real fields:
+//   (1) every thread loads what its mode's march reads (in flight during the transform);
+//   (2) the y transforms of the streaming current's three row spectra, the filters and the smoothing -> u;
+//   (3) the march of slice n (march_point, src/sim_kernels.hpp:173-210) from its level-s0 values with the currents of half-cell n, the beam's plus
+//       u, and of half-cell n-1, the beam's plus the prediction t = js0(n-1) + d + w (d - dl), d = u - js0(n) (previous
+//       predictor: js0(n-1));
+//   (4) the inverse y transforms of the slice's new R, L, E_z, B_z from shared memory -> plane 0 of W, which the rows
+//       kernel of the real fields takes (one plane for every slice, so that it stays in L2).
+// jk holds the beam's current alone until half-cell n is final, so nothing has to be exchanged between passes: a pass
+// before the last (a predictor, LAST = 0) stores only W, and the slice's level-s0 values stay where they are for the next
+// pass. The last pass stores the slice and makes half-cell n final (src/sim_plasma.cpp:381-403): jkx, jky gain u (jkz
+// stays the beam's: that is what the sponge's bound field needs), R of slice n+1 is corrected for the prediction pin it
+// was solved with, the change from level s0 goes to dl and the current to js0(n), and t is the prediction that
+// slice n was solved with (pin).
+// Before, jk was rewritten on every pass with the replaced streaming part, the slice saved and restored between passes and
+// the half-cell's correction a kernel of its own: 46 values of a mode read and 36 written per two-pass half-cell beside
+// what is left now, and one launch more.
+// Bound by latency (one CTA of NY threads per SM): the loads of 34 values a thread, whose 16-byte (8-byte) accesses use
+// half (a quarter) of a 32-byte sector, then two transforms and the march one after the other. The transforms run on
+// FftShape<NY>::T threads a line, each line in one warp, with the twiddles in shared memory; the three current lines on
+// three of them, the six field lines on six (two lines each where a column has too few threads). Per launch with the
+// events' ~5 us: 256 x 256 mixed 19.5 -> 15.7 us, FP64 20.5 -> 15.6 us, 64 x 64 FP64 11.6 -> 8.4 us; the correction's
+// launch, 8.5 to 9.6 us per half-cell, is gone.
+template <int NY, class T, class WT, bool LAST>
 __global__ void __launch_bounds__(NY) k_pass_cols(PlasmaPtrs p, Geo g, const cpx* __restrict__ T0, const cpx* __restrict__ T1,
                                                   const cpx* __restrict__ T2, double a2, int keep0, cpx* __restrict__ Rx,
                                                   cpx* __restrict__ Ry, T* __restrict__ Ez, T* __restrict__ Bz, T* __restrict__ Lx,
                                                   T* __restrict__ Ly, const T* __restrict__ j0x, const T* __restrict__ j0y,
-                                                  double D, int n, int extrap, double w, const cpx* __restrict__ bk,
-                                                  const WT* __restrict__ twi, WT* __restrict__ W0, WT* __restrict__ W1,
-                                                  WT* __restrict__ W2, WT* __restrict__ W3, WT* __restrict__ W4, WT* __restrict__ W5) {
+                                                  double D, int n, int extrap, double w, double q, const WT* __restrict__ twi,
+                                                  WT* __restrict__ W0, WT* __restrict__ W1, WT* __restrict__ W2,
+                                                  WT* __restrict__ W3, WT* __restrict__ W4, WT* __restrict__ W5) {
     using S = FftShape<NY>;
     using Tile = ColTile<NY, 1>;
+    constexpr int NI = 6 * S::T <= NY ? 1 : 2;                        // field lines per thread group
     extern __shared__ double smp[];
-    cpx* fl[3] = {reinterpret_cast<cpx*>(smp), reinterpret_cast<cpx*>(smp) + Tile::size, reinterpret_cast<cpx*>(smp) + 2 * Tile::size};
-    WT* ib = reinterpret_cast<WT*>(reinterpret_cast<cpx*>(smp) + 3 * Tile::size);
+    cpx* const fl = reinterpret_cast<cpx*>(smp);                      // three current lines, then the twiddles
+    cpx* const ftw = fl + 3 * Tile::size;
+    WT* const ib = reinterpret_cast<WT*>(ftw + NY);                   // six field lines, then their twiddles
+    const WT* itw = ib + 6 * Tile::size;
+    if constexpr (std::is_same<WT, cpx>::value) itw = ftw;            // the same table
     const int kxi = blockIdx.x, j = threadIdx.x;
     const long nk = g.nkh, i = long(j) * g.H + kxi;
-    // the transforms: three groups of S::T threads, one line (forward) or one line pair (inverse) each
-    const int grp = j / S::T < 2 ? j / S::T : 2, tl = j - (j / S::T) * S::T;
-    const bool act = j < 3 * S::T;
-    // (1) the march's loads
+    const int grp = j / S::T, tl = j % S::T;
+    // (1) the loads, none of them converted yet: a conversion would wait for its load and hold back the ones behind it
+    const cpx c0 = T0[i], c1 = T1[i], c2 = T2[i];
     const long hp = long(n + 1) * nk + i, hq = long(n) * nk + i;      // half-cells n and n-1
-    T* jk[3] = {static_cast<T*>(p.jkx), static_cast<T*>(p.jky), static_cast<T*>(p.jkz)};
-    const bool pred = extrap && n >= 1;
-    cpx sn[3], kp[3], kq[3], s0p[3], s0q[3], dl[3], pn[3];
+    T* const jk[3] = {static_cast<T*>(p.jkx), static_cast<T*>(p.jky), static_cast<T*>(p.jkz)};
+    cpx* const s0[3] = {p.js0x, p.js0y, p.js0z};
+    const bool pred = n >= 1, ext = pred && extrap != 0;
+    T kp[3], kq[2];
+    cpx s0p[2], s0q[2], dl[2], pn[2];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        sn[k] = p.sin_[k * nk + i];
-        kp[k] = widen(jk[k][hp]); kq[k] = widen(jk[k][hq]);
-        if (pred) {
-            const cpx* s0[3] = {p.js0x, p.js0y, p.js0z};
-            s0p[k] = s0[k][hp]; s0q[k] = s0[k][hq]; dl[k] = p.dl[k * nk + i]; pn[k] = p.pin[k * nk + i];
-        }
+        kp[k] = jk[k][hp];
+        if (k == 2) continue;                                         // j_z of half-cell n-1 is not read by slice n
+        s0p[k] = LAST || ext ? s0[k][hp] : C(0);
+        kq[k] = jk[k][hq];
+        s0q[k] = pred ? s0[k][hq] : C(0);
+        dl[k] = ext && w != 0 ? p.dl[k * nk + i] : C(0);
+        pn[k] = LAST ? p.pin[k * nk + i] : C(0);
     }
-    const double kx = g.kxd[kxi], ky = g.kyd[j], k2 = kx * kx + ky * ky, wl = g.wlo[n], wu = g.whi[n];
-    const long o = long(n - g.a) * nk + i, ou = o + nk;
-    const cpx j0xd = widen(j0x[o]), j0xu = widen(j0x[ou]), j0yd = widen(j0y[o]), j0yu = widen(j0y[ou]);
-    const cpx rx = bk ? bk[i] : Rx[o], ry = bk ? bk[nk + i] : Ry[o];
-    const cpx ez = bk ? widen(narrow<T>(bk[2 * nk + i])) : widen(Ez[o]), bz = bk ? widen(narrow<T>(bk[3 * nk + i])) : widen(Bz[o]);
-    const bool front = n == g.N - 1;
-    cpx pRx = C(0), pRy = C(0), pEz = C(0), pBz = C(0), pLx = C(0), pLy = C(0);
-    if (!front) {
-        const long pp = o + nk;
-        pRx = Rx[pp]; pRy = Ry[pp]; pEz = widen(Ez[pp]); pBz = widen(Bz[pp]); pLx = widen(Lx[pp]); pLy = widen(Ly[pp]);
-    }
-    const double h = front ? 0.0 : g.hcg[n + 2];
+    const long o = long(n - g.a) * nk + i, ou = o + nk, pp = ou;
+    const T j0xd = j0x[o], j0xu = j0x[ou], j0yd = j0y[o], j0yu = j0y[ou];
+    const cpx rx = Rx[o], ry = Ry[o];
+    const T ez_ = Ez[o], bz_ = Bz[o];
+    const cpx pRx = Rx[pp], pRy = Ry[pp];
+    const T pEz_ = Ez[pp], pBz_ = Bz[pp], pLx_ = Lx[pp], pLy_ = Ly[pp];
+    const double kx = g.kxd[kxi], ky = g.kyd[j], kxs = g.kxs[kxi], kys = g.kys[j], fxy = g.filt[kxi] * g.filty[j];
+    const double wl = g.wlo[n], wu = g.whi[n], h = g.hcg[n + 2];
+    stage_twiddles<NY>(ftw, g.twy, j, NY);
+    if constexpr (!std::is_same<WT, cpx>::value) stage_twiddles<NY>(ib + 6 * Tile::size, twi, j, NY);
     // (2) the current's column, transformed and filtered
-    const long ot = long(j) * g.H + kxi;
-    fl[0][Tile::at(j, 0)] = T0[ot]; fl[1][Tile::at(j, 0)] = T1[ot]; fl[2][Tile::at(j, 0)] = T2[ot];
+    fl[Tile::at(j, 0)] = c0; fl[Tile::size + Tile::at(j, 0)] = c1; fl[2 * Tile::size + Tile::at(j, 0)] = c2;
+    const double k2 = kx * kx + ky * ky;
+    const double f = (kxi == 0 && j == 0 && !keep0) ? 0.0 : a2 == 0 ? fxy : fxy / (1 + a2 * (kxs * kxs + kys * kys));
+    const double rden = 1 / (1 + 0.25 * h * (D + 0.25 * h) * k2);
     __syncthreads();
     {
-        cpx* const ls_[1] = {fl[grp]};
-        fft_lines_some<NY, 1>(ls_, RowAddr{0}, tl, g.twy, act);
+        cpx* const ls_[1] = {fl + (grp < 3 ? grp : 0) * Tile::size};
+        fft_lines_slice<NY, 1>(ls_, RowAddr{0}, tl, ftw, grp < 3);
     }
-    const double k2f = g.kxs[kxi] * g.kxs[kxi] + g.kys[j] * g.kys[j];
-    const double f = (kxi == 0 && j == 0 && !keep0) ? 0.0 : g.filt[kxi] * g.filty[j] / (1 + a2 * k2f);
+    __syncthreads();
     cpx u[3];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) { u[k] = f * fl[k][Tile::at(j, 0)]; p.jsn[k * nk + i] = u[k]; }
-    // (3) replace(n, sin, jsn), the prediction of n-1, the march of slice n
+    for (int k = 0; k < 3; ++k) u[k] = f * fl[k * Tile::size + Tile::at(j, 0)];
+    // (3) the currents of half-cells n and n-1, the march of slice n
+    cpx cp[3], cq[2], t[2];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const T np_ = narrow<T>(kp[k] + u[k] - sn[k]);
-        jk[k][hp] = np_; kp[k] = widen(np_);
-        p.sin_[k * nk + i] = u[k];
-        if (pred) {
+    for (int k = 0; k < 3; ++k) cp[k] = widen(kp[k]) + u[k];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        t[k] = s0q[k];
+        if (ext) {
             const cpx d = u[k] - s0p[k];
-            const cpx t = s0q[k] + d + w * (d - dl[k]);
-            const T nq_ = narrow<T>(kq[k] + t - pn[k]);
-            jk[k][hq] = nq_; kq[k] = widen(nq_);
-            p.pin[k * nk + i] = t;
+            t[k] = t[k] + d;
+            if (w != 0) t[k] = t[k] + w * (d - dl[k]);
         }
+        cq[k] = widen(kq[k]) + t[k];
     }
-    const cpx Jx = wl * (j0xd + kq[0]) + wu * (j0xu + kp[0]);
-    const cpx Jy = wl * (j0yd + kq[1]) + wu * (j0yu + kp[1]);
+    const cpx ez = widen(ez_), bz = widen(bz_);
+    const cpx Jx = wl * (widen(j0xd) + cq[0]) + wu * (widen(j0xu) + cp[0]);
+    const cpx Jy = wl * (widen(j0yd) + cq[1]) + wu * (widen(j0yu) + cp[1]);
     const cpx Rsx = rx + D * (ik(kx, ez) + ik(ky, bz)) - D * Jx;
     const cpx Rsy = ry + D * (ik(ky, ez) - ik(kx, bz)) - D * Jy;
-    cpx nv[6];                                        // slice n as stored: R_x, R_y, L_x, L_y, E_z, B_z
-    if (front) {
-        Rx[o] = Rsx; Ry[o] = Rsy;
-        Ez[o] = narrow<T>(C(0)); Bz[o] = narrow<T>(C(0)); Lx[o] = narrow<T>(C(0)); Ly[o] = narrow<T>(C(0));
-        nv[0] = Rsx; nv[1] = Rsy;
-        nv[2] = nv[3] = nv[4] = nv[5] = widen(narrow<T>(C(0)));
-    } else {
-        const cpx upx = kp[0], upy = kp[1], upz = kp[2];
-        const cpx Lsx = pLx - 0.25 * h * (ik(kx, pEz) - ik(ky, pBz)) - 0.5 * h * upx;
-        const cpx Lsy = pLy - 0.25 * h * (ik(kx, pBz) + ik(ky, pEz)) - 0.5 * h * upy;
-        const cpx Cp = 0.5 * (ik(kx, pRy + pLy) - ik(ky, pRx + pLx));
-        const cpx Qp = -0.5 * ik(kx, pRx - pLx) + 0.5 * ik(ky, pLy - pRy);
-        const cpx SB = ik(kx, Rsy) + ik(kx, Lsy) - ik(ky, Rsx) - ik(ky, Lsx);
-        const cpx SE = -ik(kx, Rsx) + ik(kx, Lsx) + ik(ky, Lsy) - ik(ky, Rsy);
-        const double den = 1 + 0.25 * h * (D + 0.25 * h) * k2;
-        const cpx Bzn = (pBz - 0.5 * h * Cp - 0.25 * h * SB) / den;
-        const cpx Ezn = (pEz - 0.5 * h * Qp - 0.25 * h * SE - h * upz) / den;
-        const T ezs = narrow<T>(Ezn), bzs = narrow<T>(Bzn);
-        const cpx nRx = Rsx + D * (ik(kx, Ezn) + ik(ky, Bzn)), nRy = Rsy + D * (ik(ky, Ezn) - ik(kx, Bzn));
-        const T lxs = narrow<T>(Lsx - 0.25 * h * (ik(kx, Ezn) - ik(ky, Bzn)));
-        const T lys = narrow<T>(Lsy - 0.25 * h * (ik(kx, Bzn) + ik(ky, Ezn)));
-        Ez[o] = ezs; Bz[o] = bzs; Rx[o] = nRx; Ry[o] = nRy; Lx[o] = lxs; Ly[o] = lys;
-        nv[0] = nRx; nv[1] = nRy; nv[2] = widen(lxs); nv[3] = widen(lys); nv[4] = widen(ezs); nv[5] = widen(bzs);
-    }
+    const cpx pEz = widen(pEz_), pBz = widen(pBz_), pLx = widen(pLx_), pLy = widen(pLy_);
+    const cpx Lsx = pLx - 0.25 * h * (ik(kx, pEz) - ik(ky, pBz)) - 0.5 * h * cp[0];
+    const cpx Lsy = pLy - 0.25 * h * (ik(kx, pBz) + ik(ky, pEz)) - 0.5 * h * cp[1];
+    const cpx Cp = 0.5 * (ik(kx, pRy + pLy) - ik(ky, pRx + pLx));
+    const cpx Qp = -0.5 * ik(kx, pRx - pLx) + 0.5 * ik(ky, pLy - pRy);
+    const cpx SB = ik(kx, Rsy) + ik(kx, Lsy) - ik(ky, Rsx) - ik(ky, Lsx);
+    const cpx SE = -ik(kx, Rsx) + ik(kx, Lsx) + ik(ky, Lsy) - ik(ky, Rsy);
+    const cpx Bzn = rden * (pBz - 0.5 * h * Cp - 0.25 * h * SB);
+    const cpx Ezn = rden * (pEz - 0.5 * h * Qp - 0.25 * h * SE - h * cp[2]);
+    // slice n as stored: R_x, R_y, L_x, L_y, E_z, B_z
+    const cpx nRx = Rsx + D * (ik(kx, Ezn) + ik(ky, Bzn)), nRy = Rsy + D * (ik(ky, Ezn) - ik(kx, Bzn));
+    const T nLx = narrow<T>(Lsx - 0.25 * h * (ik(kx, Ezn) - ik(ky, Bzn))), nLy = narrow<T>(Lsy - 0.25 * h * (ik(kx, Bzn) + ik(ky, Ezn)));
+    const T nEz = narrow<T>(Ezn), nBz = narrow<T>(Bzn);
     // (4) the real fields' y transforms of slice n (pairs as k_rf_cols: R -> W0, W1; L -> W2, W3; E_z, B_z -> W4, W5)
+    {
+        const cpx nv[6] = {nRx, nRy, widen(nLx), widen(nLy), widen(nEz), widen(nBz)};
 #pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        if constexpr (std::is_same<WT, cpx>::value) ib[k * Tile::size + Tile::at(j, 0)] = conj(nv[k]);
-        else ib[k * Tile::size + Tile::at(j, 0)] = conj(to_f(nv[k]));
+        for (int k = 0; k < 6; ++k) {
+            if constexpr (std::is_same<WT, cpx>::value) ib[k * Tile::size + Tile::at(j, 0)] = conj(nv[k]);
+            else ib[k * Tile::size + Tile::at(j, 0)] = conj(to_f(nv[k]));
+        }
+    }
+    if constexpr (LAST) {
+        Rx[o] = nRx; Ry[o] = nRy; Ez[o] = nEz; Bz[o] = nBz; Lx[o] = nLx; Ly[o] = nLy;
+        Rx[pp] = pRx - q * (u[0] - pn[0]); Ry[pp] = pRy - q * (u[1] - pn[1]);
+        jk[0][hp] = narrow<T>(cp[0]); jk[1][hp] = narrow<T>(cp[1]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            if (k < 2) { p.dl[k * nk + i] = u[k] - s0p[k]; p.pin[k * nk + i] = t[k]; }
+            s0[k][hp] = u[k];
+        }
     }
     __syncthreads();
     {
-        WT* const ls_[2] = {ib + (2 * grp) * Tile::size, ib + (2 * grp + 1) * Tile::size};
-        fft_lines_some<NY, 2>(ls_, RowAddr{0}, tl, twi, act);
+        const int g6 = grp < 6 / NI ? grp : 0;
+        if constexpr (NI == 1) {
+            WT* const ls_[1] = {ib + g6 * Tile::size};
+            fft_lines_slice<NY, 1>(ls_, RowAddr{0}, tl, itw, grp < 6);
+        } else {
+            WT* const ls_[2] = {ib + (2 * g6) * Tile::size, ib + (2 * g6 + 1) * Tile::size};
+            fft_lines_slice<NY, 2>(ls_, RowAddr{0}, tl, itw, grp < 3);
+        }
     }
-    WT* out[6] = {W0, W1, W2, W3, W4, W5};
-    const long ow = long(n) * nk + long(j) * g.H + kxi;
+    __syncthreads();
+    WT* const out[6] = {W0, W1, W2, W3, W4, W5};
 #pragma unroll
-    for (int k = 0; k < 6; ++k) out[k][ow] = conj(ib[k * Tile::size + Tile::at(j, 0)]);
+    for (int k = 0; k < 6; ++k) out[k][i] = conj(ib[k * Tile::size + Tile::at(j, 0)]);
 }
 // freed electrons join the march (appended after the streaming particles; the count stays on the device)
 __global__ void k_born_append(const StrmDev* __restrict__ sd, const int* __restrict__ bcnt, int bcap, long* __restrict__ nstrm_dev,
@@ -1212,11 +1216,9 @@ void launch_stream(Ctx& c, const StreamArgs& a) {
 // Half spectra of three real planes J[0..2] (jx, jy, jz layout) into out[0..2]; T is scratch (3 half planes).
 template <int NX, class JT>
 static void ss_rows(Ctx& c, JT* J, cpx* T, int clear = 0, int* bcnt = nullptr) {
-    using S = FftShape<NX>;
-    constexpr int LPC = 128 / S::T;
-    const size_t smem = size_t(2) * LPC * row_stride<NX>() * sizeof(cpx);
+    const size_t smem = (size_t(2) * row_stride<NX>() + NX) * sizeof(cpx);
     smem_attr(reinterpret_cast<const void*>(k_ss_rows<NX, JT>), smem);
-    k_ss_rows<NX, JT><<<unsigned((c.ny + LPC - 1) / LPC), 128, smem, c.stream>>>(c.geo(), J, T, T + c.nkh, T + 2 * c.nkh, clear, bcnt);
+    k_ss_rows<NX, JT><<<unsigned(c.ny), slice_row_threads<NX>(), smem, c.stream>>>(c.geo(), J, T, T + c.nkh, T + 2 * c.nkh, clear, bcnt);
     c.check_launch("k_ss_rows");
 }
 template <int NY>
@@ -1454,11 +1456,7 @@ void launch_slice_prologue(Ctx& c, int n, int pred_m, int copy_in, int backup) {
     PlasmaState& P = *c.pl;
     const long o = long(n - c.a) * c.nkh;
     const int tok = c.prof_begin("slice_prologue");
-    if (c.mixed)
-        k_slice_prologue<cpxf><<<ew_blocks(c.nkh), 256, 0, c.stream>>>(P.ptrs(c), P.jsin.p, P.jsi0.p, P.bk.p, c.Rx.p, c.Ry.p,
-                                                                       c.mx.Ez.p, c.mx.Bz.p, o, pred_m, copy_in, backup);
-    else
-        k_slice_prologue<cpx><<<ew_blocks(c.nkh), 256, 0, c.stream>>>(P.ptrs(c), P.jsin.p, P.jsi0.p, P.bk.p, c.Rx.p, c.Ry.p,
+    k_slice_prologue<cpx><<<ew_blocks(c.nkh), 256, 0, c.stream>>>(P.ptrs(c), P.jsin.p, P.jsi0.p, P.bk.p, c.Rx.p, c.Ry.p,
                                                                       c.Ez.p, c.Bz.p, o, pred_m, copy_in, backup);
     c.check_launch("k_slice_prologue");
     c.prof_end(tok);
@@ -1467,10 +1465,7 @@ void launch_pass_prologue(Ctx& c, int n, int restore) {
     PlasmaState& P = *c.pl;
     const long o = long(n - c.a) * c.nkh, nj = 3 * long(c.nk);
     const int tok = c.prof_begin("pass_prologue");
-    if (c.mixed)
-        k_pass_prologue<cpxf, float><<<ew_blocks(nj), 256, 0, c.stream>>>(P.bk.p, c.Rx.p, c.Ry.p, c.mx.Ez.p, c.mx.Bz.p, o, c.nkh,
-                                                                          P.jsrf.p, nj, P.bcnt.p, restore);
-    else if (c.f32s)                  // free-hand y, mixed: FP64 spectra, FP32 streaming planes
+    if (c.f32s)                       // free-hand y, mixed: FP64 spectra, FP32 streaming planes
         k_pass_prologue<cpx, float><<<ew_blocks(nj), 256, 0, c.stream>>>(P.bk.p, c.Rx.p, c.Ry.p, c.Ez.p, c.Bz.p, o, c.nkh,
                                                                          P.jsrf.p, nj, P.bcnt.p, restore);
     else
@@ -1479,18 +1474,9 @@ void launch_pass_prologue(Ctx& c, int n, int restore) {
     c.check_launch("k_pass_prologue");
     c.prof_end(tok);
 }
-void launch_replace(Ctx& c, int m, cpx* old, const cpx* nw) {
-    const long h = long(m + 1) * c.nkh;
-    if (c.mixed)
-        k_replace<cpxf><<<ew_blocks(c.nkh), 256, 0, c.stream>>>(c.mx.jkx.p + h, c.mx.jky.p + h, c.mx.jkz.p + h, old, nw, c.nkh);
-    else
-        k_replace<cpx><<<ew_blocks(c.nkh), 256, 0, c.stream>>>(c.jkx.p + h, c.jky.p + h, c.jkz.p + h, old, nw, c.nkh);
-    c.check_launch("k_replace");
-}
 void launch_replace_pred(Ctx& c, int n, int extrap, double w) {
     const int tok = c.prof_begin("replace_pred");
-    if (c.mixed) k_replace_pred<cpxf><<<ew_blocks(c.nkh), 256, 0, c.stream>>>(c.pl->ptrs(c), n, extrap, w);
-    else k_replace_pred<cpx><<<ew_blocks(c.nkh), 256, 0, c.stream>>>(c.pl->ptrs(c), n, extrap, w);
+    k_replace_pred<cpx><<<ew_blocks(c.nkh), 256, 0, c.stream>>>(c.pl->ptrs(c), n, extrap, w);
     c.check_launch("k_replace_pred");
     c.prof_end(tok);
 }
@@ -1503,58 +1489,55 @@ void launch_correct_prologue(Ctx& c, int n, double q, int own, int pred_m, int b
     PlasmaState& P = *c.pl;
     const long o = long(n - 1 - c.a) * c.nkh;
     const int tok = c.prof_begin("correct_prologue");
-    if (c.mixed)
-        k_correct_prologue<cpxf><<<ew_blocks(c.nkh), 256, 0, c.stream>>>(P.ptrs(c), c.Rx.p, c.Ry.p, n, q, own, P.jsin.p, P.jsi0.p, P.bk.p,
-                                                                         c.mx.Ez.p, c.mx.Bz.p, o, pred_m, backup);
-    else
-        k_correct_prologue<cpx><<<ew_blocks(c.nkh), 256, 0, c.stream>>>(P.ptrs(c), c.Rx.p, c.Ry.p, n, q, own, P.jsin.p, P.jsi0.p, P.bk.p,
+    k_correct_prologue<cpx><<<ew_blocks(c.nkh), 256, 0, c.stream>>>(P.ptrs(c), c.Rx.p, c.Ry.p, n, q, own, P.jsin.p, P.jsi0.p, P.bk.p,
                                                                         c.Ez.p, c.Bz.p, o, pred_m, backup);
     c.check_launch("k_correct_prologue");
     c.prof_end(tok);
 }
-void launch_march_slice(Ctx& c, double D, int n) {
-    if (!c.yf) { launch_march_slice_fh(c, D, n); return; }
-    const int tok = c.prof_begin("march_slice");
-    const unsigned blocks = unsigned((c.nkh + 127) / 128);
-    if (c.mixed) {
-        MixedBufs& m = c.mx;
-        k_march_slice<cpxf><<<blocks, 128, 0, c.stream>>>(c.geo(), c.Rx.p, c.Ry.p, m.Ez.p, m.Bz.p, m.Lx.p, m.Ly.p, m.j0x.p, m.j0y.p,
-                                                          m.jkx.p, m.jky.p, m.jkz.p, D, n);
-    } else {
-        k_march_slice<cpx><<<blocks, 128, 0, c.stream>>>(c.geo(), c.Rx.p, c.Ry.p, c.Ez.p, c.Bz.p, c.Lx.p, c.Ly.p, c.j0x.p, c.j0y.p,
-                                                         c.jkx.p, c.jky.p, c.jkz.p, D, n);
-    }
-    c.check_launch("k_march_slice");
-    c.prof_end(tok);
+template <int NY, class T, class WT, bool LAST>
+static void pass_cols_form(Ctx& c, double D, int n, int extrap, double w, double q, T* Ez, T* Bz, T* Lx, T* Ly, const T* j0x, const T* j0y,
+                           const WT* tw, DevBuf<WT>* W) {
+    PlasmaState& P = *c.pl;
+    const double a2 = P.cfg.smooth_length * P.cfg.smooth_length;
+    const cpx* S = P.tsp.p;
+    const size_t smem = (3 * ColTile<NY, 1>::size + NY) * sizeof(cpx) +
+                        (6 * ColTile<NY, 1>::size + (std::is_same<WT, cpx>::value ? 0 : NY)) * sizeof(WT);
+    auto kern = k_pass_cols<NY, T, WT, LAST>;
+    smem_attr(reinterpret_cast<const void*>(kern), smem);
+    kern<<<unsigned(c.H), NY, smem, c.stream>>>(P.ptrs(c), c.geo(), S, S + c.nkh, S + 2 * c.nkh, a2, P.box_mean ? 1 : 0, c.Rx.p, c.Ry.p, Ez,
+                                                Bz, Lx, Ly, j0x, j0y, D, n, extrap, w, q, tw, W[0].p, W[1].p, W[2].p, W[3].p, W[4].p,
+                                                W[5].p);
 }
 template <int NY>
-static void pass_cols(Ctx& c, double D, int n, int extrap, double w, int restore) {
-    PlasmaState& P = *c.pl;
-    const PlasmaPtrs pp = P.ptrs(c);
-    const cpx* bk = restore ? P.bk.p : nullptr;
-    const double a2 = P.cfg.smooth_length * P.cfg.smooth_length;
-    const int keep0 = P.box_mean ? 1 : 0;
-    const cpx* T = P.tsp.p;
-    using Tile = ColTile<NY, 1>;
+static void pass_cols(Ctx& c, double D, int n, int extrap, double w, double q, bool last) {
     if (c.mixed) {
         MixedBufs& m = c.mx;
-        const size_t smem = 3 * Tile::size * sizeof(cpx) + 6 * Tile::size * sizeof(cpxf);
-        smem_attr(reinterpret_cast<const void*>(k_pass_cols<NY, cpxf, cpxf>), smem);
-        k_pass_cols<NY, cpxf, cpxf><<<unsigned(c.H), NY, smem, c.stream>>>(
-            pp, c.geo(), T, T + c.nkh, T + 2 * c.nkh, a2, keep0, c.Rx.p, c.Ry.p, m.Ez.p, m.Bz.p, m.Lx.p, m.Ly.p, m.j0x.p, m.j0y.p,
-            D, n, extrap, w, bk, m.twy.p, m.W[0].p, m.W[1].p, m.W[2].p, m.W[3].p, m.W[4].p, m.W[5].p);
+        auto f = last ? pass_cols_form<NY, cpxf, cpxf, true> : pass_cols_form<NY, cpxf, cpxf, false>;
+        f(c, D, n, extrap, w, q, m.Ez.p, m.Bz.p, m.Lx.p, m.Ly.p, m.j0x.p, m.j0y.p, m.twy.p, m.W);
     } else {
-        const size_t smem = 9 * Tile::size * sizeof(cpx);
-        smem_attr(reinterpret_cast<const void*>(k_pass_cols<NY, cpx, cpx>), smem);
-        k_pass_cols<NY, cpx, cpx><<<unsigned(c.H), NY, smem, c.stream>>>(
-            pp, c.geo(), T, T + c.nkh, T + 2 * c.nkh, a2, keep0, c.Rx.p, c.Ry.p, c.Ez.p, c.Bz.p, c.Lx.p, c.Ly.p, c.j0x.p, c.j0y.p,
-            D, n, extrap, w, bk, c.twy.p, c.W[0].p, c.W[1].p, c.W[2].p, c.W[3].p, c.W[4].p, c.W[5].p);
+        auto f = last ? pass_cols_form<NY, cpx, cpx, true> : pass_cols_form<NY, cpx, cpx, false>;
+        f(c, D, n, extrap, w, q, c.Ez.p, c.Bz.p, c.Lx.p, c.Ly.p, c.j0x.p, c.j0y.p, c.twy.p, c.W);
     }
 }
-void launch_pass_cols(Ctx& c, double D, int n, int extrap, double w, int restore) {
+// q: the correction's factor D wlo(n + 1) (the last pass)
+void launch_pass_cols(Ctx& c, double D, int n, int extrap, double w, double q, bool last) {
     const int tok = c.prof_begin("pass_cols");
-    G3D_DISPATCH_N(c.ny, NY, pass_cols<NY>(c, D, n, extrap, w, restore));
+    G3D_DISPATCH_N(c.ny, NY, pass_cols<NY>(c, D, n, extrap, w, q, last));
     c.check_launch("k_pass_cols");
+    c.prof_end(tok);
+}
+void launch_front(Ctx& c, double D) {
+    PlasmaState& P = *c.pl;
+    const int tok = c.prof_begin("front");
+    if (c.mixed) {
+        MixedBufs& m = c.mx;
+        k_front<cpxf><<<ew_blocks(c.nkh), 256, 0, c.stream>>>(P.ptrs(c), c.geo(), c.Rx.p, c.Ry.p, m.Ez.p, m.Bz.p, m.Lx.p, m.Ly.p, m.j0x.p,
+                                                              m.j0y.p, D);
+    } else {
+        k_front<cpx><<<ew_blocks(c.nkh), 256, 0, c.stream>>>(P.ptrs(c), c.geo(), c.Rx.p, c.Ry.p, c.Ez.p, c.Bz.p, c.Lx.p, c.Ly.p, c.j0x.p,
+                                                             c.j0y.p, D);
+    }
+    c.check_launch("k_front");
     c.prof_end(tok);
 }
 void launch_stream_spectra_rows(Ctx& c) {
