@@ -460,7 +460,7 @@ void march_plasma(Ctx& c, double s0, double s1) {
         sa.bcap = ionz ? int(P.born_cap) : 0; sa.dry = 0; sa.n = 0; sa.pass = 0;
         sa.ylo = c.yf ? -1e300 : c.ynode_h[1]; sa.yhi = c.yf ? 1e300 : c.ynode_h[size_t(c.ny) - 1];
         sa.Fmid = c.yf || c.f32s ? static_cast<const void*>(P.fmid.p) : nullptr;   // null if never allocated
-        sa.inv_dx = 1 / c.dx; sa.inv_dy = 1 / c.dy; sa.dep_norm = 0;
+        sa.inv_dx = 1 / c.dx; sa.inv_dy = 1 / c.dy; sa.ia0 = 1 / c.dy; sa.dep_norm = 0; sa.zn = sa.zn1 = 0;
         sa.Fd = c.mixed ? nullptr : c.Fd.p;
         sa.recd = rec_x ? P.recd.p : nullptr;
         sa.ext = c.ext;
@@ -476,7 +476,7 @@ void march_plasma(Ctx& c, double s0, double s1) {
             if (rec && !rec_x) launch_record_particles(c, n);
             for (int pass = 0; pass < passes; ++pass) {
                 if (fh) launch_pass_prologue(c, n, pass > 0 ? 1 : 0);
-                sa.n = n;
+                sa.n = n; sa.zn = c.zeta[size_t(n)]; sa.zn1 = c.zeta[size_t(n) + 1];
                 sa.dep_norm = 1 / (Delta * (c.zeta[size_t(n) + 1] - c.zeta[size_t(n)]) * c.dx);
                 sa.pass = pass;
                 sa.dry = pass + 1 < passes ? 1 : 0;

@@ -51,8 +51,10 @@ struct StreamArgs {
     const void* Fmid;          // Fourier y: the six fields half-way between slices n and n+1, interleaved per point
                                // (FP32: 8 floats, FP64: 6 doubles per point), or null
     ExtDev ext;                // external magnetic elements (none: nu = nm = 0)
-    double inv_dx, inv_dy;     // 1/dx, 1/dy (the mixed form's FP32 gathers and deposit)
-    double dep_norm;           // 1 / (Delta h_n dx): the deposit factor of half-cell n per unit of q w dt (the mixed form's FP32 deposit)
+    double zn, zn1;            // the slices n and n + 1
+    double inv_dx, inv_dy;     // 1/dx, 1/dy
+    double ia0;                // 1/A of the Fourier y grid's nodes
+    double dep_norm;           // 1 / (Delta h_n dx): the deposit factor of half-cell n per unit of q w dt
     const double* Fd;          // exact fields (FP64 form, Fourier y, no ionization, no analytic wave): the F planes in FP64 for
                                // the gather of a particle that starts inside the half-cell (null: the float planes F)
     const struct RecDev* recd; // the same variant, recording for the adjoint: the state of every particle entering half-cell n

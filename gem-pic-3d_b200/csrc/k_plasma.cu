@@ -34,11 +34,11 @@ template <class A>
 __device__ __forceinline__ void boris(A& ux, A& uy, A& uz, const A E[3], const A B[3], A qm, A dt) {
     const A qh = A(0.5) * qm * dt;
     const A umx = ux + qh * E[0], umy = uy + qh * E[1], umz = uz + qh * E[2];
-    const A qg = qh / sqrt(A(1) + umx * umx + umy * umy + umz * umz);     // q dt / (2 m gamma-)
+    const A qg = qh * rsqrt(A(1) + umx * umx + umy * umy + umz * umz);    // q dt / (2 m gamma-)
     const A tx = qg * B[0], ty = qg * B[1], tz = qg * B[2];
     const A t2 = tx * tx + ty * ty + tz * tz;
     const A upx = umx + (umy * tz - umz * ty), upy = umy + (umz * tx - umx * tz), upz = umz + (umx * ty - umy * tx);
-    const A sf = A(2) / (A(1) + t2);
+    const A sf = A(2) * (A(1) / (A(1) + t2));
     const A vx = umx + sf * (upy * tz - upz * ty), vy = umy + sf * (upz * tx - upx * tz), vz = umz + sf * (upx * ty - upy * tx);
     ux = vx + qh * E[0]; uy = vy + qh * E[1]; uz = vz + qh * E[2];
 }
@@ -132,67 +132,52 @@ __device__ __forceinline__ void sgather_exact(const StreamArgs& c, double x, dou
         if (comp < 3) E[comp] = v; else B[comp - 3] = v;
     }
 }
+// The streaming push's TSC on a periodic grid: the cell coordinate t = x / d and the nearest node in FP64 (x spans the
+// box, so the index needs the double), the offset from that node and the three weights in W (FP32 in the mixed form).
+// x may lie outside the box: the first index is wrapped (its two neighbours by a compare), and as a particle is rarely
+// more than a cell outside, the remainder (some twenty instructions) is behind a branch.
+template <class W>
+__device__ __forceinline__ void tsc_stream(double x, double inv_d, int n, int idx[3], W w[3]) {
+    const double t = x * inv_d;
+    const double c = floor(t + 0.5);
+    const W f = W(t - c);
+    w[0] = W(0.5) * (W(0.5) - f) * (W(0.5) - f);
+    w[1] = W(0.75) - f * f;
+    w[2] = W(0.5) * (W(0.5) + f) * (W(0.5) + f);
+    int b = int(c) - 1;
+    if (unsigned(b) >= unsigned(n)) { b %= n; if (b < 0) b += n; }
+    const int b1 = b + 1 == n ? 0 : b + 1;
+    idx[0] = b; idx[1] = b1; idx[2] = b1 + 1 == n ? 0 : b1 + 1;
+}
 // The gather half-way through the half-cell (zeta = the slice midpoint, a particle crossing the whole half-cell):
-// TSC in x and y of the interleaved midpoint fields, one vector load per point (Fourier y).
+// TSC in x and y of the interleaved midpoint fields, two (FP32) or three (FP64) vector loads per point (Fourier y).
 template <bool F32>
 __device__ __forceinline__ void sgather_mid(const StreamArgs& c, double x, double y, double E[3], double B[3]) {
-    const Geo& g = c.g;
-    int ix[3], jn[3]; double wx[3], wn[3];
-    tsc_periodic(x, g.dx, g.nx, ix, wx);
-    tsc_periodic(y, g.dy, g.ny, jn, wn);
     typedef typename std::conditional<F32, float, double>::type R;
+    int ix[3], jn[3]; R wx[3], wn[3];
+    tsc_stream<R>(x, c.inv_dx, c.g.nx, ix, wx);
+    tsc_stream<R>(y, c.inv_dy, c.g.ny, jn, wn);
     R a[6] = {0, 0, 0, 0, 0, 0};
 #pragma unroll
-    for (int j = 0; j < 3; ++j)
+    for (int j = 0; j < 3; ++j) {
+        const int k0 = jn[j] * c.g.nx;
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            const long k = long(jn[j]) * g.nx + ix[i];
-            const R w = R(wx[i] * wn[j]);
+            const int k = k0 + ix[i];
+            const R w = wx[i] * wn[j];
             if constexpr (F32) {
-                const float4* p = reinterpret_cast<const float4*>(c.Fmid) + 2 * k;
+                const float4* p = static_cast<const float4*>(c.Fmid) + 2 * k;
                 const float4 u = __ldg(p), v = __ldg(p + 1);
                 a[0] += w * u.x; a[1] += w * u.y; a[2] += w * u.z; a[3] += w * u.w; a[4] += w * v.x; a[5] += w * v.y;
             } else {
-                const double2* p = reinterpret_cast<const double2*>(c.Fmid) + 3 * k;
+                const double2* p = static_cast<const double2*>(c.Fmid) + 3 * k;
                 const double2 u = __ldg(p), v = __ldg(p + 1), q = __ldg(p + 2);
                 a[0] += w * u.x; a[1] += w * u.y; a[2] += w * v.x; a[3] += w * v.y; a[4] += w * q.x; a[5] += w * q.y;
             }
         }
+    }
     E[0] = double(a[0]); E[1] = double(a[1]); E[2] = double(a[2]);
     B[0] = double(a[3]); B[1] = double(a[4]); B[2] = double(a[5]);
-}
-// The mixed form's TSC on a periodic grid: the cell coordinate t = x / d and the nearest node in FP64 (x spans the
-// box, so the index needs the double), the offset from that node in FP32, the three weights in FP32.
-__device__ __forceinline__ void tsc_f32(double x, double inv_d, int n, int idx[3], float w[3]) {
-    const double t = x * inv_d;
-    const double c = floor(t + 0.5);
-    const float f = float(t - c);
-    w[0] = 0.5f * (0.5f - f) * (0.5f - f);
-    w[1] = 0.75f - f * f;
-    w[2] = 0.5f * (0.5f + f) * (0.5f + f);
-    int b = (int(c) - 1) % n;
-    if (b < 0) b += n;
-    const int b1 = b + 1 == n ? 0 : b + 1;
-    idx[0] = b; idx[1] = b1; idx[2] = b1 + 1 == n ? 0 : b1 + 1;
-}
-// The mixed form's midpoint gather (Fourier y): the interleaved midpoint fields with FP32 weights, straight into
-// the FP32 fields of the Boris push.
-__device__ __forceinline__ void sgather_mid_f32(const StreamArgs& c, double x, double y, float E[3], float B[3]) {
-    int ix[3], jn[3]; float wx[3], wn[3];
-    tsc_f32(x, c.inv_dx, c.g.nx, ix, wx);
-    tsc_f32(y, c.inv_dy, c.g.ny, jn, wn);
-    float a[6] = {0, 0, 0, 0, 0, 0};
-    const float4* F4 = reinterpret_cast<const float4*>(c.Fmid);
-#pragma unroll
-    for (int j = 0; j < 3; ++j)
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const long k = long(jn[j]) * c.g.nx + ix[i];
-            const float w = wx[i] * wn[j];
-            const float4 u = __ldg(F4 + 2 * k), v = __ldg(F4 + 2 * k + 1);
-            a[0] += w * u.x; a[1] += w * u.y; a[2] += w * u.z; a[3] += w * u.w; a[4] += w * v.x; a[5] += w * v.y;
-        }
-    E[0] = a[0]; E[1] = a[1]; E[2] = a[2]; B[0] = a[3]; B[1] = a[4]; B[2] = a[5];
 }
 // The mixed form's midpoint gather on the free-hand y grid: per TSC point one float4 of the node row (E_x, E_z, B_y)
 // and one of the half-node row (E_y, B_x, B_z) of the interleaved midpoint fields, rows beyond the walls left out
@@ -362,14 +347,33 @@ __device__ void ionize(const StreamArgs& c, const StrmDev& S, long i, double E1,
     if (Z != Z0 && !c.dry) { S.q[i] = Z; S.qm[i] = Z / I.mass; }
 }
 
-// The deposit of one particle in one half-cell: f (v_x, v_y, v_z, 1) at (x, y) (stream_deposit)
+// The deposit of one particle in one half-cell: f (v_x, v_y, v_z, 1) at (x, y) (stream_deposit); T: FP32 in the mixed form
+// on the Fourier y grid
+template <class T>
 struct DepReq {
-    double x, y, f, vx, vy, vz;
+    double x, y;
+    T f, v[3];
     bool on;
-    bool f32;                  // the mixed form on the Fourier y grid: FP32 deposit weights from ff, fv (sdeposit_warp)
-    float ff, fv[3];
 };
+template <bool F32, bool YF>
+struct DepType { typedef typename std::conditional<F32 && YF, float, double>::type T; };
+// the charge of a particle at rest on the density lines (its current is zero)
+__device__ __forceinline__ void scharge_lines(const StreamArgs& c, double x, double y, double f) {
+    if (!c.rl[f < 0 ? 0 : 1]) return;
+    int ix[3], jn[3];
+    double wx[3], wn[3];
+    tsc_periodic(x, c.g.dx, c.g.nx, ix, wx);
+    tsc_periodic(y, c.g.dy, c.g.ny, jn, wn);
+    sdeposit_lines(c, f, ix, jn, [&](int u, int v) { return f * wx[u] * wn[v] * c.ia0; });
+}
 
+// A streaming particle's state as the push reads it: all of it at once, before any branch or store (a load behind a
+// branch waits for the branch's own load, and a load behind a store to another column, which the compiler must assume may
+// alias it, for that store). Every index below the list's capacity is a valid slot of every column.
+struct StreamState {
+    double x, y, zeta, px, py, pz, w, z, q, qm;
+    int alive, sp;
+};
 // one streaming particle through half-cell n (stream_one, sim_stream.hpp:104-171); its deposit is returned to
 // the caller, the rare second deposit of a trapped particle that joins the beam list is made here. A predictor
 // pass (c.dry) computes and deposits the same but leaves the particle as it was, so every pass of a half-cell
@@ -379,21 +383,16 @@ struct DepReq {
 // EX: exact fields (FP64 form, Fourier y, neither ionization nor the analytic wave): the gathers from the FP64 planes.
 // REC: the variant that writes the adjoint's record (c.recd, first pass), launched only when recording.
 template <bool F32, bool ION, bool LASER, bool YF, bool EX = false, bool REC = false>
-__device__ __forceinline__ DepReq stream_one(const StreamArgs& c, const StrmDev& S, long i) {
-    DepReq d{0, 0, 0, 0, 0, 0, false, false, 0.f, {0.f, 0.f, 0.f}};
+__device__ __forceinline__ DepReq<typename DepType<F32, YF>::T> stream_one(const StreamArgs& c, const StrmDev& S, long i, const StreamState& s, double sTrap) {
+    typedef typename DepType<F32, YF>::T DT;
+    DepReq<DT> d{0, 0, DT(0), {DT(0), DT(0), DT(0)}, false};
     const Geo& g = c.g;
     const int n = c.n;
-    const double zn = g.zs[n], zn1 = g.zs[n + 1], h = zn1 - zn;
-    // The whole state is loaded at once, before any branch or store: a load behind a branch waits for the
-    // branch's own load, and a load behind a store to another array of the state (which the compiler must
-    // assume may alias it) waits for that store. Every index below the count is a valid slot of every array.
+    const double zn = c.zn, zn1 = c.zn1, h = zn1 - zn;
     typedef double A;     // the push arithmetic: FP64 in both forms (the mixed form's FP32 push gave 3-4x its F error)
-    int alive = S.alive[i];
-    const int sp = S.sp[i];
-    const double zeta = S.zeta[i], x = S.x[i], y = S.y[i], z = S.z[i];
-    const double px_ = S.px[i], py_ = S.py[i], pz_ = S.pz[i], qm_ = S.qm[i];
-    const double qw = S.q[i] * S.w[i];
-    const double sTrap = c.sv->sTrap, s1 = c.sv->s1;
+    int alive = s.alive;
+    const int sp = s.sp;
+    const double zeta = s.zeta, x = s.x, y = s.y, z = s.z, px_ = s.px, py_ = s.py, pz_ = s.pz, qm_ = s.qm, qw = s.q * s.w;
     if constexpr (REC) {
         if (c.recd && c.pass == 0) {                 // the adjoint's record: the state entering half-cell n
             const RecDev R = *c.recd;
@@ -412,7 +411,10 @@ __device__ __forceinline__ DepReq stream_one(const StreamArgs& c, const StrmDev&
     const bool ion = sp >= SP_ION && sp < SP_FREED;
     if (ion && !c.ions[sp - SP_ION].mobile) {        // fixed ion: its charge, then the ionization
         const double f = qw * hl / (c.Delta * h * g.dx);
-        if (f != 0) d = DepReq{x, y, f, 0, 0, 0, true, false, 0.f, {0.f, 0.f, 0.f}};
+        if (f != 0) {
+            if constexpr (YF) scharge_lines(c, x, y, f);
+            else d = DepReq<DT>{x, y, DT(f), {DT(0), DT(0), DT(0)}, true};
+        }
         if (!c.dry) S.zeta[i] = zn;
         if constexpr (ION) {
             const double E1 = field_abs<F32, YF>(c, x, y, z, zeta), E0 = field_abs<F32, YF>(c, x, y, z, zn);
@@ -424,9 +426,11 @@ __device__ __forceinline__ DepReq stream_one(const StreamArgs& c, const StrmDev&
     // steps, gamma, 1 - v_z and velocities are FP64 (measured on the laser-plasma workload: FP32 arithmetic here put
     // 3-4x more error into F over 1-5 s-steps, for 2.6 % less time in this kernel)
     const A px = A(px_), py = A(py_), pz = A(pz_), qm = A(qm_);
-    const A g0 = sqrt(A(1) + px * px + py * py + pz * pz), ig0 = A(1) / g0;
-    const A omv0 = (A(1) + px * px + py * py) / (g0 * (g0 + pz));     // 1 - v_z, no cancellation
-    const A dt0 = A(hl) / omv0;
+    // 1 - v_z = N / D with N = 1 + p_perp^2, D = gamma (gamma + p_z): no cancellation; gamma by rsqrt, which gives
+    // 1/gamma too, and one quotient for the time (an FP64 quotient or root is 15 to 20 instructions here)
+    const A N0 = A(1) + px * px + py * py, a0 = N0 + pz * pz, ig0 = rsqrt(a0), g0 = a0 * ig0;
+    const A D0 = g0 * (g0 + pz);
+    const A dt0 = A(hl) * D0 / N0;
     const A hd = A(0.5) * dt0 * ig0;
     const double xm = x + double(hd * px), ym = y + double(hd * py);
     const double zm = z + double(hd * pz), zetam = zeta - 0.5 * hl;
@@ -436,16 +440,15 @@ __device__ __forceinline__ DepReq stream_one(const StreamArgs& c, const StrmDev&
         // a neutral atom: the Boris pushes below leave u exactly as it is whatever the (finite) fields, so they
         // are not gathered (the gas of an ionization-injection run is mostly neutral until the laser arrives)
         for (int k = 0; k < 3; ++k) { E[k] = A(0); B[k] = A(0); }
-    } else if (F32 && mid && !LASER && !c.ext.any()) {
-        if constexpr (F32) {
+    } else if (!YF && F32 && mid && !LASER && !c.ext.any()) {
+        if constexpr (F32 && !YF) {                               // free-hand: Fmid is FP32-only
             float Ef[3], Bf[3];
-            if constexpr (YF) sgather_mid_f32(c, wrapx(g, xm), wrapy<YF>(g, ym), Ef, Bf);
-            else sgather_mid_fh_f32(c, wrapx(g, xm), ym, Ef, Bf);
+            sgather_mid_fh_f32(c, wrapx(g, xm), ym, Ef, Bf);
             for (int k = 0; k < 3; ++k) { E[k] = A(Ef[k]); B[k] = A(Bf[k]); }
         }
     } else {
         double Ed[3], Bd[3], Ee[3], Be[3];
-        if (YF && mid) sgather_mid<F32>(c, wrapx(g, xm), wrapy<YF>(g, ym), Ed, Bd);   // free-hand: Fmid is FP32-only
+        if (YF && mid) sgather_mid<F32>(c, xm, ym, Ed, Bd);
         else if (EX) sgather_exact(c, wrapx(g, xm), wrapy<YF>(g, ym), zetam, Ed, Bd);
         else sgather<F32, YF>(c, wrapx(g, xm), wrapy<YF>(g, ym), zetam, Ed, Bd);
         if constexpr (LASER) {
@@ -455,14 +458,16 @@ __device__ __forceinline__ DepReq stream_one(const StreamArgs& c, const StrmDev&
         if (c.ext.any()) add_external(c.ext, xm + c.sv->X0, ym + c.sv->Y0, zm, Bd);   // sim_stream.hpp:133
         for (int k = 0; k < 3; ++k) { E[k] = A(Ed[k]); B[k] = A(Bd[k]); }
     }
-    A ux = px, uy = py, uz = pz;
-    boris<A>(ux, uy, uz, E, B, qm, dt0);
-    A g1 = sqrt(A(1) + ux * ux + uy * uy + uz * uz);
-    A dt = A(2) * A(hl) / (omv0 + (A(1) + ux * ux + uy * uy) / (g1 * (g1 + uz)));
-    ux = px; uy = py; uz = pz;
-    boris<A>(ux, uy, uz, E, B, qm, dt);
-    g1 = sqrt(A(1) + ux * ux + uy * uy + uz * uz);
-    A ig1 = A(1) / g1;
+    A ux = px, uy = py, uz = pz, dt = dt0, ig1 = ig0;
+    if (qm_ != 0) {                   // a neutral atom keeps u, and the time of its half-cell is dt0
+        boris<A>(ux, uy, uz, E, B, qm, dt0);
+        // dt = 2 hl / ((1 - v_z)_0 + (1 - v_z)_1), over the common denominator
+        const A N1 = A(1) + ux * ux + uy * uy, a1 = N1 + uz * uz, g1 = a1 * rsqrt(a1), D1 = g1 * (g1 + uz);
+        dt = A(2) * A(hl) * D0 * D1 / (N0 * D1 + N1 * D0);
+        ux = px; uy = py; uz = pz;
+        boris<A>(ux, uy, uz, E, B, qm, dt);
+        ig1 = rsqrt(A(1) + ux * ux + uy * uy + uz * uz);
+    }
     A vx = A(0.5) * (px * ig0 + ux * ig1), vy = A(0.5) * (py * ig0 + uy * ig1), vz = A(0.5) * (pz * ig0 + uz * ig1);
     double zeta_end = zn;
     bool trapped = false;
@@ -471,8 +476,7 @@ __device__ __forceinline__ DepReq stream_one(const StreamArgs& c, const StrmDev&
         const double dtp = (sTrap - z) / vv > 0 ? (sTrap - z) / vv : 0.0;
         ux = px; uy = py; uz = pz;
         boris<A>(ux, uy, uz, E, B, qm, A(dtp));
-        g1 = sqrt(A(1) + ux * ux + uy * uy + uz * uz);
-        ig1 = A(1) / g1;
+        ig1 = rsqrt(A(1) + ux * ux + uy * uy + uz * uz);
         vx = A(0.5) * (px * ig0 + ux * ig1); vy = A(0.5) * (py * ig0 + uy * ig1); vz = A(0.5) * (pz * ig0 + uz * ig1);
         dt = A(dtp);
         zeta_end = zeta - (1 - double(vz)) * dtp;
@@ -481,21 +485,15 @@ __device__ __forceinline__ DepReq stream_one(const StreamArgs& c, const StrmDev&
     const double xn = x + double(vx * dt), yn = y + double(vy * dt);
     if (!c.dry) {
         S.x[i] = xn; S.y[i] = yn;
-        S.z[i] = trapped ? s1 : z + double(vz * dt);
+        S.z[i] = trapped ? c.sv->s1 : z + double(vz * dt);
         S.px[i] = ux; S.py[i] = uy; S.pz[i] = uz;
         S.zeta[i] = zeta_end;
     }
-    if constexpr (F32) {
-        if constexpr (YF) {           // FP32 deposit: the factor 1 / (Delta h dx) taken once per half-cell
-            const float ff = float(qw * c.dep_norm) * float(dt);
-            if (ff != 0.f) d = DepReq{0.5 * (x + xn), 0.5 * (y + yn), 0, 0, 0, 0, true, true, ff, {float(vx), float(vy), float(vz)}};
-        } else {
-            const double f = qw * double(dt) / (c.Delta * h * g.dx);
-            if (f != 0) d = DepReq{0.5 * (x + xn), 0.5 * (y + yn), f, double(vx), double(vy), double(vz), true, false, 0.f, {0.f, 0.f, 0.f}};
-        }
-    } else {
-        const double f = qw * double(dt) / (c.Delta * h * g.dx);
-        if (f != 0) d = DepReq{0.5 * (x + xn), 0.5 * (y + yn), f, double(vx), double(vy), double(vz), true, false, 0.f, {0.f, 0.f, 0.f}};
+    {
+        DT f;
+        if constexpr (F32 && YF) f = float(qw * c.dep_norm) * float(dt);
+        else f = qw * double(dt) * c.dep_norm;
+        if (f != DT(0)) d = DepReq<DT>{0.5 * (x + xn), 0.5 * (y + yn), f, {DT(vx), DT(vy), DT(vz)}, true};
     }
     if (!YF && (yn < c.ylo || yn > c.yhi)) {        // free-hand y: reached the cell at a wall
         if (!c.dry) S.alive[i] = 0;
@@ -507,8 +505,9 @@ __device__ __forceinline__ DepReq stream_one(const StreamArgs& c, const StrmDev&
     if (trapped) {
         if (!c.dry) S.alive[i] = 5;
         const double vze = double(uz * ig1);
-        if (vze >= c.vz_beam)         // joins the beam list: its beam current of level s1 from now on
+        if (vze >= c.vz_beam) {       // joins the beam list: its beam current of level s1 from now on
             sdeposit<F32, YF>(c, xn, yn, qw / (h * g.dx * vze), double(ux * ig1), double(uy * ig1), vze);
+        }
     }
     return d;
 }
@@ -516,29 +515,20 @@ __device__ __forceinline__ DepReq stream_one(const StreamArgs& c, const StrmDev&
 // The deposit of a warp's particles on the Fourier y grid, the adds of particles that share a TSC stencil summed in
 // registers first. Lanes whose stencils start at the same grid point form a group (a match on the stencil's first
 // point): on the plasma lattice the electron and the ion of a lattice point and the neighbouring points that round to
-// the same node, about three lanes. A tree inside each group (every round, each lane of even rank in the group adds
+// the same node, about four lanes. A tree inside each group (every round, each lane of even rank in the group adds
 // the value of the next remaining member above it, and the odd ranks leave) leaves the group's sum with its lowest
-// lane, which alone issues the adds: a third of the reductions into L2, which bound the streaming push (measured:
-// without its deposit adds the FP64 push takes 36 % less time, the mixed one 21 %). Row by row (three points of
-// three components), so that few values are live. Every lane of the warp calls it; `on` false: nothing to deposit.
+// lane, which alone issues the adds: a third of the reductions into L2. Row by row (three points of three components),
+// so that few values are live. Every lane of the warp calls it; d.on false: nothing to deposit.
 template <bool F32>
-__device__ __forceinline__ void sdeposit_warp(const StreamArgs& c, const DepReq& d, bool on, int lane) {
-    typedef typename std::conditional<F32, float, double>::type T;
+__device__ __forceinline__ void sdeposit_warp(const StreamArgs& c, const DepReq<typename DepType<F32, true>::T>& d, int lane) {
+    typedef typename DepType<F32, true>::T T;
     const Geo& g = c.g;
     int ix[3], jn[3];
-    T wx[3], wn[3], fa, v3[3];
-    if constexpr (F32) {
-        tsc_f32(d.x, c.inv_dx, g.nx, ix, wx);
-        tsc_f32(d.y, c.inv_dy, g.ny, jn, wn);
-        fa = d.ff * float(g.iA[0]);
-        v3[0] = d.fv[0]; v3[1] = d.fv[1]; v3[2] = d.fv[2];
-    } else {
-        tsc_periodic(d.x, g.dx, g.nx, ix, wx);
-        tsc_periodic(d.y, g.dy, g.ny, jn, wn);
-        fa = d.f;
-        v3[0] = d.vx; v3[1] = d.vy; v3[2] = d.vz;
-    }
-    const double ia0 = g.iA[0];
+    T wx[3], wn[3];
+    const bool on = d.on;
+    tsc_stream<T>(d.x, c.inv_dx, g.nx, ix, wx);
+    tsc_stream<T>(d.y, c.inv_dy, g.ny, jn, wn);
+    const T fa = d.f * T(c.ia0);
     const unsigned all = 0xffffffffu;
     const int key = on ? jn[0] * g.nx + ix[0] : -1 - lane;
     const unsigned peers = __match_any_sync(all, key);
@@ -549,11 +539,9 @@ __device__ __forceinline__ void sdeposit_warp(const StreamArgs& c, const DepReq&
         T a[3][3];
 #pragma unroll
         for (int u = 0; u < 3; ++u) {
-            T w;
-            if constexpr (F32) w = fa * wx[u] * wn[v];
-            else w = fa * wx[u] * wn[v] * ia0;
+            const T w = fa * wx[u] * wn[v];
 #pragma unroll
-            for (int k = 0; k < 3; ++k) a[u][k] = on ? w * v3[k] : T(0);
+            for (int k = 0; k < 3; ++k) a[u][k] = on ? w * d.v[k] : T(0);
         }
         unsigned above = above0, rank = rank0;
         while (__any_sync(all, above != 0u)) {
@@ -574,7 +562,7 @@ __device__ __forceinline__ void sdeposit_warp(const StreamArgs& c, const DepReq&
         if (on && rank0 == 0u) {
 #pragma unroll
             for (int u = 0; u < 3; ++u) {
-                const long k = long(jn[v]) * g.nx + ix[u];
+                const int k = jn[v] * g.nx + ix[u];
                 if constexpr (F32) {
                     atomicAdd(reinterpret_cast<float4*>(c.Jf) + k, make_float4(a[u][0], a[u][1], a[u][2], 0.f));
                 } else {
@@ -583,10 +571,7 @@ __device__ __forceinline__ void sdeposit_warp(const StreamArgs& c, const DepReq&
             }
         }
     }
-    if (on) {
-        if constexpr (F32) sdeposit_lines(c, d.ff, ix, jn, [&](int u, int v) { return fa * wx[u] * wn[v]; });
-        else sdeposit_lines(c, d.f, ix, jn, [&](int u, int v) { return d.f * wx[u] * wn[v] * ia0; });
-    }
+    if (on) sdeposit_lines(c, fa, ix, jn, [&](int u, int v) { return fa * wx[u] * wn[v]; });
 }
 
 // One thread per streaming particle, a fixed grid striding over their count (which freed electrons raise; it is
@@ -595,11 +580,18 @@ __device__ __forceinline__ void sdeposit_warp(const StreamArgs& c, const DepReq&
 // neighbouring lattice particles make to the same points. F32 (the mixed form): the gathers in FP32 from FP32 field
 // planes, the deposit into FP32 planes; the push arithmetic and the particle state stay FP64.
 constexpr int ST_NT = 128;
-// Resident CTAs per SM the register budget of the plain variant is sized for, by form. With the per-thread deposit,
-// 5 (96 registers) against 6 (80) gave 55.8 against 57.8 us per launch in the mixed form and 89.7 against 91.8 us in
-// the FP64 form (laser-plasma workload, one box); 4, 7 and 8 were slower. With the warp-summed deposit the mixed form
-// prefers 6 (47.1 and 46.6 against 47.7 and 48.9 us, 4: 52.6) and the FP64 form keeps 5 (66.5 against 66.8 at 6, 71.4
-// at 4; 256 x 256 x 128 case, all builds alternated in one call).
+// Resident CTAs per SM the register budget of the plain variant is sized for, by form: the mixed form 6 (80 registers; 38.6 us
+// per launch against 41.8 at 5), the FP64 form 5 (96 registers; 57.5 us against 58.1 at 4), the events' ~5 us included
+// (256 x 256 laser-plasma case, 540,000 particles, all builds in one call).
+// What bounds the push is latency and instructions, not bytes: a warp's chain is the particle state, the gather, two Boris
+// pushes and the deposit, at 20 to 24 resident warps. So the code on that chain is kept short: one root and one quotient
+// where a textbook form has two or three of each, no integer remainder, no product formed twice, the deposit handed on
+// as four values of the form's own precision (with an FP64 copy of them beside, the mixed kernel spilled). That took
+// 66.4 -> 57.5 us (FP64) and 54.8 -> 38.6 us (mixed) per launch; the roots and quotients alone 40.2 -> 38.6 us in the mixed form.
+// Tried and slower: the next particles' state on its way into shared memory by cp.async during the push (a persistent grid:
+// 58.4 -> 61.3 us mixed; the 28 KB a CTA come out of L1, where the gather lives); the points of a warp's groups dealt
+// to all its lanes through shared memory instead of the tree of shuffles (38.6 -> 41.2 us mixed, 57.5 -> 60.3 us FP64); the rare
+// branches out of line (64 x 64: 15.4 -> 16.9 us).
 #ifndef G3D_STREAM_MINB
 #define G3D_STREAM_MINB 5
 #endif
@@ -609,45 +601,44 @@ constexpr int ST_NT = 128;
 // YF: the Fourier y grid (true) or the free-hand one, fixed for a run, so that each variant holds only its own grid's
 // gathers and deposits (fewer registers and no local arrays).
 template <bool F32, bool ION, bool LASER, bool YF, bool EX = false, bool REC = false>
-__global__ void __launch_bounds__(ST_NT, (ION || LASER) ? 4 : F32 ? G3D_STREAM_MINB_F32 : G3D_STREAM_MINB) k_stream(StreamArgs c,
+__global__ void __launch_bounds__(ST_NT, (ION || LASER) ? 4 : F32 ? G3D_STREAM_MINB_F32 : G3D_STREAM_MINB) k_stream(const __grid_constant__ StreamArgs c,
                                                                                        const long* __restrict__ nstrm) {
     const StrmDev S = c.sd[0];
     const long n = *nstrm;
     const int lane = int(threadIdx.x & 31u);
+    const double sTrap = c.sv->sTrap;
+    typedef typename DepType<F32, YF>::T DT;
     // the warp strides as a whole (its lanes meet in the warp's deposit): b is the warp's first particle
     for (long b = long(blockIdx.x) * ST_NT + long(threadIdx.x & ~31u); b < n; b += long(gridDim.x) * ST_NT) {
         const long i = b + lane;
-        DepReq d{0, 0, 0, 0, 0, 0, false, false, 0.f, {0.f, 0.f, 0.f}};
-        if (i < n) d = stream_one<F32, ION, LASER, YF, EX, REC>(c, S, i);
-        if constexpr (YF) {
-            const bool warp = d.on && (!F32 || d.f32);   // F32: a fixed ion's charge alone takes the plain deposit
-            sdeposit_warp<F32>(c, d, warp, lane);
-            if (d.on && !warp) sdeposit<F32, YF>(c, d.x, d.y, d.f, d.vx, d.vy, d.vz);
-        } else if (d.on) {
-            sdeposit<F32, YF>(c, d.x, d.y, d.f, d.vx, d.vy, d.vz);
+        DepReq<DT> d{0, 0, DT(0), {DT(0), DT(0), DT(0)}, false};
+        if (i < n) {
+            const StreamState s{S.x[i], S.y[i], S.zeta[i], S.px[i], S.py[i], S.pz[i], S.w[i], S.z[i], S.q[i], S.qm[i], S.alive[i], S.sp[i]};
+            d = stream_one<F32, ION, LASER, YF, EX, REC>(c, S, i, s, sTrap);
         }
+        if constexpr (YF) sdeposit_warp<F32>(c, d, lane);
+        else if (d.on) sdeposit<F32, YF>(c, d.x, d.y, d.f, d.v[0], d.v[1], d.v[2]);
     }
 }
 template <bool F32, bool YF>
 static void stream_launch_y(Ctx& c, const StreamArgs& a, unsigned blocks) {
     PlasmaState& P = *c.pl;
     const bool ion = P.any_ionizing, las = c.laser.on != 0;
+    auto go = [&](void (*kern)(StreamArgs, const long*)) {
+        kern<<<blocks, ST_NT, 0, c.stream>>>(a, P.nstrm_dev.p);
+    };
     if constexpr (!F32 && YF) {
-        if (a.Fd && !ion && !las) {                  // exact fields (the adjoint's forward, writing its record when asked)
-            k_stream<false, false, false, true, true, true><<<blocks, ST_NT, 0, c.stream>>>(a, P.nstrm_dev.p);
-            return;
-        }
+        if (a.Fd && !ion && !las) { go(k_stream<false, false, false, true, true, true>); return; }   // exact fields (the
+                                                      // adjoint's forward, writing its record when asked)
     }
     if constexpr (F32 && YF) {
-        if (a.recd && !ion && !las) {                // the mixed form's forward of the adjoint, writing its record
-            k_stream<true, false, false, true, false, true><<<blocks, ST_NT, 0, c.stream>>>(a, P.nstrm_dev.p);
-            return;
-        }
+        if (a.recd && !ion && !las) { go(k_stream<true, false, false, true, false, true>); return; } // the mixed form's
+                                                      // forward of the adjoint, writing its record
     }
-    if (ion && las) k_stream<F32, true, true, YF><<<blocks, ST_NT, 0, c.stream>>>(a, P.nstrm_dev.p);
-    else if (ion) k_stream<F32, true, false, YF><<<blocks, ST_NT, 0, c.stream>>>(a, P.nstrm_dev.p);
-    else if (las) k_stream<F32, false, true, YF><<<blocks, ST_NT, 0, c.stream>>>(a, P.nstrm_dev.p);
-    else k_stream<F32, false, false, YF><<<blocks, ST_NT, 0, c.stream>>>(a, P.nstrm_dev.p);
+    if (ion && las) go(k_stream<F32, true, true, YF>);
+    else if (ion) go(k_stream<F32, true, false, YF>);
+    else if (las) go(k_stream<F32, false, true, YF>);
+    else go(k_stream<F32, false, false, YF>);
 }
 template <bool F32>
 static void stream_launch(Ctx& c, const StreamArgs& a, unsigned blocks) {
@@ -673,6 +664,7 @@ __global__ void __launch_bounds__(slice_row_threads<NX>()) k_ss_rows(Geo g, JT* 
     const long nk = g.nk, k0 = long(row) * NX;
     // every load first, then the clears for the next pass's deposit, then shared memory: a clear between two loads
     // would keep the second waiting for the first (the compiler cannot move a load above a store it may alias)
+    stage_twiddles<NX>(stw, g.twx, tid, NTH);
     double jx[EPT], jy[EPT], jz[EPT];
 #pragma unroll
     for (int u = 0; u < EPT; ++u) {
@@ -688,7 +680,6 @@ __global__ void __launch_bounds__(slice_row_threads<NX>()) k_ss_rows(Geo g, JT* 
             }
         }
     }
-    stage_twiddles<NX>(stw, g.twx, tid, NTH);
     if (clear) {
 #pragma unroll
         for (int u = 0; u < EPT; ++u) {
