@@ -23,6 +23,7 @@
 #include <cub/device/device_scan.cuh>
 #include "g3d_plasma.hpp"
 #include "k_external.cuh"
+#include "k_pdl.cuh"
 #include "k_fft.cuh"
 #include "k_dispatch.cuh"
 
@@ -608,6 +609,8 @@ __global__ void __launch_bounds__(ST_NT, (ION || LASER) ? 4 : F32 ? G3D_STREAM_M
     const int lane = int(threadIdx.x & 31u);
     const double sTrap = c.sv->sTrap;
     typedef typename DepType<F32, YF>::T DT;
+    pdl_wait();
+    pdl_next();
     // the warp strides as a whole (its lanes meet in the warp's deposit): b is the warp's first particle
     for (long b = long(blockIdx.x) * ST_NT + long(threadIdx.x & ~31u); b < n; b += long(gridDim.x) * ST_NT) {
         const long i = b + lane;
@@ -625,7 +628,7 @@ static void stream_launch_y(Ctx& c, const StreamArgs& a, unsigned blocks) {
     PlasmaState& P = *c.pl;
     const bool ion = P.any_ionizing, las = c.laser.on != 0;
     auto go = [&](void (*kern)(StreamArgs, const long*)) {
-        kern<<<blocks, ST_NT, 0, c.stream>>>(a, P.nstrm_dev.p);
+        launch_pdl(c.stream, kern, blocks, ST_NT, 0, a, P.nstrm_dev.p);
     };
     if constexpr (!F32 && YF) {
         if (a.Fd && !ion && !las) { go(k_stream<false, false, false, true, true, true>); return; }   // exact fields (the
@@ -665,6 +668,8 @@ __global__ void __launch_bounds__(slice_row_threads<NX>()) k_ss_rows(Geo g, JT* 
     // every load first, then the clears for the next pass's deposit, then shared memory: a clear between two loads
     // would keep the second waiting for the first (the compiler cannot move a load above a store it may alias)
     stage_twiddles<NX>(stw, g.twx, tid, NTH);
+    pdl_wait();
+    pdl_next();
     double jx[EPT], jy[EPT], jz[EPT];
 #pragma unroll
     for (int u = 0; u < EPT; ++u) {
@@ -878,8 +883,8 @@ __global__ void __launch_bounds__(NY) k_pass_cols(PlasmaPtrs p, Geo g, const cpx
     const int kxi = blockIdx.x, j = threadIdx.x;
     const long nk = g.nkh, i = long(j) * g.H + kxi;
     const int grp = j / S::T, tl = j % S::T;
-    // (1) the loads, none of them converted yet: a conversion would wait for its load and hold back the ones behind it
-    const cpx c0 = T0[i], c1 = T1[i], c2 = T2[i];
+    // (1) the loads, none of them converted yet: a conversion would wait for its load and hold back the ones behind it. The
+    // rows kernel before this one writes only T0..T2: all else is loaded while it still runs.
     const long hp = long(n + 1) * nk + i, hq = long(n) * nk + i;      // half-cells n and n-1
     T* const jk[3] = {static_cast<T*>(p.jkx), static_cast<T*>(p.jky), static_cast<T*>(p.jkz)};
     cpx* const s0[3] = {p.js0x, p.js0y, p.js0z};
@@ -906,6 +911,9 @@ __global__ void __launch_bounds__(NY) k_pass_cols(PlasmaPtrs p, Geo g, const cpx
     const double wl = g.wlo[n], wu = g.whi[n], h = g.hcg[n + 2];
     stage_twiddles<NY>(ftw, g.twy, j, NY);
     if constexpr (!std::is_same<WT, cpx>::value) stage_twiddles<NY>(ib + 6 * Tile::size, twi, j, NY);
+    pdl_wait();
+    pdl_next();
+    const cpx c0 = T0[i], c1 = T1[i], c2 = T2[i];
     // (2) the current's column, transformed and filtered
     fl[Tile::at(j, 0)] = c0; fl[Tile::size + Tile::at(j, 0)] = c1; fl[2 * Tile::size + Tile::at(j, 0)] = c2;
     const double k2 = kx * kx + ky * ky;
@@ -1209,7 +1217,7 @@ template <int NX, class JT>
 static void ss_rows(Ctx& c, JT* J, cpx* T, int clear = 0, int* bcnt = nullptr) {
     const size_t smem = (size_t(2) * row_stride<NX>() + NX) * sizeof(cpx);
     smem_attr(reinterpret_cast<const void*>(k_ss_rows<NX, JT>), smem);
-    k_ss_rows<NX, JT><<<unsigned(c.ny), slice_row_threads<NX>(), smem, c.stream>>>(c.geo(), J, T, T + c.nkh, T + 2 * c.nkh, clear, bcnt);
+    launch_pdl(c.stream, k_ss_rows<NX, JT>, unsigned(c.ny), slice_row_threads<NX>(), smem, c.geo(), J, T, T + c.nkh, T + 2 * c.nkh, clear, bcnt);
     c.check_launch("k_ss_rows");
 }
 template <int NY>
@@ -1495,9 +1503,8 @@ static void pass_cols_form(Ctx& c, double D, int n, int extrap, double w, double
                         (6 * ColTile<NY, 1>::size + (std::is_same<WT, cpx>::value ? 0 : NY)) * sizeof(WT);
     auto kern = k_pass_cols<NY, T, WT, LAST>;
     smem_attr(reinterpret_cast<const void*>(kern), smem);
-    kern<<<unsigned(c.H), NY, smem, c.stream>>>(P.ptrs(c), c.geo(), S, S + c.nkh, S + 2 * c.nkh, a2, P.box_mean ? 1 : 0, c.Rx.p, c.Ry.p, Ez,
-                                                Bz, Lx, Ly, j0x, j0y, D, n, extrap, w, q, tw, W[0].p, W[1].p, W[2].p, W[3].p, W[4].p,
-                                                W[5].p);
+    launch_pdl(c.stream, kern, unsigned(c.H), NY, smem, P.ptrs(c), c.geo(), S, S + c.nkh, S + 2 * c.nkh, a2, P.box_mean ? 1 : 0, c.Rx.p,
+               c.Ry.p, Ez, Bz, Lx, Ly, j0x, j0y, D, n, extrap, w, q, tw, W[0].p, W[1].p, W[2].p, W[3].p, W[4].p, W[5].p);
 }
 template <int NY>
 static void pass_cols(Ctx& c, double D, int n, int extrap, double w, double q, bool last) {

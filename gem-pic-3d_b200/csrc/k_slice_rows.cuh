@@ -10,6 +10,7 @@
 #pragma once
 #include "g3d_ctx.hpp"
 #include "k_fft.cuh"
+#include "k_pdl.cuh"
 
 namespace g3d {
 
@@ -30,15 +31,7 @@ __global__ void __launch_bounds__(slice_row_threads<NX>()) k_rf_row_slice(Geo g,
     T* stw = reinterpret_cast<T*>(smr) + 3 * RS;
     const int row = blockIdx.x, tid = threadIdx.x;
     const long fpl = long(g.ns + 2) * g.nk, k0 = long(row) * NX, base = long(lw) * g.nkh + long(row) * H;
-    // every load before the first store to shared memory
-    const T* in[6] = {W0, W1, W2, W3, W4, W5};
-    T v[EI][6];
-#pragma unroll
-    for (int u = 0; u < EI; ++u) {
-        const int p = tid + u * NTH;
-#pragma unroll
-        for (int f = 0; f < 6; ++f) v[u][f] = p < H ? in[f][base + p] : mk<T>(0, 0);
-    }
+    // the other slice was written long before the columns kernel this one follows: loaded while that still runs
     float oth[XM ? 1 : EO][6];                                      // the midpoint fields' other slice
     double othd[XM ? EO : 1][6];
     if (fm.out) {
@@ -55,6 +48,16 @@ __global__ void __launch_bounds__(slice_row_threads<NX>()) k_rf_row_slice(Geo g,
         }
     }
     stage_twiddles<NX>(stw, tw, tid, NTH);
+    pdl_wait();
+    pdl_next();
+    const T* in[6] = {W0, W1, W2, W3, W4, W5};
+    T v[EI][6];
+#pragma unroll
+    for (int u = 0; u < EI; ++u) {
+        const int p = tid + u * NTH;
+#pragma unroll
+        for (int f = 0; f < 6; ++f) v[u][f] = p < H ? in[f][base + p] : mk<T>(0, 0);
+    }
 #pragma unroll
     for (int u = 0; u < EI; ++u) {
         const int p = tid + u * NTH;
@@ -115,7 +118,7 @@ static void rf_row_slice(Ctx& c, const T* tw, const T* W0, const T* W1, const T*
     auto kern = k_rf_row_slice<NX, T, XM>;
     smem_attr(reinterpret_cast<const void*>(kern), smem);
     const int tok = c.prof_begin("real_rows_slice");
-    kern<<<unsigned(c.ny), slice_row_threads<NX>(), smem, c.stream>>>(c.geo(), tw, W0, W1, W2, W3, W4, W5, c.F.p, l, lw, Fd, fm);
+    launch_pdl(c.stream, kern, unsigned(c.ny), slice_row_threads<NX>(), smem, c.geo(), tw, W0, W1, W2, W3, W4, W5, c.F.p, l, lw, Fd, fm);
     c.check_launch("k_rf_row_slice");
     c.prof_end(tok);
 }
