@@ -68,7 +68,9 @@ struct LaserDev {
         const double xi = eta(x, z, t) - eta_c;
         double g, gp;
         if (!envelope(xi, g, gp)) return;
-        const double ph = kL * xi + cep, c = cos(ph), s = sin(ph);
+        const double ph = kL * xi + cep;
+        double c, s;
+        sincos(ph, &s, &c);
         const double d1 = a0 * (gp * c - kL * g * s), d2 = a0 * (gp * s + kL * g * c);
         if (pol == 0) { E[1] = -d1; }
         else if (pol == 1) { E[0] = -d1 * kz; E[2] = d1 * kx; }
