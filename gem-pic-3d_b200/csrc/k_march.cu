@@ -22,7 +22,7 @@ namespace g3d {
 namespace {
 constexpr int MA = 9;       // complex arrays streamed per slice
 constexpr int MC = 3;       // per-slice coefficients streamed with them: w_lo, w_hi, h
-constexpr int slot_doubles(int bt) { return MA * bt + MC * bt; }   // doubles per ring slot (one value per lane)
+constexpr int slot_doubles(int bt) { return (MA + MC) * bt; }      // doubles per ring slot (one value per lane)
 
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
     const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
@@ -54,10 +54,13 @@ __device__ __forceinline__ double ring_re(const double* cell) {
 // (Im R, Im L, Re E_z, Re B_z); each lane makes the same products and sums as the component c of the complex
 // formulas (i k z contributes +-k times the other component, an exact sign change), so nothing is rounded
 // differently. The pair of a mode sits in adjacent lanes, so a warp's 8-byte loads cover 16 modes contiguously.
-// Per slice each lane streams its 9 values (R_x, R_y, E_z, B_z, j0x, j0y, jkx, jky, jkz) and the slice's
-// coefficients DEPTH slices ahead with per-thread cp.async into its own column of a shared-memory ring; the
-// recurrence touches only registers and that ring. The denominator 1 + (h/4)(D + h/4) k_perp^2 is inverted one
-// slice ahead, off the chain.
+// Per slice each lane streams its 9 values (R_x, R_y, E_z, B_z, j0x, j0y, jkx, jky, jkz) DEPTH slices ahead with per-thread
+// cp.async into its own column of a shared-memory ring; the recurrence touches only registers and that ring. What a slice
+// needs that does not hang on the slice above (R of level s0 with the current's half, R_s; the inverse of the denominator
+// 1 + (h/4)(D + h/4) k_perp^2) is made one slice ahead, in the same straight run of code as the chain of the slice being
+// solved, so that its loads and products fill the chain's gaps: with three or four warps per SM nothing else does.
+// The 128 x 128 x 1024 window (FP64, floor 0.31 ms) 550 -> 508 us, the 64 x 64 x 256 one (33 CTAs' worth of
+// modes, a chain of 256 slices) 105 -> 97 us.
 // T is the storage of E_z, B_z, L and the currents: complex128 (the FP64 form) or complex64 (the mixed form).
 // R stays complex128 and the recurrence runs in FP64 in both forms: its carried values never leave the
 // registers, so the mixed form only rounds what it stores, and the cancellations in curl R and div R that make
@@ -102,7 +105,6 @@ __global__ void __launch_bounds__(BT) k_march(Geo g, cpx* __restrict__ Rx, cpx* 
     double* Rxr = reinterpret_cast<double*>(Rx);
     double* Ryr = reinterpret_cast<double*>(Ry);
     auto cell = [&](int sl, int k) { return ringd + size_t(sl) * slot_doubles(BT) + k * BT + tid; };
-    auto coef = [&](int sl, int k) { return ringd + size_t(sl) * slot_doubles(BT) + MA * BT + k * BT + tid; };
     // ring cells: 0 j0x, 1 jkx, 2 j0y, 3 jky (own), 4 jkz (other), 5 R_x, 6 R_y (own), 7 E_z, 8 B_z (other)
     // PEER: the slab arrays of the rank holding slice n (R_x, R_y, E_z, B_z, L_x, L_y, j0x, j0y, jkx, jky, jkz) and the
     // element offset of this lane's mode in its plane
@@ -112,8 +114,7 @@ __global__ void __launch_bounds__(BT) k_march(Geo g, cpx* __restrict__ Rx, cpx* 
         o = long(n - sp.a[r]) * sp.nkh + g.m0 + ii;
         return reinterpret_cast<double* const*>(sp.arr[r]);
     };
-    auto fetch = [&](int n) {                  // slice n (plane n - a) into its ring slot
-        const int sl = (g.b - 1 - n) % DEPTH;
+    auto fetch = [&](int n, int sl) {          // slice n (plane n - a) into ring slot sl
         if constexpr (PEER) {
             long o;
             double* const* q = peer(n, o);
@@ -138,9 +139,7 @@ __global__ void __launch_bounds__(BT) k_march(Geo g, cpx* __restrict__ Rx, cpx* 
             cp_async_re(cell(sl, 7), Ezr + oth(o));
             cp_async_re(cell(sl, 8), Bzr + oth(o));
         }
-        cp_async8(coef(sl, 0), g.wlo + n);
-        cp_async8(coef(sl, 1), g.whi + n);
-        cp_async8(coef(sl, 2), g.hcg + n + 2);
+        cp_async8(cell(sl, 9), g.wlo + n); cp_async8(cell(sl, 10), g.whi + n); cp_async8(cell(sl, 11), g.hcg + n + 2);
     };
     // upper half-cell of the front slice: plane ns (PEER: the top rank's last half-cell plane)
     const Re* uj0x = j0xr; const Re* ujkx = jkxr; const Re* uj0y = j0yr; const Re* ujky = jkyr; const Re* ujkz = jkzr;
@@ -154,32 +153,31 @@ __global__ void __launch_bounds__(BT) k_march(Geo g, cpx* __restrict__ Rx, cpx* 
     }
     double jxu = double(uj0x[own(ou)]) + double(ujkx[own(ou)]), jyu = double(uj0y[own(ou)]) + double(ujky[own(ou)]);
     double upx = ujkx[own(ou)], upy = ujky[own(ou)], upz = sgn * double(ujkz[oth(ou)]);
-    double pRx = 0, pRy = 0, pE = 0, pB = 0, pLx = 0, pLy = 0;    // level s1 of the slice above: R, E~, B~, L
 #pragma unroll
     for (int q = 0; q < DEPTH; ++q) {
         const int n = g.b - 1 - q;
-        if (n >= g.a) fetch(n);
+        if (n >= g.a) fetch(n, q);
         cp_commit();                          // empty groups keep the count of groups per slice uniform
     }
-    double rden = 0;                          // 1 / denominator of the slice being solved
-    bool have_rden = false;
-    for (int n = g.b - 1; n >= g.a; --n) {
-        cp_wait<DEPTH - 1>();                 // the group of slice n has landed (this lane's own copies)
-        const int sl = (g.b - 1 - n) % DEPTH;
-        const double dx0 = ring_re<Re>(cell(sl, 0)), dxk = ring_re<Re>(cell(sl, 1));
-        const double dy0 = ring_re<Re>(cell(sl, 2)), dyk = ring_re<Re>(cell(sl, 3));
-        const double dzk = sgn * ring_re<Re>(cell(sl, 4));
-        const double rx = *cell(sl, 5), ry = *cell(sl, 6);
+    // the parts of a slice that do not hang on the slice above: R_s (x and y), the lower half-cell's current, 1/denominator
+    struct Pre { double Rsx, Rsy, jxd, jyd, dxk, dyk, dzk, h, rden; };
+    auto prepare = [&](int sl, double jxu_, double jyu_) {
+        Pre p;
+        const double wl = *cell(sl, 9), wu = *cell(sl, 10), h = *cell(sl, 11);
+        p.dxk = ring_re<Re>(cell(sl, 1)); p.dyk = ring_re<Re>(cell(sl, 3)); p.dzk = sgn * ring_re<Re>(cell(sl, 4));
+        p.jxd = ring_re<Re>(cell(sl, 0)) + p.dxk; p.jyd = ring_re<Re>(cell(sl, 2)) + p.dyk;
         const double e = sgn * ring_re<Re>(cell(sl, 7)), b = sgn * ring_re<Re>(cell(sl, 8));
-        const double wl = *coef(sl, 0), wu = *coef(sl, 1), h = *coef(sl, 2);
-        if (!have_rden) rden = 1 / (1 + 0.25 * h * (D + 0.25 * h) * k2);
-        // the next slice's inverse denominator, while this slice's chain runs
-        double rden_next = 0;
-        if (n > g.a) {
-            cp_wait<DEPTH - 2>();
-            const double hn = *coef((sl + 1) % DEPTH, 2);
-            rden_next = 1 / (1 + 0.25 * hn * (D + 0.25 * hn) * k2);
-        }
+        p.Rsx = *cell(sl, 5) + D * (kx * e + ky * b) - D * (wl * p.jxd + wu * jxu_);
+        p.Rsy = *cell(sl, 6) + D * (ky * e - kx * b) - D * (wl * p.jyd + wu * jyu_);
+        p.h = h;
+        p.rden = 1 / (1 + 0.25 * h * (D + 0.25 * h) * k2);
+        return p;
+    };
+    cp_wait<DEPTH - 1>();                     // the group of the front slice has landed (this lane's own copies)
+    Pre p = prepare(0, jxu, jyu);
+    double pRx = 0, pRy = 0, pE = 0, pB = 0, pLx = 0, pLy = 0;    // level s1 of the slice above: R, E~, B~, L
+    int sl = 0;                               // ring slot of slice n
+    for (int n = g.b - 1; n >= g.a; --n) {
         long o = long(n - g.a) * nk + ii;
         Re* sEz = Ezr; Re* sBz = Bzr; Re* sLx = Lxr; Re* sLy = Lyr;
         double* sRx = Rxr; double* sRy = Ryr;
@@ -187,11 +185,10 @@ __global__ void __launch_bounds__(BT) k_march(Geo g, cpx* __restrict__ Rx, cpx* 
             double* const* q = peer(n, o);
             sRx = q[0]; sRy = q[1]; sEz = q[2]; sBz = q[3]; sLx = q[4]; sLy = q[5];
         }
-        const double jxd = dx0 + dxk, jyd = dy0 + dyk;
-        const double Jx = wl * jxd + wu * jxu;
-        const double Jy = wl * jyd + wu * jyu;
-        const double Rsx = rx + D * (kx * e + ky * b) - D * Jx;
-        const double Rsy = ry + D * (ky * e - kx * b) - D * Jy;
+        const int sn = sl + 1 == DEPTH ? 0 : sl + 1;
+        cp_wait<DEPTH - 2>();                 // slice n - 1 has landed (below the rear: a slot that is not used)
+        const Pre q = prepare(sn, p.jxd, p.jyd);
+        const double Rsx = p.Rsx, Rsy = p.Rsy, h = p.h;
         if (n == g.N - 1) {          // front of the window: L = E_z = B_z = 0
             if (live) {
                 sRx[own(o)] = Rsx; sRy[own(o)] = Rsy;
@@ -199,32 +196,32 @@ __global__ void __launch_bounds__(BT) k_march(Geo g, cpx* __restrict__ Rx, cpx* 
             }
             pRx = Rsx; pRy = Rsy; pE = 0; pB = 0; pLx = 0; pLy = 0;
         } else {
-            const double Lsx = pLx - 0.25 * h * (kx * pE - ky * pB) - 0.5 * h * upx;
-            const double Lsy = pLy - 0.25 * h * (kx * pB + ky * pE) - 0.5 * h * upy;
-            const double iCp = 0.5 * ((-kx * (pRy + pLy)) - (-ky * (pRx + pLx)));        // (i C_p)_c
-            const double iQp = -0.5 * (-kx * (pRx - pLx)) + 0.5 * (-ky * (pLy - pRy));    // (i Q_p)_c
-            const double iSB = (-kx * Rsy) + (-kx * Lsy) - (-ky * Rsx) - (-ky * Lsx);     // (i S_B)_c
-            const double iSE = (kx * Rsx) + (-kx * Lsx) + (-ky * Lsy) - (-ky * Rsy);      // (i S_E)_c
-            const double Bn = (pB - 0.5 * h * iCp - 0.25 * h * iSB) * rden;                // (i B_z)_c
-            const double En = (pE - 0.5 * h * iQp - 0.25 * h * iSE - h * upz) * rden;      // (i E_z)_c
+            const double h2 = 0.5 * h, h4 = 0.25 * h;
+            const double Lsx = pLx - h4 * (kx * pE - ky * pB) - h2 * upx;
+            const double Lsy = pLy - h4 * (kx * pB + ky * pE) - h2 * upy;
+            const double iCp = 0.5 * (ky * (pRx + pLx) - kx * (pRy + pLy));               // (i C_p)_c
+            const double iQp = 0.5 * (kx * (pRx - pLx) + ky * (pRy - pLy));               // (i Q_p)_c
+            const double iSB = ky * (Rsx + Lsx) - kx * (Rsy + Lsy);                       // (i S_B)_c
+            const double iSE = kx * (Rsx - Lsx) + ky * (Rsy - Lsy);                       // (i S_E)_c
+            const double Bn = (pB - h2 * iCp - h4 * iSB) * p.rden;                        // (i B_z)_c
+            const double En = (pE - h2 * iQp - h4 * iSE - h * upz) * p.rden;              // (i E_z)_c
             const double nRx = Rsx + D * (kx * En + ky * Bn);
             const double nRy = Rsy + D * (ky * En - kx * Bn);
-            const double nLx = Lsx - 0.25 * h * (kx * En - ky * Bn);
-            const double nLy = Lsy - 0.25 * h * (kx * Bn + ky * En);
+            const double nLx = Lsx - h4 * (kx * En - ky * Bn);
+            const double nLy = Lsy - h4 * (kx * Bn + ky * En);
             if (live) {
                 sEz[oth(o)] = Re(sgn * En); sBz[oth(o)] = Re(sgn * Bn); sRx[own(o)] = nRx; sRy[own(o)] = nRy;
                 sLx[own(o)] = Re(nLx); sLy[own(o)] = Re(nLy);
             }
             pRx = nRx; pRy = nRy; pE = En; pB = Bn; pLx = nLx; pLy = nLy;
         }
-        rden = rden_next;
-        have_rden = n > g.a;
         // the lower half-cell of this slice is the upper one of the next
-        jxu = jxd; jyu = jyd; upx = dxk; upy = dyk; upz = dzk;
-        // refill this slot (its values are consumed above) with the slice DEPTH below
+        upx = p.dxk; upy = p.dyk; upz = p.dzk;
+        // refill this slot (its values were read a slice ago) with the slice DEPTH below
         const int nn = n - DEPTH;
-        if (nn >= g.a) fetch(nn);
+        if (nn >= g.a) fetch(nn, sl);
         cp_commit();
+        p = q; sl = sn;
     }
     cp_wait<0>();
 }
