@@ -12,10 +12,11 @@
 // ring of shared memory with cp.async (16-byte copies, one commit group per slice): several hundred
 // bytes per thread in flight keep HBM busy although one thread owns a whole chain of slices.
 //
-// k_comoving: Simulation::comoving_field for Fourier y (src/sim_fields.cpp:44-151): per mode the
-// tridiagonal system of -(k_perp^2 + gamma^-2 d_zeta^2) psi = rho along zeta (Thomas), then
-// R = -(1 + beta) i k psi, E_z = B_z = 0.
+// k_comoving, k_comoving_pcr, k_comoving_c: Simulation::comoving_field for Fourier y (src/sim_fields.cpp:44-151): per mode
+// the tridiagonal system of -(k_perp^2 + gamma^-2 d_zeta^2) psi = rho along zeta (Thomas; parallel cyclic reduction; the
+// diagonal system of beta = 1), then R = -(1 + beta) i k psi, E_z = B_z = 0.
 #include "g3d_ctx.hpp"
+#include "k_comoving.cuh"
 
 namespace g3d {
 
@@ -327,9 +328,10 @@ void launch_march_f(Ctx& c, double D) {
 static void comoving_launch(Ctx& c, const Geo& g, const cpx* jz, double* cpb, cpx* dpb, cpx* Rx, cpx* Ry, cpx* Ez, cpx* Bz,
                             double beta, double gm2) {
     const int tok = c.prof_begin("comoving");
-    const unsigned blocks = unsigned((g.nkh + 127) / 128);
-    if (blocks) k_comoving<<<blocks, 128, 0, c.stream>>>(g, jz, cpb, dpb, Rx, Ry, Ez, Bz, beta, gm2);
-    c.check_launch("k_comoving");
+    if (!comoving_parallel<cpx>(c, g, jz, Rx, Ry, Ez, Bz, beta, gm2)) {
+        k_comoving<<<unsigned((g.nkh + 127) / 128), 128, 0, c.stream>>>(g, jz, cpb, dpb, Rx, Ry, Ez, Bz, beta, gm2);
+        c.check_launch("k_comoving");
+    }
     c.prof_end(tok);
 }
 void launch_comoving(Ctx& c, double beta, double gm2) {

@@ -12,6 +12,7 @@
 //   * the particles and their push are FP64 (the push reads the float F of both forms).
 #include "g3d_ctx.hpp"
 #include "k_fft.cuh"
+#include "k_comoving.cuh"
 #include "k_dispatch.cuh"
 #include "k_slice_rows.cuh"
 
@@ -519,6 +520,7 @@ void launch_cur_fft_f(Ctx& c, bool keep0) {
     G3D_DISPATCH_N(c.ny, NY, cur_cols_f<NY>(c, keep0));
 }
 void launch_comoving_f(Ctx& c, double beta, double gm2) {
+    if (comoving_parallel<cpxf>(c, c.geo(), c.mx.jkz.p, c.Rx.p, c.Ry.p, c.mx.Ez.p, c.mx.Bz.p, beta, gm2)) return;
     DevBuf<cpx> dp;
     dp.alloc(size_t(c.ns) * c.nkh, c.stream);
     k_comoving_mixed<<<unsigned((c.nkh + 127) / 128), 128, 0, c.stream>>>(c.geo(), c.mx.jkz.p, c.rscratch.p, dp.p, c.Rx.p, c.Ry.p,
