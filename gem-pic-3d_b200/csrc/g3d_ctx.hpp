@@ -334,6 +334,22 @@ __device__ __forceinline__ void fmid_store(const FmidOut& fm, long k, const floa
         o[0] = make_double2(m[0], m[1]); o[1] = make_double2(m[2], m[3]); o[2] = make_double2(m[4], m[5]);
     }
 }
+void launch_rf_rows_f(Ctx& c);              // k_fields.cu: the mixed form's rows of the real fields
+// A complex line of the rows kernel of the currents: two real rows of raw planes. The first ny units of a half-cell plane
+// are j_x + i j_y of a row, the others j_z of the rows 2q and 2q + 1 (the last of an odd ny alone); a, b: the rows exist.
+struct CurUnit {
+    int ca, ra, cb, rb;                      // component and row of the real and of the imaginary part
+    bool a, b;
+    static int count(int ny) { return ny + (ny + 1) / 2; }
+    __device__ CurUnit(int u, int ny) {
+        if (u < ny) { ca = 0; cb = 1; ra = rb = u; a = b = true; return; }
+        ca = cb = 2;
+        ra = 2 * (u - ny); rb = ra + 1;
+        a = ra < ny; b = rb < ny;
+        if (!a) ra = 0;
+        if (!b) rb = 0;
+    }
+};
 void launch_real_fields_slice_fh(Ctx& c, int l, FmidOut fm = FmidOut());
 void launch_ss_lines_fh(Ctx& c, const cpx* T3, cpx* out3, double a2);
 void launch_sp_rows(Ctx& c);                // k_fields.cu

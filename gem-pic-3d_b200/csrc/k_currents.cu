@@ -15,6 +15,7 @@
 #include <algorithm>
 #include "g3d_ctx.hpp"
 #include "k_fft.cuh"
+#include "k_fftr.cuh"
 #include "k_dispatch.cuh"
 #include "k_tma.cuh"
 
@@ -59,28 +60,40 @@ __global__ void __launch_bounds__(DT) k_dep_bound(PartsDev P, long np, Geo g, do
     for (long i = long(blockIdx.x) * DT + threadIdx.x; i < np; i += long(gridDim.x) * DT) dep_bound_one(P, i, g, ia_max, acc);
     block_sum3(acc, part + 3 * blockIdx.x);
 }
-// the bound's three totals into tot[0..2]
-__global__ void __launch_bounds__(DT) k_dep_total(const double* __restrict__ part, double* __restrict__ tot) {
+// scale[c] = 2^e_c, scale[3 + c] = 2^-e_c from the total of component c
+__device__ __forceinline__ void dep_scale_one(double total, int c, double* __restrict__ scale) {
+    const double B = total * (1 + 1e-12) + 1e-300;              // the rounding of the bound's own sum; never 0
+    int x;
+    frexp(B, &x);                                               // B < 2^x
+    const int e = min(62 - x, 1000);
+    scale[c] = ldexp(1.0, e); scale[3 + c] = ldexp(1.0, -e);
+}
+// the bound's three totals into tot[0..2] and, on one rank, the scales (a sharded run sums the totals over the ranks first)
+__global__ void __launch_bounds__(DT) k_dep_total(const double* __restrict__ part, double* __restrict__ tot, double* __restrict__ scale) {
     double acc[3] = {0, 0, 0};
     for (int b = threadIdx.x; b < DB; b += DT)
         for (int k = 0; k < 3; ++k) acc[k] += part[3 * b + k];
     block_sum3(acc, tot);
+    if (scale && threadIdx.x == 0)                              // the thread that wrote them
+        for (int k = 0; k < 3; ++k) dep_scale_one(tot[k], k, scale);
 }
-// scale[c] = 2^e_c, scale[3 + c] = 2^-e_c from the totals
 __global__ void k_dep_scale(const double* __restrict__ tot, double* __restrict__ scale) {
-    if (threadIdx.x < 3) {
-        const double B = tot[threadIdx.x] * (1 + 1e-12) + 1e-300;   // the rounding of the bound's own sum; never 0
-        int x;
-        frexp(B, &x);                                               // B < 2^x
-        const int e = min(62 - x, 1000);
-        scale[threadIdx.x] = ldexp(1.0, e); scale[3 + threadIdx.x] = ldexp(1.0, -e);
-    }
+    if (threadIdx.x < 3) dep_scale_one(tot[threadIdx.x], int(threadIdx.x), scale);
 }
+// A raw value holding the deposit's integer, as a double: its two 32-bit halves placed into the mantissas of 2^52 and 2^84
+// and the offsets taken away (the classic exact construction; the one rounding is the last addition's, as in a
+// conversion). Two FP64 additions: the 64-bit integer conversions ran at a small fraction of that rate and bound the
+// rows kernel, which makes nine of them per point.
+__device__ __forceinline__ double fix_value(double raw) {
+    const double lo = __hiloint2double(0x43300000, __double2loint(raw));                        // 2^52 + low half
+    const double hi = __hiloint2double(0x45300000, __double2hiint(raw) ^ int(0x80000000u));     // 2^84 + 2^32 (high half + 2^31)
+    return (hi - (0x1p84 + 0x1p63 + 0x1p52)) + lo;
+}
+
 // pl: the values of one component (its planes)
 __global__ void k_fix_to_double(double* __restrict__ J, long n, long pl, const double* __restrict__ scale) {
     for (long i = long(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += long(gridDim.x) * blockDim.x) {
-        const long long q = reinterpret_cast<const long long*>(J)[i];
-        J[i] = double(q) * scale[3 + int(i / pl)];
+        J[i] = fix_value(J[i]) * scale[3 + int(i / pl)];
     }
 }
 
@@ -126,76 +139,63 @@ __global__ void __launch_bounds__(256) k_deposit(PartsDev P, const int32_t* __re
 // ---------------------------------------------------------------- zeta filter + FFT along x (rows)
 constexpr int CUR_NT = 128;     // threads of the row kernel
 
-// One CTA = LPC rows of one half-cell plane. The filter reads the three raw planes hk, hk+1, hk+2; the CTAs
-// of neighbouring planes run together (blockIdx.x = rows is the fast index), so each raw plane comes from
-// DRAM once and from L2 for its two neighbours.
+// The filter reads the three raw planes hk, hk+1, hk+2; the CTAs of neighbouring planes run together (blockIdx.x = units
+// is the fast index), so each raw plane comes from DRAM once and from L2 for its two neighbours. A unit of work is a
+// complex line of two real rows (CurUnit): jx + i jy of a row, or jz of two neighbouring rows; its line goes from the raw
+// planes through registers to the half spectra (k_fftr.cuh). 128 x 128 x 1024: 645 -> 205 us (every row's jz a line of
+// its own with no imaginary part, the lines through shared memory at both ends, one element's loads in flight a thread).
 // iscale (the fixed-point deposit's 2^-e_c per component, or null): the raw planes still hold the deposit's 64-bit
-// integers, turned into doubles here as they are read (the same product as k_fix_to_double, without its pass over
+// integers (FIX), turned into doubles here as they are read (the same product as k_fix_to_double, without its pass over
 // the planes)
-template <int NX>
-__global__ void __launch_bounds__(CUR_NT) k_cur_rows(Geo g, const double* __restrict__ J, cpx* __restrict__ TX,
-                                                    cpx* __restrict__ TY, cpx* __restrict__ TZ, int zf,
-                                                    const double* __restrict__ iscale) {
-    using S = FftShape<NX>;
-    constexpr int LPC = CUR_NT / S::T, RS = row_stride<NX>(), H = NX / 2 + 1;
+template <int NX, bool FIX>
+__global__ void __launch_bounds__(CUR_NT, 3) k_cur_rows(Geo g, const double* __restrict__ J, cpx* __restrict__ TX,
+                                                       cpx* __restrict__ TY, cpx* __restrict__ TZ, int zf,
+                                                       const double* __restrict__ iscale) {
+    using S = FftRegPlan<NX>;
+    constexpr int LPC = CUR_NT / S::T, H = NX / 2 + 1;
     extern __shared__ cpx sm[];
-    cpx* a0 = sm;                    // jx + i jy lines
-    cpx* a1 = sm + LPC * RS;         // jz lines
-    const int tid = threadIdx.x, r0 = blockIdx.x * LPC, hk = blockIdx.y;
-    const long nk = g.nk, cpl = long(g.nh) * nk, nkh = long(g.ny) * H;
+    const int r = threadIdx.x / S::T, t = threadIdx.x % S::T, hk = blockIdx.y;
+    const CurUnit un(blockIdx.x * LPC + r, g.ny);
+    const long nk = g.nk, cpl = long(g.nh) * nk;
     const int hw = hk + 1, hc = g.a - 1 + hk;
     const bool live = hc >= 0 && hc <= g.N - 2;
-    double wm = 0.25, w0 = 0.5, wp = 0.25, inv = 1.0;
-    if (zf && !g.zeta_uniform && live) { wm = 0.25 * g.hcg[hc + 1]; w0 = 0.5 * g.hcg[hc + 2]; wp = 0.25 * g.hcg[hc + 3]; inv = g.hcg[hc + 2]; }
-    #pragma unroll 1
-    for (int u_ = 0; u_ < (LPC * NX + CUR_NT - 1) / CUR_NT; ++u_) {
-        const int e = tid + u_ * CUR_NT;
-        if (e >= LPC * NX) break;
-        const int rr = e / NX, p = e - rr * NX, row = r0 + rr;
-        double v[3] = {0, 0, 0};
-        if (live && row < g.ny) {
-            const long i = long(row) * NX + p;
+    // one form of the filter for every grid, so that nothing branches among the loads: no filter is (0, 1, 0)
+    double wm = 0.25, w0 = 0.5, wp = 0.25, rinv = 1.0;
+    if (!zf) { wm = wp = 0.0; w0 = 1.0; }
+    else if (!g.zeta_uniform && live) { wm = 0.25 * g.hcg[hc + 1]; w0 = 0.5 * g.hcg[hc + 2]; wp = 0.25 * g.hcg[hc + 3]; rinv = 1 / g.hcg[hc + 2]; }
+    cpx v[S::E];
+    // the E values of one real row: all its 3 E loads first
+    auto part = [&](int comp, int row, double* out) {
+        const double* Jc = J + comp * cpl + long(hw) * nk + long(row) * NX + t;
+        const double sc = FIX ? iscale[comp] : 1.0;
+        double jm[S::E], j0[S::E], jp[S::E];
 #pragma unroll
-            for (int comp = 0; comp < 3; ++comp) {
-                const double* Jc = J + comp * cpl + i;
-                double jm, j0, jp;
-                if (iscale) {
-                    const long long* Qc = reinterpret_cast<const long long*>(Jc);
-                    const double sc = iscale[comp];
-                    jm = double(__ldg(Qc + (hw - 1) * nk)) * sc; j0 = double(__ldg(Qc + hw * nk)) * sc;
-                    jp = double(__ldg(Qc + (hw + 1) * nk)) * sc;
-                } else {
-                    jm = __ldg(Jc + (hw - 1) * nk); j0 = __ldg(Jc + hw * nk); jp = __ldg(Jc + (hw + 1) * nk);
-                }
-                if (zf && g.zeta_uniform) v[comp] = 0.25 * jm + 0.5 * j0 + 0.25 * jp;
-                else if (zf) v[comp] = (wm * jm + w0 * j0 + wp * jp) / inv;
-                else v[comp] = j0;
-            }
+        for (int j = 0; j < S::E; ++j) { jm[j] = __ldg(Jc - nk + S::T * j); j0[j] = __ldg(Jc + S::T * j); jp[j] = __ldg(Jc + nk + S::T * j); }
+#pragma unroll
+        for (int j = 0; j < S::E; ++j) {
+            if constexpr (FIX) { jm[j] = fix_value(jm[j]) * sc; j0[j] = fix_value(j0[j]) * sc; jp[j] = fix_value(jp[j]) * sc; }
+            out[j] = (wm * jm[j] + w0 * j0[j] + wp * jp[j]) * rinv;
         }
-        a0[rr * RS + p + (p >> 3)] = C(v[0], v[1]);
-        a1[rr * RS + p + (p >> 3)] = C(v[2], 0.0);
+    };
+    if (live) {
+        double re[S::E], im[S::E];
+        part(un.ca, un.ra, re);
+        part(un.cb, un.rb, im);
+#pragma unroll
+        for (int j = 0; j < S::E; ++j) v[j] = C(re[j], un.b ? im[j] : 0.0);
+    } else {
+#pragma unroll
+        for (int j = 0; j < S::E; ++j) v[j] = C(0);
     }
-    __syncthreads();
-    const int r = tid / S::T, t = tid - r * S::T;
-    {
-        decltype(a0) const ls_[2] = {a0, a1};
-        fft_lines<NX, 2>(ls_, RowAddr{r * RS}, t, g.twx);
-    }
-    const long base = long(hk) * nkh;
-    #pragma unroll 1
-    for (int u_ = 0; u_ < (LPC * H + CUR_NT - 1) / CUR_NT; ++u_) {
-        const int e = tid + u_ * CUR_NT;
-        if (e >= LPC * H) break;
-        const int rr = e / H, kx = e - rr * H, row = r0 + rr;
-        if (row >= g.ny) continue;
-        const int km = (NX - kx) % NX;
-        const cpx z = a0[rr * RS + kx + (kx >> 3)], zm = conj(a0[rr * RS + km + (km >> 3)]);
-        const cpx d = z - zm;
-        const long o = base + long(row) * H + kx;
-        TX[o] = 0.5 * (z + zm);
-        TY[o] = 0.5 * C(d.y, -d.x);
-        TZ[o] = a1[rr * RS + kx + (kx >> 3)];
-    }
+    cpx* const line = sm + r * row_stride<NX>();
+    fft_reg<NX>(v, line, t, g.twx);
+    const long base = long(hk) * long(g.ny) * H;
+    cpx* const A = (un.ca == 0 ? TX : TZ) + base + long(un.ra) * H;
+    cpx* const B = (un.cb == 1 ? TY : TZ) + base + long(un.rb) * H;
+    split_pair<NX>(v, line, t, [&](int k, cpx a, cpx b) {
+        if (un.a) A[k] = a;
+        if (un.b) B[k] = b;
+    });
 }
 
 // ---------------------------------------------------------------- FFT along y (columns) + k-filters
@@ -286,11 +286,13 @@ const double* launch_deposit_scale(Ctx& c, double ia_max) {
     double* tot = c.depfix.p + 3 * DB + 6;
     k_dep_bound<<<DB, DT, 0, c.stream>>>(c.parts, c.np, c.geo(), ia_max, c.depfix.p);
     c.check_launch("k_dep_bound");
-    k_dep_total<<<1, DT, 0, c.stream>>>(c.depfix.p, tot);
+    k_dep_total<<<1, DT, 0, c.stream>>>(c.depfix.p, tot, c.sharded() ? nullptr : c.depfix.p + 3 * DB);
     c.check_launch("k_dep_total");
-    c.all_sum(tot, 3, G3D_SUM_F64);                      // a sharded run: the bound of every rank's particles
-    k_dep_scale<<<1, 32, 0, c.stream>>>(tot, c.depfix.p + 3 * DB);
-    c.check_launch("k_dep_scale");
+    if (c.sharded()) {
+        c.all_sum(tot, 3, G3D_SUM_F64);                  // the bound of every rank's particles
+        k_dep_scale<<<1, 32, 0, c.stream>>>(tot, c.depfix.p + 3 * DB);
+        c.check_launch("k_dep_scale");
+    }
     return c.depfix.p + 3 * DB;
 }
 // the fixed-point planes back to doubles (the free-hand deposit, and the raw planes read through the ABI)
@@ -319,15 +321,13 @@ void launch_deposit(Ctx& c) {
 
 template <int NX>
 static void cur_rows(Ctx& c, cpx* TX, cpx* TY, cpx* TZ) {
-    using S = FftShape<NX>;
-    constexpr int LPC = CUR_NT / S::T;
-    const size_t smem = size_t(2) * LPC * row_stride<NX>() * sizeof(cpx);
-    auto kern = k_cur_rows<NX>;
+    constexpr int LPC = CUR_NT / FftRegPlan<NX>::T;
+    const size_t smem = size_t(LPC) * row_stride<NX>() * sizeof(cpx);
+    auto kern = c.jw_fixed ? k_cur_rows<NX, true> : k_cur_rows<NX, false>;
     smem_attr(reinterpret_cast<const void*>(kern), smem);
-    const dim3 grid(unsigned((c.ny + LPC - 1) / LPC), unsigned(c.ns + 1));
+    const dim3 grid(unsigned((CurUnit::count(c.ny) + LPC - 1) / LPC), unsigned(c.ns + 1));
     const int tok = c.prof_begin("cur_rows");
-    kern<<<grid, CUR_NT, smem, c.stream>>>(c.geo(), c.jw.p, TX, TY, TZ, c.P.zeta_filter ? 1 : 0,
-                                           c.jw_fixed ? c.depfix.p + 3 * DB + 3 : nullptr);
+    kern<<<grid, CUR_NT, smem, c.stream>>>(c.geo(), c.jw.p, TX, TY, TZ, c.P.zeta_filter ? 1 : 0, c.depfix.p + 3 * DB + 3);
     c.check_launch("k_cur_rows");
     c.prof_end(tok);
 }

@@ -11,13 +11,15 @@
 //   k_sp_rows      per row: u + i v by one inverse FFT along x, 1/(nx ny), the mask, one forward FFT along x,
 //                  split back into the half spectra of u and v
 //   k_sp_cols_fwd  forward FFT along y, + R_b
-// Real fields: k_rf_cols transforms R_x, R_y, L_x, L_y, E_z, B_z along y (a pair per CTA); k_rf_rows rebuilds R_x + i R_y,
-// L_x + i L_y, E_z + i B_z per row, transforms along x and writes the six float components of F with the
-// reference's combinations (E_x = (r1 + l1)/2, ...).
+// Real fields: k_rf_cols combines R and L into the components' spectra (E_x = (R_x + L_x)/2, ...) and transforms them along
+// y (a pair per CTA); k_rf_rows transforms E_x + i E_y, B_x + i B_y, E_z + i B_z along x, row by row, into the six float
+// components of F.
 #include "g3d_ctx.hpp"
 #include "k_fft.cuh"
+#include "k_fftr.cuh"
 #include "k_dispatch.cuh"
 #include "k_tma.cuh"
+#include "k_psi.cuh"
 #include "k_slice_rows.cuh"
 
 namespace g3d {
@@ -25,47 +27,6 @@ namespace g3d {
 namespace {
 constexpr int NT = 128;    // threads of the row kernels
 constexpr int CW = 8;      // columns per tile of the column kernels
-
-// psi of the slice charge of slice n = a + l at the half-spectrum mode i (reference: the Fourier-y lambda
-// of sim_fields.cpp:176-201)
-__device__ __forceinline__ cpx bound_psi(const Geo& g, const cpx* __restrict__ jz, const cpx* __restrict__ jg, int l, long i,
-                                         double kx, double ky, double g2) {
-    const long nk = g.nkh;
-    const int n = g.a + l;
-    auto half = [&](int hk) -> cpx {
-        if (hk < 0) return jg[i];
-        if (hk > g.ns) return jg[nk + i];
-        return jz[long(hk) * nk + i];
-    };
-    auto rho_at = [&](int dl) -> cpx {
-        const int nn = n + dl;
-        if (nn < 0 || nn > g.N - 1) return C(0);
-        return g.wlo[nn] * half(l + dl) + g.whi[nn] * half(l + dl + 1);
-    };
-    const double hm = g.hcg[n + 1], hp = g.hcg[n + 2];
-    const double cm = 2 / ((hm + hp) * hm), cp_ = 2 / ((hm + hp) * hp);
-    const double k2 = kx * kx + ky * ky;
-    cpx psi = C(0);
-    if (k2 > 0) {
-        const cpx d2 = g2 * (cp_ * rho_at(1) - (cm + cp_) * rho_at(0) + cm * rho_at(-1));
-        psi = (rho_at(0) + d2 / k2) / k2;
-    }
-    return psi;
-}
-
-// Full row z[0..NX) from the half rows A, B (k_x = 0..NX/2) of two real fields: z = A + i B with
-// A(NX - k) = conj A(k), B(NX - k) = conj B(k); stored conjugated for an inverse transform.
-template <int NX>
-__device__ __forceinline__ void full_row_conj(cpx* line, int p, cpx a, cpx b, bool mirror) {
-    // p in 0..NX/2: position p gets a + i b; its mirror NX - p gets conj(a) + i conj(b)
-    const cpx z = C(a.x - b.y, a.y + b.x);
-    line[p + (p >> 3)] = conj(z);
-    if (mirror) {
-        const int q = NX - p;
-        const cpx zm = C(a.x + b.y, -a.y + b.x);                     // conj(a) + i conj(b)
-        line[q + (q >> 3)] = conj(zm);
-    }
-}
 }  // namespace
 
 // ---------------------------------------------------------------- sponge, pass 1: columns (psi, pack, inverse y)
@@ -81,6 +42,7 @@ __global__ void __launch_bounds__(CW * FftShape<NY>::T) k_sp_cols_inv(Geo g, con
     const int l = blockIdx.y, c0 = blockIdx.x * CW, tid = threadIdx.x, nthr = CW * S::T;
     const int H = g.H;
     const long base = long(l) * g.nkh;
+    const BoundPsi<cpx> bp(g, jz, jg, l, g2);
     #pragma unroll
     for (int u_ = 0; u_ < (NY * CW + nthr - 1) / nthr; ++u_) {
         const int e = tid + u_ * nthr;
@@ -90,7 +52,7 @@ __global__ void __launch_bounds__(CW * FftShape<NY>::T) k_sp_cols_inv(Geo g, con
         if (kxi < H) {
             const long i = long(p) * H + kxi, o = base + i;
             const double kx = g.kxd[kxi], ky = g.kyd[p];
-            const cpx psi = bound_psi(g, jz, jg, l, i, kx, ky, g2);
+            const cpx psi = bp.at(i, kx * kx + ky * ky);
             PSI[o] = psi;
             u = Rx[o] - (-opb * ik(kx, psi));
             v = Ry[o] - (-opb * ik(ky, psi));
@@ -134,6 +96,7 @@ __global__ void __launch_bounds__(8 * FftShape<NY>::T) k_sp_cols_inv_tma(Geo g, 
     cpx* s1 = s0 + NY * 8;
     const int idx[2] = {0, 1};
     cpx* const dst[2] = {s0, s1};
+    const BoundPsi<cpx> bp(g, jz, jg, l, g2);
     if (!tma_tiles<NY>(maps, idx, 2, dst, c0, l * g.ny, &bar, &ok, wt)) return;
     #pragma unroll
     for (int u_ = 0; u_ < (NY * 8 + nthr - 1) / nthr; ++u_) {
@@ -144,7 +107,7 @@ __global__ void __launch_bounds__(8 * FftShape<NY>::T) k_sp_cols_inv_tma(Geo g, 
         if (kxi < H) {
             const long i = long(p) * H + kxi, o = base + i;
             const double kx = g.kxd[kxi], ky = g.kyd[p];
-            const cpx psi = bound_psi(g, jz, jg, l, i, kx, ky, g2);
+            const cpx psi = bp.at(i, kx * kx + ky * ky);
             PSI[o] = psi;
             u = s0[e] - (-opb * ik(kx, psi));
             v = s1[e] - (-opb * ik(ky, psi));
@@ -171,52 +134,36 @@ __global__ void __launch_bounds__(8 * FftShape<NY>::T) k_sp_cols_inv_tma(Geo g, 
 }
 
 // ---------------------------------------------------------------- sponge, pass 2: rows (inverse x, mask, forward x)
+// The line stays in registers from the load through both transforms (k_fftr.cuh).
 template <int NX>
-__global__ void __launch_bounds__(NT) k_sp_rows(Geo g, cpx* __restrict__ U, cpx* __restrict__ V) {
-    using S = FftShape<NX>;
-    constexpr int LPC = NT / S::T, RS = row_stride<NX>(), H = NX / 2 + 1;
+__global__ void __launch_bounds__(NT, 3) k_sp_rows(Geo g, cpx* __restrict__ U, cpx* __restrict__ V) {
+    using S = FftRegPlan<NX>;
+    constexpr int LPC = NT / S::T, H = NX / 2 + 1;
     extern __shared__ cpx sm[];
-    const int l = blockIdx.y, r0 = blockIdx.x * LPC, tid = threadIdx.x;
-    const long base = long(l) * g.nkh;
-    #pragma unroll
-    for (int u_ = 0; u_ < (LPC * H + NT - 1) / NT; ++u_) {
-        const int e = tid + u_ * NT;
-        if (e >= LPC * H) break;
-        const int r = e / H, p = e - r * H, row = r0 + r;
-        cpx a = C(0), b = C(0);
-        if (row < g.ny) { const long o = base + long(row) * H + p; a = U[o]; b = V[o]; }
-        full_row_conj<NX>(sm + r * RS, p, a, b, p > 0 && p < NX / 2);
+    const int l = blockIdx.y, r = threadIdx.x / S::T, t = threadIdx.x % S::T, row = blockIdx.x * LPC + r;
+    const bool on = row < g.ny;
+    const long o = long(l) * g.nkh + long(on ? row : 0) * H;
+    cpx* const line = sm + r * row_stride<NX>();
+    cpx v[S::E];
+#pragma unroll
+    for (int j = 0; j < S::E; ++j) {
+        const int k = t + S::T * j;
+        const bool up = k > NX / 2;
+        const long i = o + (up ? NX - k : k);
+        v[j] = pair_conj(up, U[i], V[i]);
     }
-    __syncthreads();
-    const int r = tid / S::T, t = tid - r * S::T;
-    fft_line<NX>(sm, RowAddr{r * RS}, t, g.twx);
+    fft_reg<NX>(v, line, t, g.twx);
     const double s = g.yf ? 1.0 / double(g.nk) : 1.0 / double(g.nx);   // free-hand y: rows only, 1/nx
-    #pragma unroll
-    for (int u_ = 0; u_ < (LPC * NX + NT - 1) / NT; ++u_) {
-        const int e = tid + u_ * NT;
-        if (e >= LPC * NX) break;
-        const int rr = e / NX, p = e - rr * NX, row = r0 + rr;
-        const int q = rr * RS + p + (p >> 3);
-        const cpx z = s * conj(sm[q]);                                  // u + i v in real space
-        const double mx = g.maskx[p];
-        const double mn = row < g.ny ? g.masky_n[row] : 0.0, mh = row < g.ny ? g.masky_h[row] : 0.0;
-        sm[q] = C(mx * mn * z.x, mx * mh * z.y);
+    const double mn = s * g.masky_n[on ? row : 0], mh = s * g.masky_h[on ? row : 0];
+#pragma unroll
+    for (int j = 0; j < S::E; ++j) {                                   // u + i v in real space, masked
+        const double mx = g.maskx[t + S::T * j];
+        v[j] = C(mx * mn * v[j].x, -(mx * mh * v[j].y));
     }
-    __syncthreads();
-    fft_line<NX>(sm, RowAddr{r * RS}, t, g.twx);
-    #pragma unroll
-    for (int u_ = 0; u_ < (LPC * H + NT - 1) / NT; ++u_) {
-        const int e = tid + u_ * NT;
-        if (e >= LPC * H) break;
-        const int rr = e / H, p = e - rr * H, row = r0 + rr;
-        if (row >= g.ny) continue;
-        const int pm = (NX - p) % NX;
-        const cpx z = sm[rr * RS + p + (p >> 3)], zm = conj(sm[rr * RS + pm + (pm >> 3)]);
-        const cpx d = z - zm;
-        const long o = base + long(row) * H + p;
-        U[o] = 0.5 * (z + zm);
-        V[o] = 0.5 * C(d.y, -d.x);
-    }
+    fft_reg<NX>(v, line, t, g.twx);
+    split_pair<NX>(v, line, t, [&](int k, cpx a, cpx b) {
+        if (on) { U[o + k] = a; V[o + k] = b; }
+    });
 }
 
 // ---------------------------------------------------------------- sponge, pass 3: columns (forward y, + R_b)
@@ -296,9 +243,18 @@ __global__ void __launch_bounds__(8 * FftShape<NY>::T) k_sp_cols_fwd_tma(Geo g, 
 }
 
 // ---------------------------------------------------------------- real fields: columns (inverse y of the six spectra)
-// blockIdx.z picks the pair (R_x, R_y), (L_x, L_y) or (E_z, B_z): two fields per CTA keep the shared memory small
-// enough for several CTAs per SM, so loads of one CTA overlap the transforms of another.
-template <int NY, int CWT>
+// Two fields per CTA (blockIdx.z) keep the shared memory small enough for several CTAs per SM, so loads of one CTA overlap
+// the transforms of another. COMB: the pairs (R_x, L_x), (R_y, L_y), (E_z, B_z) come out as the real fields' own
+// spectra, (R + L)/2 and (R - L)/2: W0..W5 = E_x, E_y, B_x, B_y, E_z, B_z, so that each line of the rows kernel is two
+// components of F. Else (one slice of the plasma march, whose rows combine) as they are: R_x, R_y, L_x, L_y, E_z, B_z.
+template <bool COMB, class T>
+__device__ __forceinline__ void rf_combine(int pr, T& a, T& b) {
+    typedef typename RealOf<T>::type Re;
+    if (!COMB || pr == 2) return;
+    const T s = Re(0.5) * (a + b), d = pr == 0 ? Re(0.5) * (a - b) : Re(0.5) * (b - a);   // B_y = (R_x - L_x)/2, B_x = (L_y - R_y)/2
+    a = s; b = d;
+}
+template <int NY, int CWT, bool COMB>
 __global__ void __launch_bounds__(CWT * FftShape<NY>::T) k_rf_cols(Geo g, const cpx* __restrict__ Rx, const cpx* __restrict__ Ry,
                                                                   const cpx* __restrict__ Lx, const cpx* __restrict__ Ly,
                                                                   const cpx* __restrict__ Ez, const cpx* __restrict__ Bz,
@@ -310,10 +266,10 @@ __global__ void __launch_bounds__(CWT * FftShape<NY>::T) k_rf_cols(Geo g, const 
     const int l = l0 + blockIdx.y, c0 = blockIdx.x * CWT, tid = threadIdx.x, nthr = CWT * S::T, pr = blockIdx.z;
     const int H = g.H;
     const long base = long(l) * g.nkh;
-    const cpx* in0 = pr == 0 ? Rx : pr == 1 ? Lx : Ez;
-    const cpx* in1 = pr == 0 ? Ry : pr == 1 ? Ly : Bz;
-    cpx* out0 = pr == 0 ? W0 : pr == 1 ? W2 : W4;
-    cpx* out1 = pr == 0 ? W1 : pr == 1 ? W3 : W5;
+    const cpx* in0 = pr == 2 ? Ez : COMB ? (pr == 0 ? Rx : Ry) : (pr == 0 ? Rx : Lx);
+    const cpx* in1 = pr == 2 ? Bz : COMB ? (pr == 0 ? Lx : Ly) : (pr == 0 ? Ry : Ly);
+    cpx* out0 = pr == 2 ? W4 : COMB ? (pr == 0 ? W0 : W1) : (pr == 0 ? W0 : W2);
+    cpx* out1 = pr == 2 ? W5 : COMB ? (pr == 0 ? W3 : W2) : (pr == 0 ? W1 : W3);
     cpx* s0 = sm;
     cpx* s1 = sm + ColTile<NY, CWT>::size;
     #pragma unroll
@@ -322,8 +278,11 @@ __global__ void __launch_bounds__(CWT * FftShape<NY>::T) k_rf_cols(Geo g, const 
         if (e >= NY * CWT) break;
         const int p = e / CWT, c = e - p * CWT, kxi = c0 + c;
         const long o = base + long(p) * H + kxi;
-        s0[ColTile<NY, CWT>::at(p, c)] = kxi < H ? conj(in0[o]) : C(0);
-        s1[ColTile<NY, CWT>::at(p, c)] = kxi < H ? conj(in1[o]) : C(0);
+        cpx a = C(0), b = C(0);
+        if (kxi < H) { a = in0[o]; b = in1[o]; }
+        rf_combine<COMB>(pr, a, b);
+        s0[ColTile<NY, CWT>::at(p, c)] = conj(a);
+        s1[ColTile<NY, CWT>::at(p, c)] = conj(b);
     }
     __syncthreads();
     const int c = tid % CWT, t = tid / CWT;
@@ -344,7 +303,7 @@ __global__ void __launch_bounds__(CWT * FftShape<NY>::T) k_rf_cols(Geo g, const 
 }
 
 // The same transforms of the whole window with the tiles loaded by the TMA (k_tma.cuh): the 8-column tiles of the
-// pair land row-major in shared memory, are conjugated in place, transformed along their columns (stride 8) and
+// pair land row-major in shared memory, are combined (COMB above) and conjugated in place, transformed along their columns (stride 8) and
 // written back conjugated; maps 0..5 are R_x, R_y, L_x, L_y, E_z, B_z.
 template <int NY>
 __global__ void __launch_bounds__(8 * FftShape<NY>::T) k_rf_cols_tma(Geo g, const __grid_constant__ TileMaps maps,
@@ -361,12 +320,16 @@ __global__ void __launch_bounds__(8 * FftShape<NY>::T) k_rf_cols_tma(Geo g, cons
     const long base = long(l) * g.nkh;
     cpx* s0 = reinterpret_cast<cpx*>(smraw + ((128 - (smem_addr(smraw) & 127)) & 127));
     cpx* s1 = s0 + NY * 8;
-    cpx* out0 = pr == 0 ? W0 : pr == 1 ? W2 : W4;
-    cpx* out1 = pr == 0 ? W1 : pr == 1 ? W3 : W5;
-    const int idx[2] = {2 * pr, 2 * pr + 1};
+    cpx* out0 = pr == 0 ? W0 : pr == 1 ? W1 : W4;
+    cpx* out1 = pr == 0 ? W3 : pr == 1 ? W2 : W5;
+    const int idx[2] = {pr == 2 ? 4 : pr, pr == 2 ? 5 : pr + 2};
     cpx* const dst[2] = {s0, s1};
     if (!tma_tiles<NY>(maps, idx, 2, dst, c0, l * g.ny, &bar, &ok, wt)) return;
-    for (int e = tid; e < NY * 8; e += nthr) { s0[e] = conj(s0[e]); s1[e] = conj(s1[e]); }
+    for (int e = tid; e < NY * 8; e += nthr) {
+        cpx a = s0[e], b = s1[e];
+        rf_combine<true>(pr, a, b);
+        s0[e] = conj(a); s1[e] = conj(b);
+    }
     __syncthreads();
     const int c = tid % 8, t = tid / 8;
     {
@@ -386,64 +349,65 @@ __global__ void __launch_bounds__(8 * FftShape<NY>::T) k_rf_cols_tma(Geo g, cons
 }
 
 // ---------------------------------------------------------------- real fields: rows (inverse x, F)
-// (one slice of the plasma march: k_rf_row_slice, k_slice_rows.cuh)
-template <int NX>
-__global__ void __launch_bounds__(NT) k_rf_rows(Geo g, const cpx* __restrict__ W0, const cpx* __restrict__ W1,
-                                               const cpx* __restrict__ W2, const cpx* __restrict__ W3,
-                                               const cpx* __restrict__ W4, const cpx* __restrict__ W5, float* __restrict__ F,
-                                               double* __restrict__ Fd) {
-    using S = FftShape<NX>;
-    constexpr int LPC = NT / S::T, RS = row_stride<NX>(), H = NX / 2 + 1;
-    extern __shared__ cpx sm[];
-    cpx* a0 = sm;
-    cpx* a1 = sm + LPC * RS;
-    cpx* a2 = sm + 2 * LPC * RS;
-    const int l = blockIdx.y, r0 = blockIdx.x * LPC, tid = threadIdx.x;
-    const long base = long(l) * g.nkh;
-    const long fpl = long(g.ns + 2) * g.nk, fbase = long(l) * g.nk;
-    constexpr int EO = (LPC * NX + NT - 1) / NT;                    // output elements of a thread
-    #pragma unroll
-    for (int u_ = 0; u_ < (LPC * H + NT - 1) / NT; ++u_) {      // unrolled: the loads of all elements in flight
-        const int e = tid + u_ * NT;
-        if (e >= LPC * H) continue;
-        const int r = e / H, p = e - r * H, row = r0 + r;
-        cpx v[6] = {C(0), C(0), C(0), C(0), C(0), C(0)};
-        if (row < g.ny) {
-            const long o = base + long(row) * H + p;
-            v[0] = W0[o]; v[1] = W1[o]; v[2] = W2[o]; v[3] = W3[o]; v[4] = W4[o]; v[5] = W5[o];
-        }
-        const bool mirror = p > 0 && p < NX / 2;
-        full_row_conj<NX>(a0 + r * RS, p, v[0], v[1], mirror);
-        full_row_conj<NX>(a1 + r * RS, p, v[2], v[3], mirror);
-        full_row_conj<NX>(a2 + r * RS, p, v[4], v[5], mirror);
-    }
-    __syncthreads();
-    const int r = tid / S::T, t = tid - r * S::T;
-    {
-        decltype(a0) const ls_[3] = {a0, a1, a2};
-        fft_lines<NX, 3>(ls_, RowAddr{r * RS}, t, g.twx);
-    }
-    const double s = g.yf ? 1.0 / double(g.nk) : 1.0 / double(g.nx);   // free-hand y: rows only, 1/nx
-    #pragma unroll
-    for (int u_ = 0; u_ < EO; ++u_) {
-        const int e = tid + u_ * NT;
-        if (e >= LPC * NX) continue;
-        const int rr = e / NX, p = e - rr * NX, row = r0 + rr;
-        if (row >= g.ny) continue;
-        const int q = rr * RS + p + (p >> 3);
-        const cpx z1 = s * conj(a0[q]), z2 = s * conj(a1[q]), z3 = s * conj(a2[q]);
-        const long idx = fbase + long(row) * NX + p;
-        const double r1 = z1.x, r2 = z1.y, l1 = z2.x, l2 = z2.y;
-        const float fv[6] = {float(0.5 * (r1 + l1)), float(0.5 * (r2 + l2)), float(z3.x),    // E_x, E_y, E_z
-                             float(0.5 * (l2 - r2)), float(0.5 * (r1 - l1)), float(z3.y)};  // B_x, B_y, B_z
+// One line per group of threads (blockIdx.z): E_x + i E_y, B_x + i B_y or E_z + i B_z of a row, from global memory through
+// registers to F (k_fftr.cuh). COMB: the input are the rows of R_x, R_y, L_x, L_y, E_z, B_z (free-hand y, no columns pass)
+// and are combined here. (One slice of the plasma march: k_rf_row_slice, k_slice_rows.cuh.)
+template <int NX, class T, bool COMB>
+__global__ void __launch_bounds__(NT, 3) k_rf_rows(Geo g, const T* __restrict__ tw, const T* __restrict__ W0, const T* __restrict__ W1,
+                                                  const T* __restrict__ W2, const T* __restrict__ W3, const T* __restrict__ W4,
+                                                  const T* __restrict__ W5, float* __restrict__ F, double* __restrict__ Fd) {
+    typedef typename RealOf<T>::type Re;
+    using S = FftRegPlan<NX>;
+    constexpr int LPC = NT / S::T, H = NX / 2 + 1;
+    extern __shared__ __align__(16) unsigned char smr[];
+    const int l = blockIdx.y, pr = blockIdx.z, r = threadIdx.x / S::T, t = threadIdx.x % S::T, row = blockIdx.x * LPC + r;
+    const bool on = row < g.ny;
+    const long o = long(l) * g.nkh + long(on ? row : 0) * H;
+    const T* a0 = pr == 0 ? W0 : pr == 1 ? (COMB ? W1 : W2) : W4;       // COMB: line 0 R_x, R_y and L_x, L_y; line 1 R_y, R_x
+    const T* b0 = pr == 0 ? W1 : pr == 1 ? (COMB ? W0 : W3) : W5;
+    const T* a1 = pr == 0 ? W2 : W3;                                   // and L_y, L_x
+    const T* b1 = pr == 0 ? W3 : W2;
+    T v[S::E];
 #pragma unroll
-        for (int comp = 0; comp < 6; ++comp) F[comp * fpl + idx] = fv[comp];
-        if (Fd) {                                      // exact fields: the same values before the rounding
-            Fd[0 * fpl + idx] = 0.5 * (r1 + l1); Fd[1 * fpl + idx] = 0.5 * (r2 + l2);
-            Fd[3 * fpl + idx] = 0.5 * (l2 - r2); Fd[4 * fpl + idx] = 0.5 * (r1 - l1);
-            Fd[2 * fpl + idx] = z3.x; Fd[5 * fpl + idx] = z3.y;
+    for (int j = 0; j < S::E; ++j) {
+        const int k = t + S::T * j;
+        const bool up = k > NX / 2;
+        const long i = o + (up ? NX - k : k);
+        T a = __ldg(a0 + i), b = __ldg(b0 + i);
+        if (COMB && pr < 2) {
+            const T c = __ldg(a1 + i), d = __ldg(b1 + i);
+            if (pr == 0) { a = Re(0.5) * (a + c); b = Re(0.5) * (b + d); }      // E_x, E_y
+            else { a = Re(0.5) * (c - a); b = Re(0.5) * (b - d); }              // B_x = (L_y - R_y)/2, B_y = (R_x - L_x)/2
         }
+        v[j] = pair_conj(up, a, b);
     }
+    fft_reg<NX>(v, reinterpret_cast<T*>(smr) + r * row_stride<NX>(), t, tw);
+    if (!on) return;
+    const Re s = g.yf ? Re(1) / Re(g.nk) : Re(1) / Re(g.nx);            // free-hand y: rows only, 1/nx
+    const long fpl = long(g.ns + 2) * g.nk, idx = long(l) * g.nk + long(row) * NX;
+    const int ca = pr == 0 ? 0 : pr == 1 ? 3 : 2, cb = pr == 0 ? 1 : pr == 1 ? 4 : 5;
+#pragma unroll
+    for (int j = 0; j < S::E; ++j) {
+        const long i = idx + t + S::T * j;
+        const Re x = s * v[j].x, y = -(s * v[j].y);
+        F[ca * fpl + i] = float(x); F[cb * fpl + i] = float(y);
+        if (Fd) { Fd[ca * fpl + i] = double(x); Fd[cb * fpl + i] = double(y); }    // exact fields: before the rounding
+    }
+}
+template <int NX, class T, bool COMB>
+static void rf_rows(Ctx& c, const T* tw, const T* W0, const T* W1, const T* W2, const T* W3, const T* W4, const T* W5, double* Fd) {
+    constexpr int LPC = NT / FftRegPlan<NX>::T;
+    const size_t smem = size_t(LPC) * row_stride<NX>() * sizeof(T);
+    auto kern = k_rf_rows<NX, T, COMB>;
+    smem_attr(reinterpret_cast<const void*>(kern), smem);
+    const int tok = c.prof_begin("real_rows");
+    kern<<<dim3(unsigned((c.ny + LPC - 1) / LPC), unsigned(c.ns), 3), NT, smem, c.stream>>>(c.geo(), tw, W0, W1, W2, W3, W4, W5, c.F.p, Fd);
+    c.check_launch("k_rf_rows");
+    c.prof_end(tok);
+}
+void launch_rf_rows_f(Ctx& c) {                       // the mixed form's (k_mixed.cu)
+    auto& m = c.mx;
+    G3D_DISPATCH_N(c.nx, NX, (rf_rows<NX, cpxf, false>(c, m.twx.p, m.W[0].p, m.W[1].p, m.W[2].p, m.W[3].p, m.W[4].p, m.W[5].p, nullptr)));
 }
 
 // ---------------------------------------------------------------- launchers
@@ -478,7 +442,7 @@ static void sp_cols_inv(Ctx& c) {
 }
 template <int NX>
 static void sp_rows(Ctx& c) {
-    constexpr int LPC = NT / FftShape<NX>::T;
+    constexpr int LPC = NT / FftRegPlan<NX>::T;
     const size_t smem = size_t(LPC) * row_stride<NX>() * sizeof(cpx);
     allow_smem(k_sp_rows<NX>, smem);
     const int tok = c.prof_begin("sponge_rows");
@@ -516,12 +480,12 @@ void launch_sponge(Ctx& c) {
 }
 
 // one slice (the plasma march): tiles of 2 columns, so that 3 x 65 CTAs spread the slice's latency over the SMs
-template <int NY, int CWT>
+template <int NY, int CWT, bool COMB>
 static void rf_cols_w(Ctx& c, int l0, int nl) {
     const size_t smem = size_t(2) * ColTile<NY, CWT>::size * sizeof(cpx);
-    allow_smem(k_rf_cols<NY, CWT>, smem);
+    allow_smem(k_rf_cols<NY, CWT, COMB>, smem);
     const int tok = c.prof_begin(nl == 1 ? "real_cols_slice" : "real_cols");
-    k_rf_cols<NY, CWT><<<dim3(unsigned((c.H + CWT - 1) / CWT), unsigned(nl), 3), CWT * FftShape<NY>::T, smem, c.stream>>>(
+    k_rf_cols<NY, CWT, COMB><<<dim3(unsigned((c.H + CWT - 1) / CWT), unsigned(nl), 3), CWT * FftShape<NY>::T, smem, c.stream>>>(
         c.geo(), c.Rx.p, c.Ry.p, c.Lx.p, c.Ly.p, c.Ez.p, c.Bz.p, c.W[0].p, c.W[1].p, c.W[2].p, c.W[3].p, c.W[4].p, c.W[5].p, l0);
     c.check_launch("k_rf_cols");
     c.prof_end(tok);
@@ -544,30 +508,19 @@ static void rf_cols_tma(Ctx& c, int l0, int nl) {
 }
 template <int NY>
 static void rf_cols(Ctx& c, int l0, int nl) {
-    if (nl == 1) { rf_cols_w<NY, 2>(c, l0, nl); return; }
+    if (nl == 1) { rf_cols_w<NY, 2, false>(c, l0, nl); return; }
     if constexpr (NY <= 256 && (NY & (NY - 1)) == 0) {
         if (c.use_tma && rf_maps(c)) { rf_cols_tma<NY>(c, l0, nl); return; }
     }
-    rf_cols_w<NY, CW>(c, l0, nl);
-}
-template <int NX>
-static void rf_rows(Ctx& c, const cpx* W0, const cpx* W1, const cpx* W2, const cpx* W3, const cpx* W4, const cpx* W5) {
-    constexpr int LPC = NT / FftShape<NX>::T;
-    const size_t smem = size_t(3) * LPC * row_stride<NX>() * sizeof(cpx);
-    allow_smem(k_rf_rows<NX>, smem);
-    const int tok = c.prof_begin("real_rows");
-    k_rf_rows<NX><<<dim3(unsigned((c.ny + LPC - 1) / LPC), unsigned(c.ns)), NT, smem, c.stream>>>(c.geo(), W0, W1, W2, W3, W4, W5, c.F.p,
-                                                                                                  c.Fd.p);
-    c.check_launch("k_rf_rows");
-    c.prof_end(tok);
+    rf_cols_w<NY, CW, true>(c, l0, nl);
 }
 void launch_real_fields(Ctx& c) {
     G3D_DISPATCH_N(c.ny, NY, rf_cols<NY>(c, 0, c.ns));
-    G3D_DISPATCH_N(c.nx, NX, rf_rows<NX>(c, c.W[0].p, c.W[1].p, c.W[2].p, c.W[3].p, c.W[4].p, c.W[5].p));
+    G3D_DISPATCH_N(c.nx, NX, (rf_rows<NX, cpx, false>(c, c.twx.p, c.W[0].p, c.W[1].p, c.W[2].p, c.W[3].p, c.W[4].p, c.W[5].p, c.Fd.p)));
 }
 // free-hand y: the spectra are already real in y; one inverse transform along x per row of R, L and E_z + i B_z
 void launch_real_fields_fh(Ctx& c) {
-    G3D_DISPATCH_N(c.nx, NX, rf_rows<NX>(c, c.Rx.p, c.Ry.p, c.Lx.p, c.Ly.p, c.Ez.p, c.Bz.p));
+    G3D_DISPATCH_N(c.nx, NX, (rf_rows<NX, cpx, true>(c, c.twx.p, c.Rx.p, c.Ry.p, c.Lx.p, c.Ly.p, c.Ez.p, c.Bz.p, c.Fd.p)));
 }
 void launch_real_fields_slice_fh(Ctx& c, int l, FmidOut fm) {
     G3D_DISPATCH_N(c.nx, NX, (rf_row_slice<NX, cpx, false>(c, c.twx.p, c.Rx.p, c.Ry.p, c.Lx.p, c.Ly.p, c.Ez.p, c.Bz.p, l, l, c.Fd.p, fm)));

@@ -12,7 +12,9 @@
 //   * the particles and their push are FP64 (the push reads the float F of both forms).
 #include "g3d_ctx.hpp"
 #include "k_fft.cuh"
+#include "k_fftr.cuh"
 #include "k_comoving.cuh"
+#include "k_psi.cuh"
 #include "k_dispatch.cuh"
 #include "k_slice_rows.cuh"
 
@@ -73,62 +75,51 @@ __global__ void __launch_bounds__(256) k_deposit_f(PartsDev P, const int32_t* __
 }
 
 // ---------------------------------------------------------------- zeta filter + FFT along x (FP32)
+// Units and packing as k_cur_rows (k_currents.cu)
 template <int NX>
-__global__ void __launch_bounds__(NT) k_cur_rows_f(Geo g, const float* __restrict__ J, const cpxf* __restrict__ tw,
-                                                  cpxf* __restrict__ TX, cpxf* __restrict__ TY, cpxf* __restrict__ TZ, int zf) {
-    using S = FftShape<NX>;
-    constexpr int LPC = NT / S::T, RS = row_stride<NX>(), H = NX / 2 + 1;
+__global__ void __launch_bounds__(NT, 5) k_cur_rows_f(Geo g, const float* __restrict__ J, const cpxf* __restrict__ tw,
+                                                     cpxf* __restrict__ TX, cpxf* __restrict__ TY, cpxf* __restrict__ TZ, int zf) {
+    using S = FftRegPlan<NX>;
+    constexpr int LPC = NT / S::T, H = NX / 2 + 1;
     extern __shared__ cpxf smf[];
-    cpxf* a0 = smf;
-    cpxf* a1 = smf + LPC * RS;
-    const int tid = threadIdx.x, r0 = blockIdx.x * LPC, hk = blockIdx.y;
-    const long nk = g.nk, cpl = long(g.nh) * nk, nkh = long(g.ny) * H;
+    const int r = threadIdx.x / S::T, t = threadIdx.x % S::T, hk = blockIdx.y;
+    const CurUnit un(blockIdx.x * LPC + r, g.ny);
+    const long nk = g.nk, cpl = long(g.nh) * nk;
     const int hw = hk + 1, hc = g.a - 1 + hk;
     const bool live = hc >= 0 && hc <= g.N - 2;
     float wm = 0.25f, w0 = 0.5f, wp = 0.25f, inv = 1.0f;
     if (zf && !g.zeta_uniform && live) {
         wm = float(0.25 * g.hcg[hc + 1]); w0 = float(0.5 * g.hcg[hc + 2]); wp = float(0.25 * g.hcg[hc + 3]); inv = float(g.hcg[hc + 2]);
     }
-    #pragma unroll
-    for (int u_ = 0; u_ < (LPC * NX + NT - 1) / NT; ++u_) {
-        const int e = tid + u_ * NT;
-        if (e >= LPC * NX) break;
-        const int rr = e / NX, p = e - rr * NX, row = r0 + rr;
-        float v[3] = {0, 0, 0};
-        if (live && row < g.ny) {
-            const long i = long(row) * NX + p;
+    cpxf v[S::E];
+    auto part = [&](int comp, int row, float* out) {                   // all the loads of a row first
+        const float* Jc = J + comp * cpl + long(hw) * nk + long(row) * NX + t;
+        float jm[S::E], j0[S::E], jp[S::E];
 #pragma unroll
-            for (int comp = 0; comp < 3; ++comp) {
-                const float* Jc = J + comp * cpl + i;
-                const float jm = __ldg(Jc + (hw - 1) * nk), j0 = __ldg(Jc + hw * nk), jp = __ldg(Jc + (hw + 1) * nk);
-                if (zf) v[comp] = sum3c(__fmul_rn(wm, jm), __fmul_rn(w0, j0), __fmul_rn(wp, jp)) / inv;
-                else v[comp] = j0;
-            }
-        }
-        a0[rr * RS + p + (p >> 3)] = Cf(v[0], v[1]);
-        a1[rr * RS + p + (p >> 3)] = Cf(v[2], 0.0f);
+        for (int j = 0; j < S::E; ++j) { jm[j] = __ldg(Jc - nk + S::T * j); j0[j] = __ldg(Jc + S::T * j); jp[j] = __ldg(Jc + nk + S::T * j); }
+#pragma unroll
+        for (int j = 0; j < S::E; ++j)
+            out[j] = zf ? sum3c(__fmul_rn(wm, jm[j]), __fmul_rn(w0, j0[j]), __fmul_rn(wp, jp[j])) / inv : j0[j];
+    };
+    if (live) {
+        float re[S::E], im[S::E];
+        part(un.ca, un.ra, re);
+        part(un.cb, un.rb, im);
+#pragma unroll
+        for (int j = 0; j < S::E; ++j) v[j] = Cf(re[j], un.b ? im[j] : 0.f);
+    } else {
+#pragma unroll
+        for (int j = 0; j < S::E; ++j) v[j] = Cf(0);
     }
-    __syncthreads();
-    const int r = tid / S::T, t = tid - r * S::T;
-    {
-        decltype(a0) const ls_[2] = {a0, a1};
-        fft_lines<NX, 2>(ls_, RowAddr{r * RS}, t, tw);
-    }
-    const long base = long(hk) * nkh;
-    #pragma unroll
-    for (int u_ = 0; u_ < (LPC * H + NT - 1) / NT; ++u_) {
-        const int e = tid + u_ * NT;
-        if (e >= LPC * H) break;
-        const int rr = e / H, kx = e - rr * H, row = r0 + rr;
-        if (row >= g.ny) continue;
-        const int km = (NX - kx) % NX;
-        const cpxf z = a0[rr * RS + kx + (kx >> 3)], zm = conj(a0[rr * RS + km + (km >> 3)]);
-        const cpxf d = z - zm;
-        const long o = base + long(row) * H + kx;
-        TX[o] = 0.5f * (z + zm);
-        TY[o] = 0.5f * Cf(d.y, -d.x);
-        TZ[o] = a1[rr * RS + kx + (kx >> 3)];
-    }
+    cpxf* const line = smf + r * row_stride<NX>();
+    fft_reg<NX>(v, line, t, tw);
+    const long base = long(hk) * long(g.ny) * H;
+    cpxf* const A = (un.ca == 0 ? TX : TZ) + base + long(un.ra) * H;
+    cpxf* const B = (un.cb == 1 ? TY : TZ) + base + long(un.rb) * H;
+    split_pair<NX>(v, line, t, [&](int k, cpxf a, cpxf b) {
+        if (un.a) A[k] = a;
+        if (un.b) B[k] = b;
+    });
 }
 
 template <int NY>
@@ -217,8 +208,8 @@ __global__ void __launch_bounds__(CW * FftShape<NY>::T) k_sp_cols_inv_f(Geo g, c
     cpxf* s0 = smf;
     cpxf* s1 = smf + ColTile<NY, CW>::size;
     const int l = blockIdx.y, c0 = blockIdx.x * CW, tid = threadIdx.x, nthr = CW * S::T, H = g.H;
-    const long nk = g.nkh, base = long(l) * nk;
-    const int n = g.a + l;
+    const long base = long(l) * g.nkh;
+    const BoundPsi<cpxf> bp(g, jz, nullptr, l, g2);                  // one rank: no ghost half-cells
     #pragma unroll
     for (int u_ = 0; u_ < (NY * CW + nthr - 1) / nthr; ++u_) {
         const int e = tid + u_ * nthr;
@@ -228,20 +219,7 @@ __global__ void __launch_bounds__(CW * FftShape<NY>::T) k_sp_cols_inv_f(Geo g, c
         if (kxi < H) {
             const long i = long(p) * H + kxi, o = base + i;
             const double kx = g.kxd[kxi], ky = g.kyd[p], k2 = kx * kx + ky * ky;
-            // bound field psi of the slice charge (one rank: no ghost half-cells)
-            auto half = [&](int hk) -> cpx { return (hk < 0 || hk > g.ns) ? C(0) : to_d(jz[long(hk) * nk + i]); };
-            auto rho_at = [&](int dl) -> cpx {
-                const int nn = n + dl;
-                if (nn < 0 || nn > g.N - 1) return C(0);
-                return g.wlo[nn] * half(l + dl) + g.whi[nn] * half(l + dl + 1);
-            };
-            const double hm = g.hcg[n + 1], hp = g.hcg[n + 2];
-            const double cm = 2 / ((hm + hp) * hm), cp_ = 2 / ((hm + hp) * hp);
-            cpx psi = C(0);
-            if (k2 > 0) {
-                const cpx d2 = g2 * (cp_ * rho_at(1) - (cm + cp_) * rho_at(0) + cm * rho_at(-1));
-                psi = (rho_at(0) + d2 / k2) / k2;
-            }
+            const cpx psi = bp.at(i, k2);
             u = to_f(Rx[o] + opb * ik(kx, psi));              // R - R_b, R_b = -(1 + beta) i k psi
             v = to_f(Ry[o] + opb * ik(ky, psi));
         }
@@ -264,56 +242,35 @@ __global__ void __launch_bounds__(CW * FftShape<NY>::T) k_sp_cols_inv_f(Geo g, c
     }
 }
 template <int NX>
-__global__ void __launch_bounds__(NT) k_sp_rows_f(Geo g, const cpxf* __restrict__ tw, cpxf* __restrict__ U, cpxf* __restrict__ V) {
-    using S = FftShape<NX>;
-    constexpr int LPC = NT / S::T, RS = row_stride<NX>(), H = NX / 2 + 1;
+__global__ void __launch_bounds__(NT, 6) k_sp_rows_f(Geo g, const cpxf* __restrict__ tw, cpxf* __restrict__ U, cpxf* __restrict__ V) {
+    using S = FftRegPlan<NX>;
+    constexpr int LPC = NT / S::T, H = NX / 2 + 1;
     extern __shared__ cpxf smf[];
-    const int l = blockIdx.y, r0 = blockIdx.x * LPC, tid = threadIdx.x;
-    const long base = long(l) * g.nkh;
-    #pragma unroll
-    for (int u_ = 0; u_ < (LPC * H + NT - 1) / NT; ++u_) {
-        const int e = tid + u_ * NT;
-        if (e >= LPC * H) break;
-        const int r = e / H, p = e - r * H, row = r0 + r;
-        cpxf a = Cf(0), b = Cf(0);
-        if (row < g.ny) { const long o = base + long(row) * H + p; a = U[o]; b = V[o]; }
-        const cpxf z = Cf(a.x - b.y, a.y + b.x);
-        smf[r * RS + p + (p >> 3)] = conj(z);
-        if (p > 0 && p < NX / 2) {
-            const int q = NX - p;
-            smf[r * RS + q + (q >> 3)] = conj(Cf(a.x + b.y, -a.y + b.x));
-        }
+    const int l = blockIdx.y, r = threadIdx.x / S::T, t = threadIdx.x % S::T, row = blockIdx.x * LPC + r;
+    const bool on = row < g.ny;
+    const long o = long(l) * g.nkh + long(on ? row : 0) * H;
+    cpxf* const line = smf + r * row_stride<NX>();
+    cpxf v[S::E];
+#pragma unroll
+    for (int j = 0; j < S::E; ++j) {
+        const int k = t + S::T * j;
+        const bool up = k > NX / 2;
+        const long i = o + (up ? NX - k : k);
+        v[j] = pair_conj(up, U[i], V[i]);
     }
-    __syncthreads();
-    const int r = tid / S::T, t = tid - r * S::T;
-    fft_line<NX>(smf, RowAddr{r * RS}, t, tw);
+    fft_reg<NX>(v, line, t, tw);
     const float s = 1.0f / float(g.nk);
-    #pragma unroll
-    for (int u_ = 0; u_ < (LPC * NX + NT - 1) / NT; ++u_) {
-        const int e = tid + u_ * NT;
-        if (e >= LPC * NX) break;
-        const int rr = e / NX, p = e - rr * NX, row = r0 + rr;
-        const int q = rr * RS + p + (p >> 3);
-        const cpxf z = s * conj(smf[q]);
-        const float mx = float(g.maskx[p]);
-        const float mn = row < g.ny ? float(g.masky_n[row]) : 1.0f, mh = row < g.ny ? float(g.masky_h[row]) : 1.0f;
-        smf[q] = Cf((mx * mn - 1.0f) * z.x, (mx * mh - 1.0f) * z.y);      // (mask - 1): the correction only
+    const float mn = on ? float(g.masky_n[row]) : 1.0f, mh = on ? float(g.masky_h[row]) : 1.0f;
+#pragma unroll
+    for (int j = 0; j < S::E; ++j) {
+        const float mx = float(g.maskx[t + S::T * j]);
+        const cpxf z = s * conj(v[j]);
+        v[j] = Cf((mx * mn - 1.0f) * z.x, (mx * mh - 1.0f) * z.y);      // (mask - 1): the correction only
     }
-    __syncthreads();
-    fft_line<NX>(smf, RowAddr{r * RS}, t, tw);
-    #pragma unroll
-    for (int u_ = 0; u_ < (LPC * H + NT - 1) / NT; ++u_) {
-        const int e = tid + u_ * NT;
-        if (e >= LPC * H) break;
-        const int rr = e / H, p = e - rr * H, row = r0 + rr;
-        if (row >= g.ny) continue;
-        const int pm = (NX - p) % NX;
-        const cpxf z = smf[rr * RS + p + (p >> 3)], zm = conj(smf[rr * RS + pm + (pm >> 3)]);
-        const cpxf d = z - zm;
-        const long o = base + long(row) * H + p;
-        U[o] = 0.5f * (z + zm);
-        V[o] = 0.5f * Cf(d.y, -d.x);
-    }
+    fft_reg<NX>(v, line, t, tw);
+    split_pair<NX>(v, line, t, [&](int k, cpxf a, cpxf b) {
+        if (on) { U[o + k] = a; V[o + k] = b; }
+    });
 }
 template <int NY>
 __global__ void __launch_bounds__(CW * FftShape<NY>::T) k_sp_cols_fwd_f(Geo g, const cpxf* __restrict__ tw, const cpxf* __restrict__ U,
@@ -353,7 +310,8 @@ __global__ void __launch_bounds__(CW * FftShape<NY>::T) k_sp_cols_fwd_f(Geo g, c
 }
 
 // ---------------------------------------------------------------- real fields (FP32 transforms of the FP64 R)
-template <int NY, int CWT>
+// COMB: as k_rf_cols (k_fields.cu), the combinations in FP64
+template <int NY, int CWT, bool COMB>
 __global__ void __launch_bounds__(CWT * FftShape<NY>::T) k_rf_cols_f(Geo g, const cpxf* __restrict__ tw, const cpx* __restrict__ Rx,
                                                                     const cpx* __restrict__ Ry, const cpxf* __restrict__ Lx,
                                                                     const cpxf* __restrict__ Ly, const cpxf* __restrict__ Ez,
@@ -365,8 +323,8 @@ __global__ void __launch_bounds__(CWT * FftShape<NY>::T) k_rf_cols_f(Geo g, cons
     extern __shared__ cpxf smf[];
     const int l = l0 + blockIdx.y, c0 = blockIdx.x * CWT, tid = threadIdx.x, nthr = CWT * S::T, pr = blockIdx.z, H = g.H;
     const long base = long(l) * g.nkh;
-    cpxf* out0 = pr == 0 ? W0 : pr == 1 ? W2 : W4;
-    cpxf* out1 = pr == 0 ? W1 : pr == 1 ? W3 : W5;
+    cpxf* out0 = pr == 2 ? W4 : COMB ? (pr == 0 ? W0 : W1) : (pr == 0 ? W0 : W2);
+    cpxf* out1 = pr == 2 ? W5 : COMB ? (pr == 0 ? W3 : W2) : (pr == 0 ? W1 : W3);
     cpxf* s0 = smf;
     cpxf* s1 = smf + ColTile<NY, CWT>::size;
     #pragma unroll
@@ -377,9 +335,13 @@ __global__ void __launch_bounds__(CWT * FftShape<NY>::T) k_rf_cols_f(Geo g, cons
         const long o = base + long(p) * H + kxi;
         cpxf a = Cf(0), b = Cf(0);
         if (kxi < H) {
-            if (pr == 0) { a = to_f(Rx[o]); b = to_f(Ry[o]); }
-            else if (pr == 1) { a = Lx[o]; b = Ly[o]; }
-            else { a = Ez[o]; b = Bz[o]; }
+            if (pr == 2) { a = Ez[o]; b = Bz[o]; }
+            else if constexpr (COMB) {
+                const cpx R = pr == 0 ? Rx[o] : Ry[o], L = to_d(pr == 0 ? Lx[o] : Ly[o]);
+                a = to_f(0.5 * (R + L));
+                b = to_f(pr == 0 ? 0.5 * (R - L) : 0.5 * (L - R));
+            } else if (pr == 0) { a = to_f(Rx[o]); b = to_f(Ry[o]); }
+            else { a = Lx[o]; b = Ly[o]; }
         }
         s0[ColTile<NY, CWT>::at(p, c)] = conj(a); s1[ColTile<NY, CWT>::at(p, c)] = conj(b);
     }
@@ -397,51 +359,6 @@ __global__ void __launch_bounds__(CWT * FftShape<NY>::T) k_rf_cols_f(Geo g, cons
         if (kxi >= H) continue;
         const long o = base + long(p) * H + kxi;
         out0[o] = conj(s0[ColTile<NY, CWT>::at(p, cc)]); out1[o] = conj(s1[ColTile<NY, CWT>::at(p, cc)]);
-    }
-}
-template <int NX>
-__global__ void __launch_bounds__(NT) k_rf_rows_f(Geo g, const cpxf* __restrict__ tw, const cpxf* __restrict__ W0,
-                                                 const cpxf* __restrict__ W1, const cpxf* __restrict__ W2,
-                                                 const cpxf* __restrict__ W3, const cpxf* __restrict__ W4,
-                                                 const cpxf* __restrict__ W5, float* __restrict__ F) {
-    using S = FftShape<NX>;
-    constexpr int LPC = NT / S::T, RS = row_stride<NX>(), H = NX / 2 + 1;
-    extern __shared__ cpxf smf[];
-    cpxf* a[3] = {smf, smf + LPC * RS, smf + 2 * LPC * RS};
-    const int l = blockIdx.y, r0 = blockIdx.x * LPC, tid = threadIdx.x;
-    const long base = long(l) * g.nkh;
-    const cpxf* in[6] = {W0, W1, W2, W3, W4, W5};
-    const long fpl = long(g.ns + 2) * g.nk, fbase = long(l) * g.nk;
-    constexpr int EO = (LPC * NX + NT - 1) / NT;                    // output elements of a thread
-    #pragma unroll
-    for (int u_ = 0; u_ < (LPC * H + NT - 1) / NT; ++u_) {
-        const int e = tid + u_ * NT;
-        if (e >= LPC * H) break;
-        const int r = e / H, p = e - r * H, row = r0 + r;
-        for (int f = 0; f < 3; ++f) {
-            cpxf x = Cf(0), y = Cf(0);
-            if (row < g.ny) { const long o = base + long(row) * H + p; x = in[2 * f][o]; y = in[2 * f + 1][o]; }
-            a[f][r * RS + p + (p >> 3)] = conj(Cf(x.x - y.y, x.y + y.x));
-            if (p > 0 && p < NX / 2) { const int q = NX - p; a[f][r * RS + q + (q >> 3)] = conj(Cf(x.x + y.y, -x.y + y.x)); }
-        }
-    }
-    __syncthreads();
-    const int r = tid / S::T, t = tid - r * S::T;
-    fft_lines<NX, 3>(a, RowAddr{r * RS}, t, tw);
-    const float s = 1.0f / float(g.nk);
-    #pragma unroll
-    for (int u_ = 0; u_ < EO; ++u_) {
-        const int e = tid + u_ * NT;
-        if (e >= LPC * NX) continue;
-        const int rr = e / NX, p = e - rr * NX, row = r0 + rr;
-        if (row >= g.ny) continue;
-        const int q = rr * RS + p + (p >> 3);
-        const cpxf z1 = s * conj(a[0][q]), z2 = s * conj(a[1][q]), z3 = s * conj(a[2][q]);
-        const long idx = fbase + long(row) * NX + p;
-        const float fv[6] = {0.5f * (z1.x + z2.x), 0.5f * (z1.y + z2.y), z3.x,      // E_x, E_y, E_z
-                             0.5f * (z2.y - z1.y), 0.5f * (z1.x - z2.x), z3.y};     // B_x, B_y, B_z
-#pragma unroll
-        for (int comp = 0; comp < 6; ++comp) F[comp * fpl + idx] = fv[comp];
     }
 }
 
@@ -496,11 +413,11 @@ void launch_deposit_f(Ctx& c) {
 }
 template <int NX>
 static void cur_rows_f(Ctx& c) {
-    constexpr int LPC = NT / FftShape<NX>::T;
-    const size_t smem = size_t(2) * LPC * row_stride<NX>() * sizeof(cpxf);
+    constexpr int LPC = NT / FftRegPlan<NX>::T;
+    const size_t smem = size_t(LPC) * row_stride<NX>() * sizeof(cpxf);
     allow_smem(k_cur_rows_f<NX>, smem);
     const int tok = c.prof_begin("cur_rows");
-    k_cur_rows_f<NX><<<dim3(unsigned((c.ny + LPC - 1) / LPC), unsigned(c.ns + 1)), NT, smem, c.stream>>>(
+    k_cur_rows_f<NX><<<dim3(unsigned((CurUnit::count(c.ny) + LPC - 1) / LPC), unsigned(c.ns + 1)), NT, smem, c.stream>>>(
         c.geo(), c.mx.jw.p, c.mx.twx.p, c.mx.W[0].p, c.mx.W[1].p, c.mx.W[2].p, c.P.zeta_filter ? 1 : 0);
     c.check_launch("k_cur_rows_f");
     c.prof_end(tok);
@@ -540,7 +457,7 @@ static void sp_cols_inv_f(Ctx& c) {
 }
 template <int NX>
 static void sp_rows_f(Ctx& c) {
-    constexpr int LPC = NT / FftShape<NX>::T;
+    constexpr int LPC = NT / FftRegPlan<NX>::T;
     const size_t smem = size_t(LPC) * row_stride<NX>() * sizeof(cpxf);
     allow_smem(k_sp_rows_f<NX>, smem);
     const int tok = c.prof_begin("sponge_rows");
@@ -564,13 +481,13 @@ void launch_sponge_f(Ctx& c) {
     G3D_DISPATCH_N(c.nx, NX, sp_rows_f<NX>(c));
     G3D_DISPATCH_N(c.ny, NY, sp_cols_fwd_f<NY>(c));
 }
-template <int NY, int CWT>
+template <int NY, int CWT, bool COMB>
 static void rf_cols_fw(Ctx& c, int l0, int nl) {
     const size_t smem = size_t(2) * ColTile<NY, CWT>::size * sizeof(cpxf);
-    allow_smem(k_rf_cols_f<NY, CWT>, smem);
+    allow_smem(k_rf_cols_f<NY, CWT, COMB>, smem);
     const int tok = c.prof_begin(nl == 1 ? "real_cols_slice" : "real_cols");
     auto& m = c.mx;
-    k_rf_cols_f<NY, CWT><<<dim3(unsigned((c.H + CWT - 1) / CWT), unsigned(nl), 3), CWT * FftShape<NY>::T, smem, c.stream>>>(
+    k_rf_cols_f<NY, CWT, COMB><<<dim3(unsigned((c.H + CWT - 1) / CWT), unsigned(nl), 3), CWT * FftShape<NY>::T, smem, c.stream>>>(
         c.geo(), m.twy.p, c.Rx.p, c.Ry.p, m.Lx.p, m.Ly.p, m.Ez.p, m.Bz.p, m.W[0].p, m.W[1].p, m.W[2].p, m.W[3].p, m.W[4].p, m.W[5].p,
         l0);
     c.check_launch("k_rf_cols_f");
@@ -579,24 +496,12 @@ static void rf_cols_fw(Ctx& c, int l0, int nl) {
 // one slice (the plasma march): tiles of 2 columns, so that 3 x 65 CTAs spread the slice's latency over the SMs
 template <int NY>
 static void rf_cols_f(Ctx& c, int l0, int nl) {
-    if (nl == 1) rf_cols_fw<NY, 2>(c, l0, nl);
-    else rf_cols_fw<NY, CW>(c, l0, nl);
-}
-template <int NX>
-static void rf_rows_f(Ctx& c) {
-    constexpr int LPC = NT / FftShape<NX>::T;
-    const size_t smem = size_t(3) * LPC * row_stride<NX>() * sizeof(cpxf);
-    allow_smem(k_rf_rows_f<NX>, smem);
-    const int tok = c.prof_begin("real_rows");
-    auto& m = c.mx;
-    k_rf_rows_f<NX><<<dim3(unsigned((c.ny + LPC - 1) / LPC), unsigned(c.ns)), NT, smem, c.stream>>>(
-        c.geo(), m.twx.p, m.W[0].p, m.W[1].p, m.W[2].p, m.W[3].p, m.W[4].p, m.W[5].p, c.F.p);
-    c.check_launch("k_rf_rows_f");
-    c.prof_end(tok);
+    if (nl == 1) rf_cols_fw<NY, 2, false>(c, l0, nl);
+    else rf_cols_fw<NY, CW, true>(c, l0, nl);
 }
 void launch_real_fields_f(Ctx& c) {
     G3D_DISPATCH_N(c.ny, NY, rf_cols_f<NY>(c, 0, c.ns));
-    G3D_DISPATCH_N(c.nx, NX, rf_rows_f<NX>(c));
+    launch_rf_rows_f(c);
 }
 // E and B of one slice (plane l) of the mixed form (the real fields of one slice of the plasma march); cols: the columns
 // too (into plane l of W); else they are in plane 0 of W, where k_pass_cols left them
