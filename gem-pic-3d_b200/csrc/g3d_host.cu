@@ -457,7 +457,7 @@ static void setup(Ctx& c, const g3d_grid& G, const g3d_params& P) {
     };
     c.twx.upload(tw(nx), s); c.twy.upload(tw(ny), s);
     realloc_slab(c);
-    c.red.alloc(size_t(297) * 17, s);
+    c.red.alloc(size_t(297) * 17 + 1 + 600, s);         // k_diag.cu: the particle sums, the field energy
     c.kerr.alloc(1, s);
     c.use_tma = std::getenv("G3D_NO_TMA") == nullptr;
     if (const char* v = std::getenv("G3D_TMA_POLLS")) c.tma_polls = std::max(1L, std::atol(v));
@@ -1984,7 +1984,6 @@ int g3d_diagnostics(g3d_ctx* ctx, double out[19]) {
         Ctx& c = ctx->c;
         double S[19] = {0};
         g3d::launch_diag(c, S);
-        S[15] = c.P.self_fields ? g3d::launch_field_energy(c) : 0;
         S[16] = double(c.lost_total);
         if (c.sharded()) {                               // the particles lost on every rank
             g3d::DevBuf<double> lost;

@@ -182,34 +182,54 @@ __global__ void __launch_bounds__(RT) k_moments(PartsDev P, long np, double X0, 
 
 // `sum`: a sum over the particles, which a sharded run adds across the ranks
 template <int NV>
-void finish(Ctx& c, double* out, bool sum, int nb = RB) {
-    k_final<NV><<<1, RT, 0, c.stream>>>(c.red.p, nb, c.red.p + nb * NV);
+void finish(Ctx& c, double* out, bool sum) {
+    k_final<NV><<<1, RT, 0, c.stream>>>(c.red.p, RB, c.red.p + RB * NV);
     c.check_launch("k_final");
-    if (sum) c.all_sum(c.red.p + nb * NV, NV, G3D_SUM_F64);
-    G3D_CUDA(cudaMemcpyAsync(out, c.red.p + nb * NV, NV * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+    if (sum) c.all_sum(c.red.p + RB * NV, NV, G3D_SUM_F64);
+    G3D_CUDA(cudaMemcpyAsync(out, c.red.p + RB * NV, NV * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
     G3D_CUDA(cudaStreamSynchronize(c.stream));
 }
 }  // namespace
 
+namespace {
+// the field energy's partial sums and total (times dx: launch_field_energy) into out
+void energy_into(Ctx& c, double* part, double* out) {
+    const int tok = c.prof_begin("field_energy");
+    k_energy<<<EB, RT, 0, c.stream>>>(c.geo(), c.F.p, part);
+    c.check_launch("k_energy");
+    c.prof_end(tok);
+    k_final<1><<<1, RT, 0, c.stream>>>(part, EB, out);
+    c.check_launch("k_final");
+}
+}  // namespace
+// The sums of diag.txt and, with self fields, the field energy S[15]: both reductions on the stream, then one copy and one
+// wait for the two.
 void launch_diag(Ctx& c, double S[19]) {
-    double r[NDIAG];
+    double r[NDIAG + 1];
     DiagArgs d{c.laser, c.X0, c.Y0, c.s, c.P.zeta_center};
+    double* const tot = c.red.p + RB * NDIAG;                // the totals, the energy's behind them, then its partial sums
     const int tok = c.prof_begin("diag");
     k_diag<<<RB, RT, 0, c.stream>>>(c.parts, c.np, d, c.red.p);
     c.check_launch("k_diag");
     c.prof_end(tok);
-    finish<NDIAG>(c, r, true);
+    k_final<NDIAG><<<1, RT, 0, c.stream>>>(c.red.p, RB, tot);
+    c.check_launch("k_final");
+    const int nv = NDIAG + (c.P.self_fields ? 1 : 0);
+    if (c.P.self_fields) energy_into(c, tot + NDIAG + 1, tot + NDIAG);
+    c.all_sum(tot, nv, G3D_SUM_F64);
+    G3D_CUDA(cudaMemcpyAsync(r, tot, size_t(nv) * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+    G3D_CUDA(cudaStreamSynchronize(c.stream));
     for (int k = 0; k < 15; ++k) S[k] = r[k];
+    S[15] = c.P.self_fields ? r[NDIAG] * c.dx : 0;
     S[17] = r[15]; S[18] = r[16];
 }
 
 double launch_field_energy(Ctx& c) {
     double r[1];
-    const int tok = c.prof_begin("field_energy");
-    k_energy<<<EB, RT, 0, c.stream>>>(c.geo(), c.F.p, c.red.p);
-    c.check_launch("k_energy");
-    c.prof_end(tok);
-    finish<1>(c, r, true, EB);                // a sharded run: the energies of the slabs
+    energy_into(c, c.red.p + 1, c.red.p);
+    c.all_sum(c.red.p, 1, G3D_SUM_F64);       // a sharded run: the energies of the slabs
+    G3D_CUDA(cudaMemcpyAsync(r, c.red.p, sizeof r, cudaMemcpyDeviceToHost, c.stream));
+    G3D_CUDA(cudaStreamSynchronize(c.stream));
     return r[0] * c.dx;
 }
 
