@@ -412,12 +412,12 @@ void march_plasma(Ctx& c, double s0, double s1) {
     G3D_CUDA(cudaMemcpyAsync(P.stepv.p, &stv, sizeof(StepVals), cudaMemcpyHostToDevice, c.stream));
     const bool ionz = P.born_cap > 0;
     const int passes = P.cfg.iterations;
-    // The slice loop is some 20 launches per half-cell (about 41,000 for 2,048 slices and two passes). Launched
-    // one by one, the host's launch rate would bound the march; as one CUDA graph they run back to back. The
-    // graph is captured once and launched every step; it is captured again only when something it holds by value
-    // changes (a buffer of the window moved, the capacity of the freed-electron list, the step length). The
-    // streaming and freed-electron lists are reached through a descriptor on the device, so they may move. While per-kernel events
-    // are recorded the loop is launched directly.
+    // The slice loop is four launches per half-cell and pass on Fourier y, some eight on the free-hand grid. On the smallest
+    // grids the host's launch rate would bound it: there it runs as a CUDA graph, captured once per set of buffers it holds
+    // by value (j0 and jk trade theirs every step) and launched every step after. It is captured again only when something it
+    // holds changes (a buffer of the window moved, the capacity of the freed-electron list, the step length). The
+    // streaming and freed-electron lists are reached through a descriptor on the device, so they may move. While per-kernel
+    // events are recorded the loop is launched directly.
     uint64_t key = 1469598103934665603ULL;
     auto mixk = [&](uint64_t v) { key = (key ^ v) * 1099511628211ULL; };
     auto ptr = [](const void* q) { return uint64_t(reinterpret_cast<uintptr_t>(q)); };
@@ -513,26 +513,41 @@ void march_plasma(Ctx& c, double s0, double s1) {
         c.launches += hit->launches;
         G3D_CUDA(cudaGraphLaunch(hit->exec, c.stream));
     } else {
-        if (P.loops.size() >= 4) { cudaGraphExecDestroy(P.loops.front().exec); P.loops.erase(P.loops.begin()); }
+        // Kernel by kernel: the device is what bounds a march on all but the smallest grids (a step of 48 x 48 x 400: 12.4 to
+        // 14.1 ms so, 12.8 to 13.6 ms as a graph; 64 x 64 x 1201: 43.7 and 42.8 ms), and a graph of some ten thousand nodes takes
+        // the host longer to capture and instantiate than many steps. On a smaller transverse grid the launches bound it
+        // (32 x 32 x 160: 5.1 to 5.5 against 4.5 ms): there the graph is made when a set of buffers comes a second time, by
+        // the host while the device works on the march (a capture records only what is issued during it, not the work in
+        // flight on the stream), for the marches to come.
         const long l0 = c.launches;
-        G3D_CUDA(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeRelaxed));
-        try {
-            issue();
-        } catch (...) {
+        issue();
+        const long l1 = c.launches;
+        const bool small = long(c.nx) * c.ny < 2048, again = std::find(P.seen.begin(), P.seen.end(), key) != P.seen.end();
+        if (small && !again) {
+            if (P.seen.size() >= 8) P.seen.erase(P.seen.begin());
+            P.seen.push_back(key);
+        } else if (small) {
+            if (P.loops.size() >= 4) { cudaGraphExecDestroy(P.loops.front().exec); P.loops.erase(P.loops.begin()); }
+            G3D_CUDA(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeRelaxed));
+            try {
+                issue();
+            } catch (...) {
+                cudaGraph_t gr = nullptr;
+                cudaStreamEndCapture(c.stream, &gr);
+                if (gr) cudaGraphDestroy(gr);
+                cudaGetLastError();
+                throw;
+            }
+            c.launches = l1;                               // captured, not launched
             cudaGraph_t gr = nullptr;
-            cudaStreamEndCapture(c.stream, &gr);
-            if (gr) cudaGraphDestroy(gr);
-            cudaGetLastError();
-            throw;
+            G3D_CUDA(cudaStreamEndCapture(c.stream, &gr));
+            cudaGraphExec_t ex = nullptr;
+            const cudaError_t e = cudaGraphInstantiate(&ex, gr, 0);
+            cudaGraphDestroy(gr);
+            G3D_CUDA(e);
+            P.loops.push_back(PlasmaState::LoopGraph{key, ex, l1 - l0});
+            G3D_CUDA(cudaGraphUpload(ex, c.stream));
         }
-        cudaGraph_t gr = nullptr;
-        G3D_CUDA(cudaStreamEndCapture(c.stream, &gr));
-        cudaGraphExec_t ex = nullptr;
-        const cudaError_t e = cudaGraphInstantiate(&ex, gr, 0);
-        cudaGraphDestroy(gr);
-        G3D_CUDA(e);
-        P.loops.push_back(PlasmaState::LoopGraph{key, ex, c.launches - l0});
-        G3D_CUDA(cudaGraphLaunch(ex, c.stream));
     }
     G3D_CUDA(cudaStreamSynchronize(c.stream));
     int flag = 0;

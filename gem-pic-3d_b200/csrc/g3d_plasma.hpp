@@ -159,6 +159,7 @@ struct PlasmaState {
     // buffers swap every step); captured again only when a buffer moved
     struct LoopGraph { uint64_t key; cudaGraphExec_t exec; long launches; };
     std::vector<LoopGraph> loops;
+    std::vector<uint64_t> seen;                // the keys of the last marches launched without a graph
     // the reverse of a march (the adjoint, k_adj_plasma.cu) as a CUDA graph, keyed like the loops
     struct AdjGraph { uint64_t key = 0; cudaGraphExec_t exec = nullptr; } adjg;
     DevBuf<StepVals> stepv;
