@@ -149,8 +149,9 @@ def algorithmic_bytes(name, cfg, mixed=False, S=0):
         "stream_spectra": 2 * (16 if mixed else 24) * nk + 48 * nkh,
         # the fused column work of a pass: the half rows read, jsn written, the replace and march of the slice
         # (less its read of jsn), the six column transforms of the slice's fields written (their inputs stay in
-        # shared memory)
-        "pass_cols": 48 * nkh + 48 * nkh + replace_pred + march_slice - 48 * nkh + 6 * cz * nkh,
+        # shared memory); the correction and the next half-cell's prologue on the last of a half-cell's passes
+        "pass_cols": 48 * nkh + 48 * nkh + replace_pred + march_slice - 48 * nkh + 6 * cz * nkh
+        + (correct + slice_prologue) // max(1, int((cfg.plasma or {}).get("iterations", 1))),
         "march_slice": march_slice,
         "real_cols_slice": (2 * 16 + 4 * cz + 6 * cz) * nkh,
         # six column transforms read, F written; the other F plane read and the midpoint fields written
@@ -475,8 +476,8 @@ def time_form(cfg, precision, a, world, dist, local):
     ms = max_over_ranks(e0.elapsed_time(e1), dist)
     clk = clocks.stop()
     launches = sim.launch_count() - l0
-    # per-kernel CUDA events in a separate pass: events around every kernel add gaps, and the plasma march is
-    # launched as one graph only when no events are recorded
+    # per-kernel CUDA events in a separate pass: events around every kernel add gaps, and the plasma march's
+    # kernels overlap their launches only when no events are recorded between them
     sim.profile(True)
     for _ in range(max(1, min(a.steps, 5))):
         sim.step_async()
