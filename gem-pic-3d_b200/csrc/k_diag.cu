@@ -13,18 +13,25 @@ namespace {
 constexpr int RB = 296;     // blocks of the first level (2 per SM)
 constexpr int RT = 256;     // threads per block
 
+// The block's sums into out[0 .. NV): a tree over each warp's lanes by shuffles, then the warps in order. (A tree in shared
+// memory per value, nine barriers each, was most of the time of the small reductions: 17 values of 8,192 particles,
+// their kernel 14.2 -> 10.5 us.)
 template <int NV>
 __device__ void block_store(double (&acc)[NV], double* __restrict__ out) {
-    __shared__ double sh[RT];
+    __shared__ double sh[RT / 32][NV];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int v = 0; v < NV; ++v) {
-        sh[threadIdx.x] = acc[v];
-        __syncthreads();
-        for (int s = RT / 2; s > 0; s >>= 1) {
-            if (int(threadIdx.x) < s) sh[threadIdx.x] += sh[threadIdx.x + s];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) out[long(blockIdx.x) * NV + v] = sh[0];
-        __syncthreads();
+        double x = acc[v];
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1) x += __shfl_xor_sync(0xffffffffu, x, s);
+        if (lane == 0) sh[warp][v] = x;
+    }
+    __syncthreads();
+    for (int v = threadIdx.x; v < NV; v += RT) {
+        double x = sh[0][v];
+#pragma unroll
+        for (int k = 1; k < RT / 32; ++k) x += sh[k][v];
+        out[v] = x;
     }
 }
 
@@ -40,10 +47,10 @@ __global__ void __launch_bounds__(RT) k_final(const double* __restrict__ part, i
 // ------------------------------------------------ particle sums of diag.txt
 struct DiagArgs { LaserDev laser; double X0, Y0, s, zc; };
 constexpr int NDIAG = 17;    // S[0..14], trapped count, trapped charge
-__global__ void __launch_bounds__(RT) k_diag(PartsDev P, long np, DiagArgs d, double* __restrict__ part) {
+__device__ void diag_block(const PartsDev& P, long np, const DiagArgs& d, int b, int nb, double* __restrict__ out) {
     double acc[NDIAG];
     for (int v = 0; v < NDIAG; ++v) acc[v] = 0;
-    for (long i = long(blockIdx.x) * RT + threadIdx.x; i < np; i += long(gridDim.x) * RT) {
+    for (long i = long(b) * RT + threadIdx.x; i < np; i += long(nb) * RT) {
         if (P.alive[i] != 1) continue;
         const double w = P.w[i];
         if (P.sp[i] > 0) { acc[15] += 1; acc[16] += P.q[i] * w; continue; }     // trapped plasma electrons
@@ -55,7 +62,7 @@ __global__ void __launch_bounds__(RT) k_diag(PartsDev P, long np, DiagArgs d, do
         for (int k = 0; k < 14; ++k) acc[k] += w * v[k];
         acc[14] += 1;
     }
-    block_store<NDIAG>(acc, part);
+    block_store<NDIAG>(acc, out);
 }
 
 // ------------------------------------------------ field energy: sum over slices of 1/2 w E^2 (dual cells)
@@ -67,14 +74,14 @@ __global__ void __launch_bounds__(RT) k_diag(PartsDev P, long np, DiagArgs d, do
 // 256 x 256 x 2048 3,180 -> 503 us. The order of the sum is fixed by the grid alone, as before.
 constexpr int EB = 592;      // blocks: 4 per SM
 constexpr int EV = 4;        // float4 per thread and chunk
-__global__ void __launch_bounds__(RT) k_energy(Geo g, const float* __restrict__ F, double* __restrict__ part) {
+__device__ void energy_block(const Geo& g, const float* __restrict__ F, int b, int nb, double* __restrict__ out) {
     double acc[1] = {0};
     const int n4 = g.nk / 4, nx4 = g.nx / 4;                 // float4 of a plane, of a row
     const long fpl = long(g.ns + 2) * g.nk;
     const int chunks = (n4 + RT * EV - 1) / (RT * EV);
     const long units = 6L * g.ns * chunks;
     const double w0 = 1 / g.iA[0];                           // Fourier y: one dual-cell size
-    for (long u = blockIdx.x; u < units; u += gridDim.x) {
+    for (long u = b; u < units; u += nb) {
         const int ch = int(u % chunks);
         const long pl = u / chunks;
         const int comp = int(pl / g.ns), l = int(pl - long(comp) * g.ns);
@@ -90,12 +97,33 @@ __global__ void __launch_bounds__(RT) k_energy(Geo g, const float* __restrict__ 
             const int i = i0 + k * RT;
             if (i >= n4) break;
             const double wj = g.yf ? w0 : 1 / (half ? g.iD : g.iA)[i / nx4];
-            const double a = v[k].x, b = v[k].y, c = v[k].z, d = v[k].w;
-            e += wj * (a * a + b * b + (c * c + d * d));
+            const double v0 = v[k].x, v1 = v[k].y, v2 = v[k].z, v3 = v[k].w;
+            e += wj * (v0 * v0 + v1 * v1 + (v2 * v2 + v3 * v3));
         }
         acc[0] += 0.5 * g.wsl[g.a + l] * e;
     }
-    block_store<1>(acc, part);
+    block_store<1>(acc, out);
+}
+__global__ void __launch_bounds__(RT) k_energy(Geo g, const float* __restrict__ F, double* __restrict__ part) {
+    energy_block(g, F, blockIdx.x, EB, part + blockIdx.x);
+}
+// The two together: the first RB blocks take the particles, the others (none without self fields) the field energy, whose
+// partial sums lie behind the particles'. A small window's diagnostics are launches and latency, not bytes: the call of
+// 32 x 32 x 64 went from 52 to 37 us, 64 x 64 x 256 from 62 to 44, 128 x 128 x 1024 from 147 to 138.
+__global__ void __launch_bounds__(RT, 3) k_diag(PartsDev P, long np, DiagArgs d, Geo g, const float* __restrict__ F,
+                                               double* __restrict__ part) {
+    const int b = blockIdx.x;
+    if (b < RB) diag_block(P, np, d, b, RB, part + b * NDIAG);
+    else energy_block(g, F, b - RB, EB, part + RB * NDIAG + (b - RB));
+}
+// totals of both: out[0 .. NDIAG), out[NDIAG] the energy's (ne partial sums)
+__global__ void __launch_bounds__(RT) k_diag_final(const double* __restrict__ part, int ne, double* __restrict__ out) {
+    double acc[NDIAG + 1];
+    for (int v = 0; v <= NDIAG; ++v) acc[v] = 0;
+    for (int b = threadIdx.x; b < RB; b += RT)
+        for (int v = 0; v < NDIAG; ++v) acc[v] += part[b * NDIAG + v];
+    for (int b = threadIdx.x; b < ne; b += RT) acc[NDIAG] += part[RB * NDIAG + b];
+    block_store<NDIAG + 1>(acc, out);
 }
 
 // ------------------------------------------------ centroid of the bunch (window shift)
@@ -106,7 +134,7 @@ __global__ void __launch_bounds__(RT) k_centroid(PartsDev P, long np, double X0,
         const double w = P.w[i];
         acc[0] += w * (P.x[i] + X0); acc[1] += w * (P.y[i] + Y0); acc[2] += w;
     }
-    block_store<3>(acc, part);
+    block_store<3>(acc, part + 3 * blockIdx.x);
 }
 
 // ------------------------------------------------ mean beta of the alive particles (co-moving field)
@@ -177,7 +205,7 @@ __global__ void __launch_bounds__(RT) k_moments(PartsDev P, long np, double X0, 
             a[4] += w * d[4] * d[4]; a[5] += w * d[0] * d[3]; a[6] += w * d[1] * d[4]; a[7] += w * d[5] * d[5];
         }
     }
-    block_store<MOM_NV>(acc, part);
+    block_store<MOM_NV>(acc, part + long(MOM_NV) * blockIdx.x);
 }
 
 // `sum`: a sum over the particles, which a sharded run adds across the ranks
@@ -191,32 +219,19 @@ void finish(Ctx& c, double* out, bool sum) {
 }
 }  // namespace
 
-namespace {
-// the field energy's partial sums and total (times dx: launch_field_energy) into out
-void energy_into(Ctx& c, double* part, double* out) {
-    const int tok = c.prof_begin("field_energy");
-    k_energy<<<EB, RT, 0, c.stream>>>(c.geo(), c.F.p, part);
-    c.check_launch("k_energy");
-    c.prof_end(tok);
-    k_final<1><<<1, RT, 0, c.stream>>>(part, EB, out);
-    c.check_launch("k_final");
-}
-}  // namespace
-// The sums of diag.txt and, with self fields, the field energy S[15]: both reductions on the stream, then one copy and one
-// wait for the two.
+// The sums of diag.txt and, with self fields, the field energy S[15]: one kernel, their totals, one copy and one wait.
 void launch_diag(Ctx& c, double S[19]) {
     double r[NDIAG + 1];
     DiagArgs d{c.laser, c.X0, c.Y0, c.s, c.P.zeta_center};
-    double* const tot = c.red.p + RB * NDIAG;                // the totals, the energy's behind them, then its partial sums
+    const int ne = c.P.self_fields ? EB : 0, nv = NDIAG + (c.P.self_fields ? 1 : 0);
+    double* const tot = c.red.p + RB * NDIAG + EB;
     const int tok = c.prof_begin("diag");
-    k_diag<<<RB, RT, 0, c.stream>>>(c.parts, c.np, d, c.red.p);
+    k_diag<<<unsigned(RB + ne), RT, 0, c.stream>>>(c.parts, c.np, d, c.geo(), c.F.p, c.red.p);
     c.check_launch("k_diag");
     c.prof_end(tok);
-    k_final<NDIAG><<<1, RT, 0, c.stream>>>(c.red.p, RB, tot);
-    c.check_launch("k_final");
-    const int nv = NDIAG + (c.P.self_fields ? 1 : 0);
-    if (c.P.self_fields) energy_into(c, tot + NDIAG + 1, tot + NDIAG);
-    c.all_sum(tot, nv, G3D_SUM_F64);
+    k_diag_final<<<1, RT, 0, c.stream>>>(c.red.p, ne, tot);
+    c.check_launch("k_diag_final");
+    c.all_sum(tot, nv, G3D_SUM_F64);                         // a sharded run: the particles and the slabs of every rank
     G3D_CUDA(cudaMemcpyAsync(r, tot, size_t(nv) * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
     G3D_CUDA(cudaStreamSynchronize(c.stream));
     for (int k = 0; k < 15; ++k) S[k] = r[k];
@@ -226,9 +241,14 @@ void launch_diag(Ctx& c, double S[19]) {
 
 double launch_field_energy(Ctx& c) {
     double r[1];
-    energy_into(c, c.red.p + 1, c.red.p);
-    c.all_sum(c.red.p, 1, G3D_SUM_F64);       // a sharded run: the energies of the slabs
-    G3D_CUDA(cudaMemcpyAsync(r, c.red.p, sizeof r, cudaMemcpyDeviceToHost, c.stream));
+    const int tok = c.prof_begin("field_energy");
+    k_energy<<<EB, RT, 0, c.stream>>>(c.geo(), c.F.p, c.red.p);
+    c.check_launch("k_energy");
+    c.prof_end(tok);
+    k_final<1><<<1, RT, 0, c.stream>>>(c.red.p, EB, c.red.p + EB);
+    c.check_launch("k_final");
+    c.all_sum(c.red.p + EB, 1, G3D_SUM_F64);  // a sharded run: the energies of the slabs
+    G3D_CUDA(cudaMemcpyAsync(r, c.red.p + EB, sizeof r, cudaMemcpyDeviceToHost, c.stream));
     G3D_CUDA(cudaStreamSynchronize(c.stream));
     return r[0] * c.dx;
 }
