@@ -6,6 +6,12 @@
 // a kernel starts early, the kernel before it is past its own wait, i.e. everything up to the kernel before that one is
 // complete. Before its wait a kernel may therefore read what the kernel directly before it does not write, and
 // writes nothing. Without the launch attribute both calls do nothing.
+//
+// What the kernel directly before writes is not constant for the life of the kernel that reads it: that one is resident
+// already. So such memory is never read through `const __restrict__` pointers or __ldg, which promise that it is and let the
+// compiler take a non-coherent load or move the load above the wait. A kernel takes it as Handed<T> (or inside its argument
+// struct, or as a plain T*) and reads it by ordinary loads after pdl_wait(), which the clobber holds there. Tables and what
+// was written two or more kernels earlier may be read as constant.
 #pragma once
 #include "g3d_common.cuh"
 
@@ -13,6 +19,13 @@ namespace g3d {
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// memory handed over by the kernel before: a pointer without aliasing promises, whose values are read after pdl_wait()
+template <class T>
+struct Handed {
+    const T* p;
+    __device__ __forceinline__ T operator[](long i) const { return p[i]; }
+};
 
 template <class... P, class... A>
 void launch_pdl(cudaStream_t s, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {

@@ -168,11 +168,11 @@ __device__ __forceinline__ void sgather_mid(const StreamArgs& c, double x, doubl
             const R w = wx[i] * wn[j];
             if constexpr (F32) {
                 const float4* p = static_cast<const float4*>(c.Fmid) + 2 * k;
-                const float4 u = __ldg(p), v = __ldg(p + 1);
+                const float4 u = p[0], v = p[1];
                 a[0] += w * u.x; a[1] += w * u.y; a[2] += w * u.z; a[3] += w * u.w; a[4] += w * v.x; a[5] += w * v.y;
             } else {
                 const double2* p = static_cast<const double2*>(c.Fmid) + 3 * k;
-                const double2 u = __ldg(p), v = __ldg(p + 1), q = __ldg(p + 2);
+                const double2 u = p[0], v = p[1], q = p[2];
                 a[0] += w * u.x; a[1] += w * u.y; a[2] += w * v.x; a[3] += w * v.y; a[4] += w * q.x; a[5] += w * q.y;
             }
         }
@@ -197,12 +197,12 @@ __device__ __forceinline__ void sgather_mid_fh_f32(const StreamArgs& c, double x
         for (int i = 0; i < 3; ++i) {
             if (nod) {
                 const float w = float(wx[i] * wn[j]);
-                const float4 u = __ldg(F4 + 2 * (long(jn[j]) * g.nx + ix[i]));
+                const float4 u = F4[2 * (long(jn[j]) * g.nx + ix[i])];
                 a[0] += w * u.x; a[2] += w * u.y; a[4] += w * u.z;
             }
             if (hal) {
                 const float w = float(wx[i] * wh[j]);
-                const float4 v = __ldg(F4 + 2 * (long(jh[j]) * g.nx + ix[i]) + 1);
+                const float4 v = F4[2 * (long(jh[j]) * g.nx + ix[i]) + 1];
                 a[1] += w * v.x; a[3] += w * v.y; a[5] += w * v.z;
             }
         }
@@ -344,7 +344,7 @@ __device__ __forceinline__ void field_abs2(const StreamArgs& c, double x, double
             for (int i = 0; i < 3; ++i) {
                 const float* q = p + jy * g.nx + ix[i];
                 const R w = R(wx[i] * wy);
-                v0 += w * R(__ldg(q)); v1 += w * R(__ldg(q + nk));
+                v0 += w * R(q[0]); v1 += w * R(q[nk]);
             }
         }
         const double d0 = double(v0) + W0[comp], d1 = double(v1) + W1[comp];
@@ -781,7 +781,7 @@ static void stream_launch(Ctx& c, const StreamArgs& a, unsigned blocks) {
 // before: per launch with the events' ~5 us 8.4 -> 6.4 us at 64 x 64 FP64, 8.5 -> 6.4 us at 32 x 32 mixed, 8.8 -> 8.5 us
 // at 256 x 256 mixed).
 template <int NX, class JT>
-__global__ void __launch_bounds__(slice_row_threads<NX>()) k_ss_rows(Geo g, JT* __restrict__ J, cpx* __restrict__ T0, cpx* __restrict__ T1,
+__global__ void __launch_bounds__(slice_row_threads<NX>()) k_ss_rows(Geo g, JT* J, cpx* __restrict__ T0, cpx* __restrict__ T1,
                                                                     cpx* __restrict__ T2, int clear, int* __restrict__ bcnt) {
     using S = FftShape<NX>;
     constexpr int NTH = slice_row_threads<NX>(), RS = row_stride<NX>(), H = NX / 2 + 1, EPT = (NX + NTH - 1) / NTH;
@@ -990,8 +990,8 @@ __global__ void k_front(PlasmaPtrs p, Geo g, cpx* __restrict__ Rx, cpx* __restri
 // events' ~5 us: 256 x 256 mixed 19.5 -> 15.7 us, FP64 20.5 -> 15.6 us, 64 x 64 FP64 11.6 -> 8.4 us; the correction's
 // launch, 8.5 to 9.6 us per half-cell, is gone.
 template <int NY, class T, class WT, bool LAST>
-__global__ void __launch_bounds__(NY) k_pass_cols(PlasmaPtrs p, Geo g, const cpx* __restrict__ T0, const cpx* __restrict__ T1,
-                                                  const cpx* __restrict__ T2, double a2, int keep0, cpx* __restrict__ Rx,
+__global__ void __launch_bounds__(NY) k_pass_cols(PlasmaPtrs p, Geo g, Handed<cpx> T0, Handed<cpx> T1, Handed<cpx> T2,
+                                                  double a2, int keep0, cpx* __restrict__ Rx,
                                                   cpx* __restrict__ Ry, T* __restrict__ Ez, T* __restrict__ Bz, T* __restrict__ Lx,
                                                   T* __restrict__ Ly, const T* __restrict__ j0x, const T* __restrict__ j0y,
                                                   double D, int n, int extrap, double w, double q, const WT* __restrict__ twi,
@@ -1629,8 +1629,8 @@ static void pass_cols_form(Ctx& c, double D, int n, int extrap, double w, double
                         (6 * ColTile<NY, 1>::size + (std::is_same<WT, cpx>::value ? 0 : NY)) * sizeof(WT);
     auto kern = k_pass_cols<NY, T, WT, LAST>;
     smem_attr(reinterpret_cast<const void*>(kern), smem);
-    launch_pdl(c.stream, kern, unsigned(c.H), NY, smem, P.ptrs(c), c.geo(), S, S + c.nkh, S + 2 * c.nkh, a2, P.box_mean ? 1 : 0, c.Rx.p,
-               c.Ry.p, Ez, Bz, Lx, Ly, j0x, j0y, D, n, extrap, w, q, tw, W[0].p, W[1].p, W[2].p, W[3].p, W[4].p, W[5].p);
+    launch_pdl(c.stream, kern, unsigned(c.H), NY, smem, P.ptrs(c), c.geo(), Handed<cpx>{S}, Handed<cpx>{S + c.nkh},
+               Handed<cpx>{S + 2 * c.nkh}, a2, P.box_mean ? 1 : 0, c.Rx.p, c.Ry.p, Ez, Bz, Lx, Ly, j0x, j0y, D, n, extrap, w, q, tw, W[0].p, W[1].p, W[2].p, W[3].p, W[4].p, W[5].p);
 }
 template <int NY>
 static void pass_cols(Ctx& c, double D, int n, int extrap, double w, double q, bool last) {

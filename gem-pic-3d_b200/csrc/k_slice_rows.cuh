@@ -17,10 +17,9 @@ namespace g3d {
 // W0..W5: the half rows (k_x = 0 .. NX/2) of plane lw; F (and Fd, when kept): plane l of every component.
 // XM (exact fields with midpoint fields, FP64 Fourier y): the midpoint fields from the FP64 values of both slices (Fd).
 template <int NX, class T, bool XM>
-__global__ void __launch_bounds__(slice_row_threads<NX>()) k_rf_row_slice(Geo g, const T* __restrict__ tw, const T* __restrict__ W0,
-                                                                         const T* __restrict__ W1, const T* __restrict__ W2,
-                                                                         const T* __restrict__ W3, const T* __restrict__ W4,
-                                                                         const T* __restrict__ W5, float* __restrict__ F, int l, int lw,
+__global__ void __launch_bounds__(slice_row_threads<NX>()) k_rf_row_slice(Geo g, const T* __restrict__ tw, Handed<T> W0, Handed<T> W1,
+                                                                         Handed<T> W2, Handed<T> W3, Handed<T> W4, Handed<T> W5,
+                                                                         float* __restrict__ F, int l, int lw,
                                                                          double* __restrict__ Fd, FmidOut fm) {
     typedef typename RealOf<T>::type Re;
     using S = FftShape<NX>;
@@ -50,7 +49,7 @@ __global__ void __launch_bounds__(slice_row_threads<NX>()) k_rf_row_slice(Geo g,
     stage_twiddles<NX>(stw, tw, tid, NTH);
     pdl_wait();
     pdl_next();
-    const T* in[6] = {W0, W1, W2, W3, W4, W5};
+    const Handed<T> in[6] = {W0, W1, W2, W3, W4, W5};
     T v[EI][6];
 #pragma unroll
     for (int u = 0; u < EI; ++u) {
@@ -118,7 +117,8 @@ static void rf_row_slice(Ctx& c, const T* tw, const T* W0, const T* W1, const T*
     auto kern = k_rf_row_slice<NX, T, XM>;
     smem_attr(reinterpret_cast<const void*>(kern), smem);
     const int tok = c.prof_begin("real_rows_slice");
-    launch_pdl(c.stream, kern, unsigned(c.ny), slice_row_threads<NX>(), smem, c.geo(), tw, W0, W1, W2, W3, W4, W5, c.F.p, l, lw, Fd, fm);
+    launch_pdl(c.stream, kern, unsigned(c.ny), slice_row_threads<NX>(), smem, c.geo(), tw, Handed<T>{W0}, Handed<T>{W1},
+               Handed<T>{W2}, Handed<T>{W3}, Handed<T>{W4}, Handed<T>{W5}, c.F.p, l, lw, Fd, fm);
     c.check_launch("k_rf_row_slice");
     c.prof_end(tok);
 }
