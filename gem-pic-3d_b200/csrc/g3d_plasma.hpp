@@ -32,7 +32,7 @@ struct StepVals {
 };
 
 struct StreamArgs {
-    const float* __restrict__ F;
+    const float* F;            // (F, Fmid, Fd: no aliasing promises, see k_pdl.cuh)
     Geo g;
     LaserDev laser;
     const StepVals* sv;

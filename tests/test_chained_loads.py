@@ -96,3 +96,8 @@ def test_the_push_gathers_by_ordinary_loads():
         assert "__ldg" not in body and "__restrict__" not in body, m.group(1)
         seen += 1
     assert seen >= 5
+    hpp = sources()["g3d_plasma.hpp"]
+    args, _ = balanced(hpp, hpp.index("{", hpp.index("struct StreamArgs")), "{", "}")
+    for m in CHAIN["k_stream"][1]:
+        decl = [d for d in args.split(";") if re.search(r"\b" + m + r"$", d.strip())]
+        assert len(decl) == 1 and "__restrict__" not in decl[0], m
