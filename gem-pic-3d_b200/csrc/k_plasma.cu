@@ -24,6 +24,7 @@
 #include "g3d_plasma.hpp"
 #include "k_external.cuh"
 #include "k_pdl.cuh"
+#include "k_stream_mid.cuh"
 #include "k_fft.cuh"
 #include "k_dispatch.cuh"
 
@@ -132,53 +133,6 @@ __device__ __forceinline__ void sgather_exact(const StreamArgs& c, double x, dou
         const double v = (1 - fz) * v0 + fz * v1;
         if (comp < 3) E[comp] = v; else B[comp - 3] = v;
     }
-}
-// The streaming push's TSC on a periodic grid: the cell coordinate t = x / d and the nearest node in FP64 (x spans the
-// box, so the index needs the double), the offset from that node and the three weights in W (FP32 in the mixed form).
-// x may lie outside the box: the first index is wrapped (its two neighbours by a compare), and as a particle is rarely
-// more than a cell outside, the remainder (some twenty instructions) is behind a branch.
-template <class W>
-__device__ __forceinline__ void tsc_stream(double x, double inv_d, int n, int idx[3], W w[3]) {
-    const double t = x * inv_d;
-    const double c = floor(t + 0.5);
-    const W f = W(t - c);
-    w[0] = W(0.5) * (W(0.5) - f) * (W(0.5) - f);
-    w[1] = W(0.75) - f * f;
-    w[2] = W(0.5) * (W(0.5) + f) * (W(0.5) + f);
-    int b = int(c) - 1;
-    if (unsigned(b) >= unsigned(n)) { b %= n; if (b < 0) b += n; }
-    const int b1 = b + 1 == n ? 0 : b + 1;
-    idx[0] = b; idx[1] = b1; idx[2] = b1 + 1 == n ? 0 : b1 + 1;
-}
-// The gather half-way through the half-cell (zeta = the slice midpoint, a particle crossing the whole half-cell):
-// TSC in x and y of the interleaved midpoint fields, two (FP32) or three (FP64) vector loads per point (Fourier y).
-template <bool F32>
-__device__ __forceinline__ void sgather_mid(const StreamArgs& c, double x, double y, double E[3], double B[3]) {
-    typedef typename std::conditional<F32, float, double>::type R;
-    int ix[3], jn[3]; R wx[3], wn[3];
-    tsc_stream<R>(x, c.inv_dx, c.g.nx, ix, wx);
-    tsc_stream<R>(y, c.inv_dy, c.g.ny, jn, wn);
-    R a[6] = {0, 0, 0, 0, 0, 0};
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-        const int k0 = jn[j] * c.g.nx;
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const int k = k0 + ix[i];
-            const R w = wx[i] * wn[j];
-            if constexpr (F32) {
-                const float4* p = static_cast<const float4*>(c.Fmid) + 2 * k;
-                const float4 u = p[0], v = p[1];
-                a[0] += w * u.x; a[1] += w * u.y; a[2] += w * u.z; a[3] += w * u.w; a[4] += w * v.x; a[5] += w * v.y;
-            } else {
-                const double2* p = static_cast<const double2*>(c.Fmid) + 3 * k;
-                const double2 u = p[0], v = p[1], q = p[2];
-                a[0] += w * u.x; a[1] += w * u.y; a[2] += w * v.x; a[3] += w * v.y; a[4] += w * q.x; a[5] += w * q.y;
-            }
-        }
-    }
-    E[0] = double(a[0]); E[1] = double(a[1]); E[2] = double(a[2]);
-    B[0] = double(a[3]); B[1] = double(a[4]); B[2] = double(a[5]);
 }
 // The mixed form's midpoint gather on the free-hand y grid: per TSC point one float4 of the node row (E_x, E_z, B_y)
 // and one of the half-node row (E_y, B_x, B_z) of the interleaved midpoint fields, rows beyond the walls left out
@@ -508,7 +462,7 @@ __device__ __forceinline__ DepReq<typename DepType<F32, YF>::T> stream_one(const
         }
     } else {
         double Ed[3], Bd[3], Ee[3], Be[3];
-        if (YF && mid) sgather_mid<F32>(c, xm, ym, Ed, Bd);
+        if (YF && mid) sgather_midpoint<F32, LASER>(c, xm, ym, Ed, Bd);
         else if (EX) sgather_exact(c, wrapx(g, xm), wrapy<YF>(g, ym), zetam, Ed, Bd);
         else sgather<F32, YF>(c, wrapx(g, xm), wrapy<YF>(g, ym), zetam, Ed, Bd);
         if constexpr (LASER) {
