@@ -442,7 +442,7 @@ __device__ __forceinline__ DepReq<typename DepType<F32, YF>::T> stream_one(const
     const A px = A(px_), py = A(py_), pz = A(pz_), qm = A(qm_);
     // 1 - v_z = N / D with N = 1 + p_perp^2, D = gamma (gamma + p_z): no cancellation; gamma by rsqrt, which gives
     // 1/gamma too, and one quotient for the time (an FP64 quotient or root is 15 to 20 instructions here)
-    const A N0 = A(1) + px * px + py * py, a0 = N0 + pz * pz, ig0 = rsqrt(a0), g0 = a0 * ig0;
+    const A N0 = A(1) + px * px + py * py, a0 = N0 + pz * pz, ig0 = rsqrt(a0), g0 = gamma_root(a0, ig0);
     const A D0 = g0 * (g0 + pz);
     const A dt0 = A(hl) * D0 / N0;
     const A hd = A(0.5) * dt0 * ig0;
@@ -475,9 +475,8 @@ __device__ __forceinline__ DepReq<typename DepType<F32, YF>::T> stream_one(const
     A ux = px, uy = py, uz = pz, dt = dt0, ig1 = ig0;
     if (qm_ != 0) {                   // a neutral atom keeps u, and the time of its half-cell is dt0
         boris<A>(ux, uy, uz, E, B, qm, dt0);
-        // dt = 2 hl / ((1 - v_z)_0 + (1 - v_z)_1), over the common denominator
-        const A N1 = A(1) + ux * ux + uy * uy, a1 = N1 + uz * uz, g1 = a1 * rsqrt(a1), D1 = g1 * (g1 + uz);
-        dt = A(2) * A(hl) * D0 * D1 / (N0 * D1 + N1 * D0);
+        const A N1 = A(1) + ux * ux + uy * uy, a1 = N1 + uz * uz, g1 = gamma_root(a1, rsqrt(a1)), D1 = g1 * (g1 + uz);
+        dt = halfcell_time(hl, N0, D0, N1, D1);
         ux = px; uy = py; uz = pz;
         boris<A>(ux, uy, uz, E, B, qm, dt);
         ig1 = rsqrt(A(1) + ux * ux + uy * uy + uz * uz);

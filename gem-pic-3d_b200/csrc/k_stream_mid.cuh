@@ -1,11 +1,26 @@
-// Pieces of the streaming push (k_plasma.cu) that a host harness runs on the CPU as well (tests/stream_mid_check.cu): the TSC of
-// the Fourier y grid and the gather of the midpoint fields.
+// Pieces of the streaming push (k_plasma.cu) that a host harness runs on the CPU as well (tests/stream_mid_check.cu): gamma and
+// the time of a half-cell, the TSC of the Fourier y grid and the gather of the midpoint fields.
 #pragma once
 #include <type_traits>
 #include "g3d_plasma.hpp"
 
 namespace g3d {
 
+// gamma = sqrt(a) from r, the reciprocal root of a to a unit in its last place (which the push needs as well): a r is off by up
+// to 1.5 units, and a Newton step on the residual (exact in the FMA) leaves the root's own rounding. gamma + p_z needs that: for
+// a particle that runs backwards the sum cancels, to 1 / (2 |p_z|) of two numbers of size |p_z|, and with a r alone it lost
+// half as many bits again and from |p_z| ~ 5e7 on came out zero or negative. (A root beside the reciprocal root is some 20
+// instructions; this is three.) Never below |p_z| when a >= p_z^2.
+G3D_HD double gamma_root(double a, double r) {
+    const double t = a * r;
+    return fma(fma(-t, t, a), 0.5 * r, t);
+}
+// dt = 2 hl / ((1 - v_z)_0 + (1 - v_z)_1) with 1 - v_z = N / D, over the common denominator; D = 0 (gamma + p_z below the
+// resolution of FP64): the time is zero, as with the quotients N / D = infinity
+G3D_HD double halfcell_time(double hl, double N0, double D0, double N1, double D1) {
+    const double den = N0 * D1 + N1 * D0;
+    return den > 0 ? 2 * hl * D0 * D1 / den : 0.0;
+}
 // The streaming push's TSC on a periodic grid: the cell coordinate t = x / d and the nearest node in FP64 (x spans the
 // box, so the index needs the double), the offset from that node and the three weights in W.
 // x may lie outside the box: the first index is wrapped (its two neighbours by a compare), and as a particle is rarely

@@ -51,6 +51,35 @@ static double weight_error(bool ext) {
     return worst;
 }
 
+// The half-cell's time of a particle that runs backwards with p_z = -P, its reciprocal roots off by a unit in the last place:
+// gamma + p_z not below zero, the time finite and not negative, and its error no larger than the one of the textbook form
+// (roots and quotients, over the same draws).
+static bool backwards(double P, double& err, double& err_ref) {
+    std::mt19937_64 rng(9);
+    std::normal_distribution<double> G(0.0, 0.3);
+    std::uniform_real_distribution<double> U(0.0, 1.0);
+    bool ok = true;
+    err = err_ref = 0;
+    for (int k = 0; k < 3000; ++k) {
+        double N[2], D[2], omv[2], ex[2];
+        for (int s = 0; s < 2; ++s) {
+            const double px = k % 3 ? G(rng) : 0.0, py = k % 3 ? G(rng) : 0.0, pz = -P * (1 + 0.2 * U(rng));
+            N[s] = 1 + px * px + py * py;
+            const double a = N[s] + pz * pz, r = 1 / std::sqrt(a);
+            const double g = gamma_root(a, k % 2 ? std::nextafter(r, 0.0) : std::nextafter(r, 2.0)), gr = std::sqrt(a);
+            ok = ok && g + pz >= 0;
+            D[s] = g * (g + pz);
+            omv[s] = N[s] / (gr * (gr + pz));
+            ex[s] = 1 + std::fabs(pz) / std::sqrt(1 + px * px + py * py + pz * pz);       // 1 - v_z, nothing cancels
+        }
+        const double dt = halfcell_time(0.2, N[0], D[0], N[1], D[1]), ref = 2 * 0.2 / (omv[0] + omv[1]), want = 2 * 0.2 / (ex[0] + ex[1]);
+        ok = ok && std::isfinite(dt) && dt >= 0;
+        err = std::max(err, std::fabs(dt - want) / want);
+        err_ref = std::max(err_ref, std::fabs(ref - want) / want);
+    }
+    return ok;
+}
+
 int main() {
     // FP64 weights: the product's one rounding to FP32, 2^-24, and FP64 roundings (the offset of a weight of 1e-4: 1e-13)
     const double one = std::ldexp(1.0, -24) * (1 + 1e-5);
@@ -67,6 +96,13 @@ int main() {
     for (const auto& q : r) {
         std::printf("weights, %s: largest relative error %.3e (bound %.3e)\n", q.what, q.err, q.bound);
         bad += !(q.err <= q.bound);
+    }
+    for (double P : {0.01, 1.0, 30.0, 1e3, 1e5, 1e7, 4e7, 6e7, 1e8, 1e10, 1e30}) {
+        double err, ref;
+        const bool ok = backwards(P, err, ref);
+        const bool good = ok && err <= 1.02 * ref + 4e-16;              // the other form's products and quotients round otherwise
+        std::printf("time at p_z = -%g: %s, largest relative error %.3e (roots and quotients %.3e)\n", P, ok ? "sound" : "NOT SOUND", err, ref);
+        bad += !good;
     }
     return bad;
 }

@@ -1,6 +1,7 @@
 """Pieces of the streaming push (csrc/k_stream_mid.cuh) checked on the CPU: a host harness (tests/stream_mid_check.cu) built with
 nvcc compares the weights that the gather of the midpoint fields applies with their FP64 values. Where the mixed
-form adds an analytic wave or an external element the weights are FP64 and only their products are rounded to FP32."""
+form adds an analytic wave or an external element the weights are FP64 and only their products are rounded to FP32. The time of
+a half-cell is compared with the form by roots and quotients for particles that run backwards, where gamma + p_z cancels."""
 import os
 import shutil
 import subprocess
