@@ -251,6 +251,7 @@ struct Ctx {
     DevBuf<unsigned char> ckpt_snap;             // its device copy of the state, kept for the next one
     cudaStream_t stream = nullptr;
     long launches = 0;
+    long graph_marches = 0;                      // plasma marches whose slice loop was launched as a graph
     bool profiling = false;
     std::vector<ProfEntry> prof;
     std::vector<PendingEvent> pending;

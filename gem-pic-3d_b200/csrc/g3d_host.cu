@@ -2093,6 +2093,7 @@ int g3d_profile_get(g3d_ctx* ctx, int32_t k, const char** name, int64_t* launche
     });
 }
 int64_t g3d_launch_count(const g3d_ctx* ctx) { return ctx ? ctx->c.launches : 0; }
+int64_t g3d_graph_count(const g3d_ctx* ctx) { return ctx ? ctx->c.graph_marches : 0; }
 
 int g3d_set_laser_modes(g3d_ctx* ctx, const double* coef) { return guarded(ctx, [&] { g3d::set_laser_modes(ctx->c, coef); }); }
 int g3d_set_exact_fields(g3d_ctx* ctx, int32_t on) {

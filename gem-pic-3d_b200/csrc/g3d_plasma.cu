@@ -394,6 +394,16 @@ static void real_fields_slice(Ctx& c, int l, int target = -1, bool cols = true, 
     else launch_real_fields_slice(c, l, fm, cols);
 }
 
+// Transverse points below which the slice loop is captured as a graph. Direct launches cost the host some 2.5 us each, a graph of
+// some thousand to ten thousand nodes its capture and instantiation (2 to 4 ms more in the step that makes it, 160 slices) and
+// memory for its nodes. Step of 160 slices, two passes, direct -> graph:
+//   free-hand y (eight to ten launches per half-cell pass): 64 x 64 17.6 -> 15.0 ms, 96 x 96 19.2 -> 16.8, 128 x 128 23.8 -> 21.4
+//   (mixed 21.3 -> 18.5), 192 x 128 20.9 -> 17.8 (one particle a cell); 192 x 192 93 -> 85, mixed 77 -> 78: the device bounds it;
+//   Fourier y (four launches): 32 x 32 5.1 -> 4.5 ms, 48 x 32 4.9 -> 4.4; above the line 48 x 48 5.4 -> 5.0, 64 x 64 5.3 -> 5.0 are
+//   still gains of 5 to 10 % once the graph is made, but 48 x 48 x 400 12.4 to 14.1 -> 12.8 to 13.6, 64 x 64 x 1201 43.7 -> 42.8,
+//   and a long window's capture costs more than many steps.
+constexpr long GRAPH_POINTS_FREEHAND = 32768, GRAPH_POINTS_FOURIER = 2048;
+
 void march_plasma(Ctx& c, double s0, double s1) {
     PlasmaState& P = *c.pl;
     const double Delta = s1 - s0, D = 0.5 * Delta;
@@ -412,8 +422,8 @@ void march_plasma(Ctx& c, double s0, double s1) {
     G3D_CUDA(cudaMemcpyAsync(P.stepv.p, &stv, sizeof(StepVals), cudaMemcpyHostToDevice, c.stream));
     const bool ionz = P.born_cap > 0;
     const int passes = P.cfg.iterations;
-    // The slice loop is four launches per half-cell and pass on Fourier y, some eight on the free-hand grid. On the smallest
-    // grids the host's launch rate would bound it: there it runs as a CUDA graph, captured once per set of buffers it holds
+    // The slice loop is four launches per half-cell and pass on Fourier y, some eight on the free-hand grid. On small
+    // grids the host's launch rate would bound it (GRAPH_POINTS): there it runs as a CUDA graph, captured once per set of buffers it holds
     // by value (j0 and jk trade theirs every step) and launched every step after. It is captured again only when something it
     // holds changes (a buffer of the window moved, the capacity of the freed-electron list, the step length). The
     // streaming and freed-electron lists are reached through a descriptor on the device, so they may move. While per-kernel
@@ -511,18 +521,16 @@ void march_plasma(Ctx& c, double s0, double s1) {
         issue();
     } else if (hit) {
         c.launches += hit->launches;
+        ++c.graph_marches;
         G3D_CUDA(cudaGraphLaunch(hit->exec, c.stream));
     } else {
-        // Kernel by kernel: the device is what bounds a march on all but the smallest grids (a step of 48 x 48 x 400: 12.4 to
-        // 14.1 ms so, 12.8 to 13.6 ms as a graph; 64 x 64 x 1201: 43.7 and 42.8 ms), and a graph of some ten thousand nodes takes
-        // the host longer to capture and instantiate than many steps. On a smaller transverse grid the launches bound it
-        // (32 x 32 x 160: 5.1 to 5.5 against 4.5 ms): there the graph is made when a set of buffers comes a second time, by
-        // the host while the device works on the march (a capture records only what is issued during it, not the work in
-        // flight on the stream), for the marches to come.
+        // Kernel by kernel; on the small transverse grids, where the launches bound a march, the graph is made when a set of
+        // buffers comes a second time, by the host while the device works on the march (a capture records only what is
+        // issued during it, not the work in flight on the stream), for the marches to come.
         const long l0 = c.launches;
         issue();
         const long l1 = c.launches;
-        const bool small = long(c.nx) * c.ny < 2048, again = std::find(P.seen.begin(), P.seen.end(), key) != P.seen.end();
+        const bool small = long(c.nx) * c.ny < (c.yf ? GRAPH_POINTS_FOURIER : GRAPH_POINTS_FREEHAND), again = std::find(P.seen.begin(), P.seen.end(), key) != P.seen.end();
         if (small && !again) {
             if (P.seen.size() >= 8) P.seen.erase(P.seen.begin());
             P.seen.push_back(key);

@@ -289,6 +289,10 @@ class Simulation:
     def launch_count(self):
         return self.lib.g3d_launch_count(self.ctx)
 
+    def graph_count(self):
+        """Plasma marches whose slice loop was launched as a captured graph (the others: kernel by kernel)."""
+        return self.lib.g3d_graph_count(self.ctx)
+
     # ---------------------------------------------------------------- adjoint march
     def set_laser_modes(self, coef=None):
         """Laser mode coefficients a[j, kx] (complex, ny x (nx/2 + 1)) multiplying the grid lasers' spectra at

@@ -386,6 +386,8 @@ int32_t g3d_profile_count(const struct g3d_ctx* ctx);
 int g3d_profile_get(struct g3d_ctx* ctx, int32_t k, const char** name, int64_t* launches, double* total_ms);
 /* Kernel launches issued on this context since creation (all kernels, profiled or not). */
 int64_t g3d_launch_count(const struct g3d_ctx* ctx);
+/* Plasma marches of this context whose slice loop was launched as a captured CUDA graph (the others: kernel by kernel). */
+int64_t g3d_graph_count(const struct g3d_ctx* ctx);
 
 /* ------------------------------------------------------------------ adjoint march (no reference counterpart) */
 /* Laser mode coefficients: every grid laser's R spectrum added at init (Simulation::add_grid_lasers,

@@ -47,17 +47,38 @@ def test_step_matches_the_restatement(cases, form, nx, ny, nz, ppc, ions, passes
 
 
 def test_graph_and_direct_launches_agree(cases):
-    """The first march with a set of buffers is launched kernel by kernel, later ones as the captured graph; with the
+    """The first two marches with a set of buffers are launched kernel by kernel, later ones as the captured graph; with the
     kernels timed one by one every march is launched directly. All give the same run up to the order of the adds."""
     case = dict(kind="lwfa", nx=32, ny=32, nz=100, n=2000, form="fp64", ppc=2, ions=True, passes=2, smooth=0.0)
     out = []
     for profiled in (False, True):
         state = cases.prepare(case, 3)
         state["sim"].profile(profiled)
-        for _ in range(5):
+        for _ in range(6):
             cases.run(state)
+        assert state["sim"].graph_count() == (0 if profiled else 2)      # two sets of buffers take turns: steps 5 and 6
         out.append({a: state["sim"].array(a) for a in ("Rx", "Ry", "Ez", "F")})
         state["sim"].close()
     for a in out[0]:
         d, n = np.linalg.norm(out[0][a] - out[1][a]), np.linalg.norm(out[1][a])
-        assert d <= 1e-8 * n, (a, d / n)       # five steps amplify the adds' rounding (1e-16) by the wake's growth
+        assert d <= 1e-8 * n, (a, d / n)       # six steps amplify the adds' rounding (1e-16) by the wake's growth
+
+
+@pytest.mark.parametrize("nx,half,form,graph", [(16, 12, "fp64", True), (64, 32, "fp64", True), (64, 32, "mixed", True),
+                                                (256, 64, "mixed", False), (48, None, "fp64", False), (32, None, "mixed", True)])
+def test_small_grids_march_as_a_graph(nx, half, form, graph):
+    """Which grids' slice loop becomes a graph (GRAPH_POINTS in csrc/g3d_plasma.cu): the free-hand grid's loop has twice the
+    launches and is bound by them up to larger grids."""
+    from g3d import Simulation, configs
+    cfg = configs.lwfa_small(nx=nx, ny=nx, nzeta=24, nmacro=500, steps=6, ppc=1)
+    if half:
+        configs.on_freehand_y(cfg, half=half, grow=1.03)
+    s = Simulation(cfg, precision=form)
+    try:
+        s.init()
+        for _ in range(6):
+            s.step()
+        assert (s.graph_count() > 0) == graph
+        assert np.isfinite(s.array("Ez")).all()
+    finally:
+        s.close()
