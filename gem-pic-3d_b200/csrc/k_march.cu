@@ -327,11 +327,10 @@ void launch_march_f(Ctx& c, double D) {
 
 static void comoving_launch(Ctx& c, const Geo& g, const cpx* jz, double* cpb, cpx* dpb, cpx* Rx, cpx* Ry, cpx* Ez, cpx* Bz,
                             double beta, double gm2) {
-    const int tok = c.prof_begin("comoving");
-    if (!comoving_parallel<cpx>(c, g, jz, Rx, Ry, Ez, Bz, beta, gm2)) {
-        k_comoving<<<unsigned((g.nkh + 127) / 128), 128, 0, c.stream>>>(g, jz, cpb, dpb, Rx, Ry, Ez, Bz, beta, gm2);
-        c.check_launch("k_comoving");
-    }
+    if (comoving_parallel<cpx>(c, g, jz, Rx, Ry, Ez, Bz, beta, gm2)) return;
+    const int tok = c.prof_begin("comoving_sweep");
+    k_comoving<<<unsigned((g.nkh + 127) / 128), 128, 0, c.stream>>>(g, jz, cpb, dpb, Rx, Ry, Ez, Bz, beta, gm2);
+    c.check_launch("k_comoving");
     c.prof_end(tok);
 }
 void launch_comoving(Ctx& c, double beta, double gm2) {

@@ -440,9 +440,11 @@ void launch_comoving_f(Ctx& c, double beta, double gm2) {
     if (comoving_parallel<cpxf>(c, c.geo(), c.mx.jkz.p, c.Rx.p, c.Ry.p, c.mx.Ez.p, c.mx.Bz.p, beta, gm2)) return;
     DevBuf<cpx> dp;
     dp.alloc(size_t(c.ns) * c.nkh, c.stream);
+    const int tok = c.prof_begin("comoving_sweep");
     k_comoving_mixed<<<unsigned((c.nkh + 127) / 128), 128, 0, c.stream>>>(c.geo(), c.mx.jkz.p, c.rscratch.p, dp.p, c.Rx.p, c.Ry.p,
                                                                           c.mx.Ez.p, c.mx.Bz.p, beta, gm2);
     c.check_launch("k_comoving_mixed");
+    c.prof_end(tok);
     G3D_CUDA(cudaStreamSynchronize(c.stream));
 }
 template <int NY>
