@@ -479,12 +479,14 @@ void launch_sponge(Ctx& c) {
     G3D_DISPATCH_N(c.ny, NY, sp_cols_fwd<NY>(c));
 }
 
-// one slice (the plasma march): tiles of 2 columns, so that 3 x 65 CTAs spread the slice's latency over the SMs
-template <int NY, int CWT, bool COMB>
+// What W holds is asked for by the caller: COMB, the whole window, whose rows kernel takes the components; else one slice (of the
+// plasma march, whose rows combine), in tiles of 2 columns, so that 3 x 65 CTAs spread the slice's latency over the SMs.
+template <int NY, bool COMB>
 static void rf_cols_w(Ctx& c, int l0, int nl) {
+    constexpr int CWT = COMB ? CW : 2;
     const size_t smem = size_t(2) * ColTile<NY, CWT>::size * sizeof(cpx);
     allow_smem(k_rf_cols<NY, CWT, COMB>, smem);
-    const int tok = c.prof_begin(nl == 1 ? "real_cols_slice" : "real_cols");
+    const int tok = c.prof_begin(COMB ? "real_cols" : "real_cols_slice");
     k_rf_cols<NY, CWT, COMB><<<dim3(unsigned((c.H + CWT - 1) / CWT), unsigned(nl), 3), CWT * FftShape<NY>::T, smem, c.stream>>>(
         c.geo(), c.Rx.p, c.Ry.p, c.Lx.p, c.Ly.p, c.Ez.p, c.Bz.p, c.W[0].p, c.W[1].p, c.W[2].p, c.W[3].p, c.W[4].p, c.W[5].p, l0);
     c.check_launch("k_rf_cols");
@@ -497,25 +499,24 @@ static bool rf_maps(Ctx& c) {
     return c.tma_rf.get(p, 6, c.H, long(c.ns) * c.ny, c.ny);
 }
 template <int NY>
-static void rf_cols_tma(Ctx& c, int l0, int nl) {
+static void rf_cols_tma(Ctx& c) {
     const size_t smem = size_t(2) * NY * 8 * sizeof(cpx) + 128;
     allow_smem(k_rf_cols_tma<NY>, smem);
     const int tok = c.prof_begin("real_cols");
-    k_rf_cols_tma<NY><<<dim3(unsigned((c.H + 7) / 8), unsigned(nl), 3), 8 * FftShape<NY>::T, smem, c.stream>>>(
-        c.geo(), c.tma_rf.maps, c.W[0].p, c.W[1].p, c.W[2].p, c.W[3].p, c.W[4].p, c.W[5].p, l0, c.tma_wait());
+    k_rf_cols_tma<NY><<<dim3(unsigned((c.H + 7) / 8), unsigned(c.ns), 3), 8 * FftShape<NY>::T, smem, c.stream>>>(
+        c.geo(), c.tma_rf.maps, c.W[0].p, c.W[1].p, c.W[2].p, c.W[3].p, c.W[4].p, c.W[5].p, 0, c.tma_wait());
     c.check_launch("k_rf_cols_tma");
     c.prof_end(tok);
 }
 template <int NY>
-static void rf_cols(Ctx& c, int l0, int nl) {
-    if (nl == 1) { rf_cols_w<NY, 2, false>(c, l0, nl); return; }
+static void rf_cols(Ctx& c) {
     if constexpr (NY <= 256 && (NY & (NY - 1)) == 0) {
-        if (c.use_tma && rf_maps(c)) { rf_cols_tma<NY>(c, l0, nl); return; }
+        if (c.use_tma && rf_maps(c)) { rf_cols_tma<NY>(c); return; }
     }
-    rf_cols_w<NY, CW, true>(c, l0, nl);
+    rf_cols_w<NY, true>(c, 0, c.ns);
 }
 void launch_real_fields(Ctx& c) {
-    G3D_DISPATCH_N(c.ny, NY, rf_cols<NY>(c, 0, c.ns));
+    G3D_DISPATCH_N(c.ny, NY, rf_cols<NY>(c));
     G3D_DISPATCH_N(c.nx, NX, (rf_rows<NX, cpx, false>(c, c.twx.p, c.W[0].p, c.W[1].p, c.W[2].p, c.W[3].p, c.W[4].p, c.W[5].p, c.Fd.p)));
 }
 // free-hand y: the spectra are already real in y; one inverse transform along x per row of R, L and E_z + i B_z
@@ -530,7 +531,7 @@ void launch_sp_rows(Ctx& c) { G3D_DISPATCH_N(c.nx, NX, sp_rows<NX>(c)); }
 // E and B of one slice (plane l) in real space (Simulation::real_fields_slice, src/sim_plasma.cpp:200-220). cols: the
 // columns too (into plane l of W); else they are in plane 0 of W, where k_pass_cols left them
 void launch_real_fields_slice(Ctx& c, int l, FmidOut fm, bool cols) {
-    if (cols) G3D_DISPATCH_N(c.ny, NY, rf_cols<NY>(c, l, 1));
+    if (cols) G3D_DISPATCH_N(c.ny, NY, (rf_cols_w<NY, false>(c, l, 1)));
     const cpx* W[6] = {c.W[0].p, c.W[1].p, c.W[2].p, c.W[3].p, c.W[4].p, c.W[5].p};
     const int lw = cols ? l : 0;
     if (c.Fd.p && fm.out && !fm.f32 && !fm.fh)         // exact fields: unrounded midpoint fields

@@ -483,11 +483,13 @@ void launch_sponge_f(Ctx& c) {
     G3D_DISPATCH_N(c.nx, NX, sp_rows_f<NX>(c));
     G3D_DISPATCH_N(c.ny, NY, sp_cols_fwd_f<NY>(c));
 }
-template <int NY, int CWT, bool COMB>
-static void rf_cols_fw(Ctx& c, int l0, int nl) {
+// COMB, tiles: as rf_cols_w (k_fields.cu)
+template <int NY, bool COMB>
+static void rf_cols_f(Ctx& c, int l0, int nl) {
+    constexpr int CWT = COMB ? CW : 2;
     const size_t smem = size_t(2) * ColTile<NY, CWT>::size * sizeof(cpxf);
     allow_smem(k_rf_cols_f<NY, CWT, COMB>, smem);
-    const int tok = c.prof_begin(nl == 1 ? "real_cols_slice" : "real_cols");
+    const int tok = c.prof_begin(COMB ? "real_cols" : "real_cols_slice");
     auto& m = c.mx;
     k_rf_cols_f<NY, CWT, COMB><<<dim3(unsigned((c.H + CWT - 1) / CWT), unsigned(nl), 3), CWT * FftShape<NY>::T, smem, c.stream>>>(
         c.geo(), m.twy.p, c.Rx.p, c.Ry.p, m.Lx.p, m.Ly.p, m.Ez.p, m.Bz.p, m.W[0].p, m.W[1].p, m.W[2].p, m.W[3].p, m.W[4].p, m.W[5].p,
@@ -495,20 +497,14 @@ static void rf_cols_fw(Ctx& c, int l0, int nl) {
     c.check_launch("k_rf_cols_f");
     c.prof_end(tok);
 }
-// one slice (the plasma march): tiles of 2 columns, so that 3 x 65 CTAs spread the slice's latency over the SMs
-template <int NY>
-static void rf_cols_f(Ctx& c, int l0, int nl) {
-    if (nl == 1) rf_cols_fw<NY, 2, false>(c, l0, nl);
-    else rf_cols_fw<NY, CW, true>(c, l0, nl);
-}
 void launch_real_fields_f(Ctx& c) {
-    G3D_DISPATCH_N(c.ny, NY, rf_cols_f<NY>(c, 0, c.ns));
+    G3D_DISPATCH_N(c.ny, NY, (rf_cols_f<NY, true>(c, 0, c.ns)));
     launch_rf_rows_f(c);
 }
 // E and B of one slice (plane l) of the mixed form (the real fields of one slice of the plasma march); cols: the columns
 // too (into plane l of W); else they are in plane 0 of W, where k_pass_cols left them
 void launch_real_fields_slice_f(Ctx& c, int l, FmidOut fm, bool cols) {
-    if (cols) G3D_DISPATCH_N(c.ny, NY, rf_cols_f<NY>(c, l, 1));
+    if (cols) G3D_DISPATCH_N(c.ny, NY, (rf_cols_f<NY, false>(c, l, 1)));
     auto& m = c.mx;
     G3D_DISPATCH_N(c.nx, NX, (rf_row_slice<NX, cpxf, false>(c, m.twx.p, m.W[0].p, m.W[1].p, m.W[2].p, m.W[3].p, m.W[4].p, m.W[5].p, l,
                                                             cols ? l : 0, nullptr, fm)));
