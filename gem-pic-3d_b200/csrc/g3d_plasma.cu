@@ -33,7 +33,7 @@ PlasmaPtrs PlasmaState::ptrs(const Ctx& c) const {
     if (c.mixed) { p.jkx = c.mx.jkx.p; p.jky = c.mx.jky.p; p.jkz = c.mx.jkz.p; }
     else { p.jkx = c.jkx.p; p.jky = c.jky.p; p.jkz = c.jkz.p; }
     p.js0x = js0x.p; p.js0y = js0y.p; p.js0z = js0z.p;
-    p.jsn = jsn.p; p.sin_ = jsin.p; p.si0 = jsi0.p; p.pin = jpred.p; p.tmp = jtmp.p; p.dl = dlt.p;
+    p.jsn = jsn.p; p.sin_ = jsin.p; p.si0 = jsi0.p; p.pin = jpred.p; p.dl = dlt.p;
     return p;
 }
 
@@ -109,8 +109,11 @@ void set_plasma(Ctx& c, const g3d_plasma& P, const g3d_ion* ions, int nions) {
     if (c.yf || c.f32s) pl->fmid.alloc(size_t(6) * c.nk, s);      // 6 doubles or 8 floats per point
     pl->rhol.alloc(size_t(pl->ion_lines ? 2 : 1) * size_t(c.N) * size_t(c.nx + c.ny), s);
     pl->stepv.alloc(1, s);
-    for (DevBuf<cpx>* b : {&pl->jsn, &pl->jsin, &pl->jpred, &pl->jtmp, &pl->jsi0, &pl->dlt, &pl->tsp}) b->alloc(3 * ph, s);
-    pl->bk.alloc(4 * ph, s);
+    for (DevBuf<cpx>* b : {&pl->jpred, &pl->dlt, &pl->tsp}) b->alloc(3 * ph, s);
+    if (!c.yf) {                                       // Fourier y: k_pass_cols keeps these in registers
+        for (DevBuf<cpx>* b : {&pl->jsn, &pl->jsin, &pl->jsi0}) b->alloc(3 * ph, s);
+        pl->bk.alloc(4 * ph, s);
+    }
     pl->nstrm_dev.alloc(1, s);
     pl->sdev.alloc(2, s);
     pl->bcnt.alloc(1, s);

@@ -79,7 +79,7 @@ struct RecDev {
 struct PlasmaPtrs {
     long nkh;
     void *jkx, *jky, *jkz;     // the window's jk: complex128, or complex64 in the mixed form
-    cpx *js0x, *js0y, *js0z, *jsn, *sin_, *si0, *pin, *tmp, *dl;
+    cpx *js0x, *js0y, *js0z, *jsn, *sin_, *si0, *pin, *dl;
 };
 
 struct IonSpec {
@@ -133,8 +133,9 @@ struct PlasmaState {
     // column i0), deposited by the last pass: the negative particles, then (ion_lines) the positive ones
     DevBuf<double> rhol;
     bool ion_lines = false;                    // some ion species is loaded (mobile or ionizing)
-    DevBuf<cpx> jsn, jsin, jpred, jtmp, jsi0, dlt, tsp;   // 3 half planes each
-    DevBuf<cpx> bk;                            // 4 half planes: R_x, R_y, E_z, B_z of the slice
+    DevBuf<cpx> jpred, dlt, tsp;               // 3 half planes each
+    DevBuf<cpx> jsn, jsin, jsi0;               // free-hand y: the same
+    DevBuf<cpx> bk;                            // free-hand y: 4 half planes, R_x, R_y, E_z, B_z of the slice
     StrmBuf s, bn;                             // streaming particles, the freed electrons
     StrmDev strm{}, born{};
     StrmDev sdh[2]{};                          // strm and born as the kernels of the slice loop read them (sdev)
@@ -228,7 +229,7 @@ void launch_slice_prologue(Ctx& c, int n, int pred_m, int copy_in, int backup);
 void launch_pass_prologue(Ctx& c, int n, int restore);
 void launch_stream_spectra(Ctx& c);
 // Fourier y: the rows of the streaming current's spectra, then the fused column work of a pass (the current's
-// y transforms and filters, the replace and march of slice n, the y transforms of slice n's fields into W)
+// y transforms and filters, the prediction and the march of slice n, the y transforms of slice n's fields into W)
 void launch_stream_spectra_rows(Ctx& c);
 void launch_front(Ctx& c, double D);
 void launch_pass_cols(Ctx& c, double D, int n, int extrap, double w, double q, bool last);

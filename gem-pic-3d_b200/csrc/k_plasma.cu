@@ -799,11 +799,10 @@ __global__ void __launch_bounds__(slice_row_threads<NX>()) k_ss_rows(Geo g, JT* 
         T2[o] = a1[kx + (kx >> 3)];
     }
 }
-// columns: FFT along y, filters and smoothing -> jsn (3 half planes)
+// columns: FFT along y of three half planes (the profiles of the grid lasers; the currents' columns are in k_pass_cols)
 template <int NY, int CW>
 __global__ void __launch_bounds__(CW * FftShape<NY>::T) k_ss_cols(Geo g, const cpx* __restrict__ T0, const cpx* __restrict__ T1,
-                                                                  const cpx* __restrict__ T2, cpx* __restrict__ out, double a2, int keep0,
-                                                                  int filter) {
+                                                                  const cpx* __restrict__ T2, cpx* __restrict__ out) {
     using S = FftShape<NY>;
     extern __shared__ cpx sm[];
     cpx* s0 = sm;
@@ -825,39 +824,28 @@ __global__ void __launch_bounds__(CW * FftShape<NY>::T) k_ss_cols(Geo g, const c
     }
     const long nkh = g.nkh;
     constexpr int EPT = NY / S::T;            // elements of a thread (e = tid + u nthr)
-    double f[EPT];
-#pragma unroll
-    for (int u = 0; u < EPT; ++u) {            // the filter factors first: their loads wait for no store
-        const int e = tid + u * nthr, p = e / CW, kx = c0 + (e - p * CW);
-        f[u] = 0;
-        if (kx < H) {
-            const double k2 = g.kxs[kx] * g.kxs[kx] + g.kys[p] * g.kys[p];
-            f[u] = !filter ? 1.0 : (kx == 0 && p == 0 && !keep0) ? 0.0 : g.filt[kx] * g.filty[p] / (1 + a2 * k2);
-        }
-    }
 #pragma unroll
     for (int u = 0; u < EPT; ++u) {
         const int e = tid + u * nthr, p = e / CW, cc = e - p * CW, kx = c0 + cc;
         if (kx >= H) continue;
         const long o = long(p) * H + kx;
-        out[o] = f[u] * s0[ColTile<NY, CW>::at(p, cc)];
-        out[nkh + o] = f[u] * s1[ColTile<NY, CW>::at(p, cc)];
-        out[2 * nkh + o] = f[u] * s2[ColTile<NY, CW>::at(p, cc)];
+        out[o] = s0[ColTile<NY, CW>::at(p, cc)];
+        out[nkh + o] = s1[ColTile<NY, CW>::at(p, cc)];
+        out[2 * nkh + o] = s2[ColTile<NY, CW>::at(p, cc)];
     }
 }
 
-// ---------------------------------------------------------------- elementwise steps of the half-cell
+// ---------------------------------------------------------------- elementwise steps of the half-cell (free-hand y)
 // after a pass: replace the streaming part of jk(n) by jsn (old = sin); with the extrapolating predictor and
 // n >= 1 the prediction of half-cell n-1: tmp = js0(n-1) + d + w (d - dl), d = jsn - js0(n); replace(n-1, pin, tmp)
-template <class T>
 __device__ __forceinline__ void replace_pred_mode(const PlasmaPtrs& p, int n, int extrap, double w, long i) {
     const long nkh = p.nkh;
     const long hp = long(n + 1) * nkh, hq = long(n) * nkh;        // planes of half-cells n and n-1 (a = 0)
     cpx u[3];
     for (int k = 0; k < 3; ++k) u[k] = p.jsn[k * nkh + i];
-    T* jk[3] = {static_cast<T*>(p.jkx), static_cast<T*>(p.jky), static_cast<T*>(p.jkz)};
+    cpx* jk[3] = {static_cast<cpx*>(p.jkx), static_cast<cpx*>(p.jky), static_cast<cpx*>(p.jkz)};
     for (int k = 0; k < 3; ++k) {
-        jk[k][hp + i] = narrow<T>(widen(jk[k][hp + i]) + u[k] - p.sin_[k * nkh + i]);
+        jk[k][hp + i] = jk[k][hp + i] + u[k] - p.sin_[k * nkh + i];
         p.sin_[k * nkh + i] = u[k];
     }
     if (extrap && n >= 1) {
@@ -865,15 +853,14 @@ __device__ __forceinline__ void replace_pred_mode(const PlasmaPtrs& p, int n, in
         for (int k = 0; k < 3; ++k) {
             const cpx d = u[k] - s0[k][hp + i];
             const cpx t = s0[k][hq + i] + d + w * (d - p.dl[k * nkh + i]);
-            jk[k][hq + i] = narrow<T>(widen(jk[k][hq + i]) + t - p.pin[k * nkh + i]);
+            jk[k][hq + i] = jk[k][hq + i] + t - p.pin[k * nkh + i];
             p.pin[k * nkh + i] = t;
         }
     }
 }
-template <class T>
 __global__ void k_replace_pred(PlasmaPtrs p, int n, int extrap, double w) {
     for (long i = long(blockIdx.x) * blockDim.x + threadIdx.x; i < p.nkh; i += long(gridDim.x) * blockDim.x)
-        replace_pred_mode<T>(p, n, extrap, w, i);
+        replace_pred_mode(p, n, extrap, w, i);
 }
 // half-cell n is final (sim_plasma.cpp:381-403): R at slice n+1 corrected for the prediction it used; the
 // change s0 -> s1 kept for the extrapolation; the current kept as the prediction of the next step
@@ -1093,16 +1080,15 @@ __global__ void k_count_add(long* __restrict__ nstrm_dev, const int* __restrict_
     if (cnt <= bcap) *nstrm_dev += cnt;
 }
 
-// ---------------------------------------------------------------- per half-cell set-up, fused
+// ---------------------------------------------------------------- per half-cell set-up, fused (free-hand y)
 // Start of half-cell n (sim_plasma.cpp:236-262): sin <- pin and si0 <- pin (copy_in); the prediction of half-cell
 // pred_m starts from its level s0 with the prediction buffer cleared: jk(pred_m) += js0(pred_m), pin <- js0(pred_m)
 // (pred_m < 0: none); the slice's R_x, R_y, E_z, B_z saved for the passes (backup).
-template <class T>
 __device__ __forceinline__ void slice_prologue_mode(const PlasmaPtrs& p, cpx* sin_, cpx* si0, cpx* bk, const cpx* Rx, const cpx* Ry,
-                                                    const T* Ez, const T* Bz, long o, int pred_m, int copy_in, int backup, long i) {
+                                                    const cpx* Ez, const cpx* Bz, long o, int pred_m, int copy_in, int backup, long i) {
     const long nkh = p.nkh;
     const long hm = long(pred_m + 1) * nkh;
-    T* jk[3] = {static_cast<T*>(p.jkx), static_cast<T*>(p.jky), static_cast<T*>(p.jkz)};
+    cpx* jk[3] = {static_cast<cpx*>(p.jkx), static_cast<cpx*>(p.jky), static_cast<cpx*>(p.jkz)};
     const cpx* s0[3] = {p.js0x, p.js0y, p.js0z};
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -1110,34 +1096,32 @@ __device__ __forceinline__ void slice_prologue_mode(const PlasmaPtrs& p, cpx* si
         if (copy_in) { const cpx v = p.pin[q]; sin_[q] = v; si0[q] = v; }
         if (pred_m >= 0) {
             const cpx t = s0[k][hm + i];
-            jk[k][hm + i] = narrow<T>(widen(jk[k][hm + i]) + t);
+            jk[k][hm + i] = jk[k][hm + i] + t;
             p.pin[q] = t;
         }
     }
     if (backup) {
         bk[i] = Rx[o + i]; bk[nkh + i] = Ry[o + i];
-        bk[2 * nkh + i] = widen(Ez[o + i]); bk[3 * nkh + i] = widen(Bz[o + i]);
+        bk[2 * nkh + i] = Ez[o + i]; bk[3 * nkh + i] = Bz[o + i];
     }
 }
-template <class T>
 __global__ void k_slice_prologue(PlasmaPtrs p, cpx* __restrict__ sin_, cpx* __restrict__ si0, cpx* __restrict__ bk,
-                                 const cpx* __restrict__ Rx, const cpx* __restrict__ Ry, const T* __restrict__ Ez,
-                                 const T* __restrict__ Bz, long o, int pred_m, int copy_in, int backup) {
+                                 const cpx* __restrict__ Rx, const cpx* __restrict__ Ry, const cpx* __restrict__ Ez,
+                                 const cpx* __restrict__ Bz, long o, int pred_m, int copy_in, int backup) {
     for (long i = long(blockIdx.x) * blockDim.x + threadIdx.x; i < p.nkh; i += long(gridDim.x) * blockDim.x)
-        slice_prologue_mode<T>(p, sin_, si0, bk, Rx, Ry, Ez, Bz, o, pred_m, copy_in, backup, i);
+        slice_prologue_mode(p, sin_, si0, bk, Rx, Ry, Ez, Bz, o, pred_m, copy_in, backup, i);
 }
 // half-cell n final (correct_mode) and the prologue of half-cell n-1 (slice_prologue_mode, copy_in), per mode in
 // one thread. Every value is loaded before anything is stored: the correction reads si0 before the prologue
 // refills it, the prologue's slice n-1 and half-cell n-1 are not touched by the correction (slice n+1, half-cell
 // n), and pin and jk are each read before they are written; so the stores see the values of the sequential
 // code, and the ~26 loads of a mode wait together instead of behind stores they might alias.
-template <class T>
 __global__ void k_correct_prologue(PlasmaPtrs p, cpx* __restrict__ Rx, cpx* __restrict__ Ry, int n, double q, int own,
-                                   cpx* __restrict__ sin_, cpx* __restrict__ si0, cpx* __restrict__ bk, const T* __restrict__ Ez,
-                                   const T* __restrict__ Bz, long o_next, int pred_m, int backup) {
+                                   cpx* __restrict__ sin_, cpx* __restrict__ si0, cpx* __restrict__ bk, const cpx* __restrict__ Ez,
+                                   const cpx* __restrict__ Bz, long o_next, int pred_m, int backup) {
     const long nkh = p.nkh, hp = long(n + 1) * nkh, hm = long(pred_m + 1) * nkh;
     cpx* s0[3] = {p.js0x, p.js0y, p.js0z};
-    T* jk[3] = {static_cast<T*>(p.jkx), static_cast<T*>(p.jky), static_cast<T*>(p.jkz)};
+    cpx* jk[3] = {static_cast<cpx*>(p.jkx), static_cast<cpx*>(p.jky), static_cast<cpx*>(p.jkz)};
     const bool pred = pred_m >= 0;
     for (long i = long(blockIdx.x) * blockDim.x + threadIdx.x; i < nkh; i += long(gridDim.x) * blockDim.x) {
         cpx u[3], sh[3], pn[3], t[3], jm[3], sx = C(0), sy = C(0), rx = C(0), ry = C(0);
@@ -1146,33 +1130,33 @@ __global__ void k_correct_prologue(PlasmaPtrs p, cpx* __restrict__ Rx, cpx* __re
         for (int k = 0; k < 3; ++k) {
             u[k] = p.jsn[k * nkh + i]; sh[k] = s0[k][hp + i]; pn[k] = p.pin[k * nkh + i];
             t[k] = pred ? s0[k][hm + i] : C(0);
-            jm[k] = pred ? widen(jk[k][hm + i]) : C(0);
+            jm[k] = pred ? jk[k][hm + i] : C(0);
         }
         if (own) { sx = p.si0[i]; sy = p.si0[nkh + i]; rx = Rx[hp + i]; ry = Ry[hp + i]; }
-        if (backup) { b0 = Rx[o_next + i]; b1 = Ry[o_next + i]; b2 = widen(Ez[o_next + i]); b3 = widen(Bz[o_next + i]); }
+        if (backup) { b0 = Rx[o_next + i]; b1 = Ry[o_next + i]; b2 = Ez[o_next + i]; b3 = Bz[o_next + i]; }
         if (own) { Rx[hp + i] = rx - q * (u[0] - sx); Ry[hp + i] = ry - q * (u[1] - sy); }
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             p.dl[k * nkh + i] = u[k] - sh[k];
             s0[k][hp + i] = u[k];
             sin_[k * nkh + i] = pn[k]; si0[k * nkh + i] = pn[k];
-            if (pred) { jk[k][hm + i] = narrow<T>(jm[k] + t[k]); p.pin[k * nkh + i] = t[k]; }
+            if (pred) { jk[k][hm + i] = jm[k] + t[k]; p.pin[k * nkh + i] = t[k]; }
         }
         if (backup) { bk[i] = b0; bk[nkh + i] = b1; bk[2 * nkh + i] = b2; bk[3 * nkh + i] = b3; }
     }
 }
 // Start of a pass on the free-hand y grid: the slice restored from the backup (restore), the streaming-current
-// planes and the count of freed electrons cleared. (Fourier y: the fused march reads the backup, the rows kernel
-// of the spectra clears the planes and the count.)
-template <class T, class JT>
-__global__ void k_pass_prologue(const cpx* __restrict__ bk, cpx* __restrict__ Rx, cpx* __restrict__ Ry, T* __restrict__ Ez,
-                                T* __restrict__ Bz, long o, long nkh, JT* __restrict__ J, long nj, int* __restrict__ bcnt,
+// planes and the count of freed electrons cleared. (Fourier y: k_pass_cols leaves the slice as it is until the last pass, the
+// rows kernel of the spectra clears the planes and the count.)
+template <class JT>
+__global__ void k_pass_prologue(const cpx* __restrict__ bk, cpx* __restrict__ Rx, cpx* __restrict__ Ry, cpx* __restrict__ Ez,
+                                cpx* __restrict__ Bz, long o, long nkh, JT* __restrict__ J, long nj, int* __restrict__ bcnt,
                                 int restore) {
     const long t0 = long(blockIdx.x) * blockDim.x + threadIdx.x, st = long(gridDim.x) * blockDim.x;
     if (restore)
         for (long i = t0; i < nkh; i += st) {
             Rx[o + i] = bk[i]; Ry[o + i] = bk[nkh + i];
-            Ez[o + i] = narrow<T>(bk[2 * nkh + i]); Bz[o + i] = narrow<T>(bk[3 * nkh + i]);
+            Ez[o + i] = bk[2 * nkh + i]; Bz[o + i] = bk[3 * nkh + i];
         }
     for (long i = t0; i < nj; i += st) J[i] = JT(0);
     if (t0 == 0) *bcnt = 0;
@@ -1300,28 +1284,24 @@ static void ss_rows(Ctx& c, JT* J, cpx* T, int clear = 0, int* bcnt = nullptr) {
     c.check_launch("k_ss_rows");
 }
 template <int NY>
-static void ss_cols(Ctx& c, const cpx* T, cpx* out, double a2, int keep0, int filter) {
+static void ss_cols(Ctx& c, const cpx* T, cpx* out) {
     constexpr int CW = 2;              // one slice: 2-column tiles spread its latency over 65 SMs (measured: 8 used 17)
     const size_t smem = size_t(3) * ColTile<NY, CW>::size * sizeof(cpx);
     smem_attr(reinterpret_cast<const void*>(k_ss_cols<NY, CW>), smem);
     k_ss_cols<NY, CW><<<unsigned((c.H + CW - 1) / CW), CW * FftShape<NY>::T, smem, c.stream>>>(
-        c.geo(), T, T + c.nkh, T + 2 * c.nkh, out, a2, keep0, filter);
+        c.geo(), T, T + c.nkh, T + 2 * c.nkh, out);
     c.check_launch("k_ss_cols");
 }
+// free-hand y: the spectra of the streaming current, rows and then the filters along the y lines
 void launch_stream_spectra(Ctx& c) {
     const int tok = c.prof_begin("stream_spectra");
     PlasmaState& P = *c.pl;
-    const double a2 = P.cfg.smooth_length * P.cfg.smooth_length;
-    if (c.f32s && c.yf) {
-        float4* J4 = reinterpret_cast<float4*>(P.jsrf.p);
-        G3D_DISPATCH_N(c.nx, NX, (ss_rows<NX, float4>(c, J4, P.tsp.p, 1, P.bcnt.p)));
-    } else if (c.f32s) {
+    if (c.f32s) {
         G3D_DISPATCH_N(c.nx, NX, (ss_rows<NX, float>(c, P.jsrf.p, P.tsp.p, 1, P.bcnt.p)));
     } else {
         G3D_DISPATCH_N(c.nx, NX, (ss_rows<NX, double>(c, P.jsr.p, P.tsp.p, 1, P.bcnt.p)));
     }
-    if (!c.yf) launch_ss_lines_fh(c, P.tsp.p, P.jsn.p, a2);           // free-hand y: filters along the y lines
-    else G3D_DISPATCH_N(c.ny, NY, ss_cols<NY>(c, P.tsp.p, P.jsn.p, a2, P.box_mean ? 1 : 0, 1));
+    launch_ss_lines_fh(c, P.tsp.p, P.jsn.p, P.cfg.smooth_length * P.cfg.smooth_length);
     c.prof_end(tok);
 }
 // plain transverse spectra (no filters) of three real planes: the grid-laser profile (free-hand y: the x spectra
@@ -1330,7 +1310,7 @@ void launch_real_to_half3(Ctx& c, const double* J3, cpx* T3, cpx* out3) {
     double* J = const_cast<double*>(J3);      // read only: the rows kernel clears nothing here
     if (!c.yf) { G3D_DISPATCH_N(c.nx, NX, (ss_rows<NX, double>(c, J, out3))); return; }
     G3D_DISPATCH_N(c.nx, NX, (ss_rows<NX, double>(c, J, T3)));
-    G3D_DISPATCH_N(c.ny, NY, ss_cols<NY>(c, T3, out3, 0.0, 1, 0));
+    G3D_DISPATCH_N(c.ny, NY, ss_cols<NY>(c, T3, out3));
 }
 
 // exclusive running sum of P.cflag[0 .. n] into P.coff (n + 1 entries); returns the total (a synchronisation)
@@ -1534,8 +1514,8 @@ void launch_slice_prologue(Ctx& c, int n, int pred_m, int copy_in, int backup) {
     PlasmaState& P = *c.pl;
     const long o = long(n - c.a) * c.nkh;
     const int tok = c.prof_begin("slice_prologue");
-    k_slice_prologue<cpx><<<ew_blocks(c.nkh), 256, 0, c.stream>>>(P.ptrs(c), P.jsin.p, P.jsi0.p, P.bk.p, c.Rx.p, c.Ry.p,
-                                                                      c.Ez.p, c.Bz.p, o, pred_m, copy_in, backup);
+    k_slice_prologue<<<ew_blocks(c.nkh), 256, 0, c.stream>>>(P.ptrs(c), P.jsin.p, P.jsi0.p, P.bk.p, c.Rx.p, c.Ry.p,
+                                                             c.Ez.p, c.Bz.p, o, pred_m, copy_in, backup);
     c.check_launch("k_slice_prologue");
     c.prof_end(tok);
 }
@@ -1544,17 +1524,17 @@ void launch_pass_prologue(Ctx& c, int n, int restore) {
     const long o = long(n - c.a) * c.nkh, nj = 3 * long(c.nk);
     const int tok = c.prof_begin("pass_prologue");
     if (c.f32s)                       // free-hand y, mixed: FP64 spectra, FP32 streaming planes
-        k_pass_prologue<cpx, float><<<ew_blocks(nj), 256, 0, c.stream>>>(P.bk.p, c.Rx.p, c.Ry.p, c.Ez.p, c.Bz.p, o, c.nkh,
-                                                                         P.jsrf.p, nj, P.bcnt.p, restore);
+        k_pass_prologue<float><<<ew_blocks(nj), 256, 0, c.stream>>>(P.bk.p, c.Rx.p, c.Ry.p, c.Ez.p, c.Bz.p, o, c.nkh,
+                                                                    P.jsrf.p, nj, P.bcnt.p, restore);
     else
-        k_pass_prologue<cpx, double><<<ew_blocks(nj), 256, 0, c.stream>>>(P.bk.p, c.Rx.p, c.Ry.p, c.Ez.p, c.Bz.p, o, c.nkh,
-                                                                          P.jsr.p, nj, P.bcnt.p, restore);
+        k_pass_prologue<double><<<ew_blocks(nj), 256, 0, c.stream>>>(P.bk.p, c.Rx.p, c.Ry.p, c.Ez.p, c.Bz.p, o, c.nkh,
+                                                                     P.jsr.p, nj, P.bcnt.p, restore);
     c.check_launch("k_pass_prologue");
     c.prof_end(tok);
 }
 void launch_replace_pred(Ctx& c, int n, int extrap, double w) {
     const int tok = c.prof_begin("replace_pred");
-    k_replace_pred<cpx><<<ew_blocks(c.nkh), 256, 0, c.stream>>>(c.pl->ptrs(c), n, extrap, w);
+    k_replace_pred<<<ew_blocks(c.nkh), 256, 0, c.stream>>>(c.pl->ptrs(c), n, extrap, w);
     c.check_launch("k_replace_pred");
     c.prof_end(tok);
 }
@@ -1567,8 +1547,8 @@ void launch_correct_prologue(Ctx& c, int n, double q, int own, int pred_m, int b
     PlasmaState& P = *c.pl;
     const long o = long(n - 1 - c.a) * c.nkh;
     const int tok = c.prof_begin("correct_prologue");
-    k_correct_prologue<cpx><<<ew_blocks(c.nkh), 256, 0, c.stream>>>(P.ptrs(c), c.Rx.p, c.Ry.p, n, q, own, P.jsin.p, P.jsi0.p, P.bk.p,
-                                                                        c.Ez.p, c.Bz.p, o, pred_m, backup);
+    k_correct_prologue<<<ew_blocks(c.nkh), 256, 0, c.stream>>>(P.ptrs(c), c.Rx.p, c.Ry.p, n, q, own, P.jsin.p, P.jsi0.p, P.bk.p,
+                                                               c.Ez.p, c.Bz.p, o, pred_m, backup);
     c.check_launch("k_correct_prologue");
     c.prof_end(tok);
 }
