@@ -56,14 +56,17 @@ def test_step_at_every_transform_length(nx, ny, nz, precision):
         s.close()
 
 
-@pytest.mark.parametrize("zeta_filter", [0, 1])
-def test_push_through_many_cells_and_slices(zeta_filter):
+@pytest.mark.parametrize("zeta_filter,graded", [(0, False), (1, False), (1, True)])
+def test_push_through_many_cells_and_slices(zeta_filter, graded):
     """Slow particles over long steps: every sub-step starts in another cell or half-cell than the one before, so the
-    stencil held in shared memory has to be loaded anew, and some particles leave the window."""
+    stencil held in shared memory has to be loaded anew, and some particles leave the window. On a graded axis the held
+    half-cell is also what locates them."""
     from g3d import configs
     cfg = configs.config1(nx=32, ny=16, nzeta=24, nmacro=5000, steps=1)
     cfg.bunches[0].update(gamma=4.0, emitx=2.0, emity=2.0, sigz=8.0, zeta_center=20.0)
     cfg.params.update(dz=12.0, dz_push=0.7, zeta_filter=zeta_filter)
+    if graded:
+        configs.on_graded_zeta(cfg)
     s, o = run(cfg, steps=2)
     try:
         p, q = s.host_particles(), o.host_particles()
