@@ -161,3 +161,29 @@ def test_mixed_form_free_hand_plasma_error_table():
     assert table["F"] <= TOL_FIELD
     for f in ["x", "y", "px", "py", "pz"]:
         assert table["plasma " + f] <= 1e-5, (f, table["plasma " + f])
+
+
+@pytest.mark.parametrize("walls", [False, True], ids=["fourier", "walls"])
+@pytest.mark.parametrize("wave,element", [(True, False), (False, True), (True, True)])
+def test_mixed_form_plasma_with_wave_and_external_element(wave, element, walls):
+    """Streaming plasma under the analytic wave, in a solenoid and in both: variants of the streaming push of their own, with
+    FP64 weights in the gather of the FP32 fields (tests/test_stream_mid.py); their distance from the FP64 form, 2 s-steps."""
+    from g3d import configs
+    cfg = configs.lwfa_small(extrapolate=1, passes=2, steps=2)
+    plain = run_plasma(configs.on_freehand_y(cfg) if walls else cfg, "fp64", 2)
+    if wave:
+        cfg.params.update(laser_on=1, a0=0.3, theta=0.02, tau=6.0, laser_envelope=0)
+    if element:
+        cfg.undulators, cfg.magnets = [], [dict(kind=2, z0=-50.0, z1=50.0, g=0.05, R=1e3, ramp=0.0, dsmax=1.0)]
+    a = run_plasma(cfg, "fp64", 2)
+    b = run_plasma(cfg, "mixed", 2)
+    assert rel_l2(a["strm"]["px"], plain["strm"]["px"]) > 1e-3             # the wave and the element act on the plasma
+    assert len(b["strm"]) == len(a["strm"]) and b["np"] == a["np"]
+    table = {n: rel_l2(b[n], a[n]) for n in ["F"]}
+    table["state"] = stacked_error(b, a, FIELDS)
+    for f in ["x", "y", "px", "py", "pz"]:
+        table["plasma " + f] = rel_l2(b["strm"][f], a["strm"][f])
+    print(f"mixed vs FP64, plasma (wave {wave}, element {element}, walls {walls}):", {k: f"{v:.2e}" for k, v in table.items()})
+    assert table["state"] <= TOL_FIELD and table["F"] <= TOL_FIELD
+    for f in ["x", "y", "px", "py", "pz"]:
+        assert table["plasma " + f] <= 1e-5, (f, table["plasma " + f])
