@@ -124,9 +124,10 @@ def algorithmic_bytes(name, cfg, mixed=False, S=0):
     move. P = beam particles: the push reads x, y, zeta, px, py, pz, z, w (64 B) and writes 48 B (both forms);
     the deposit reads 56 B.
     The per-half-cell kernels of the plasma march work on one slice: nk = nx ny points, nkh = ny (nx/2 + 1) modes,
-    S = streaming particles, each read (80 B) and written (64 B) once per half-cell pass (the per-unit figure of
-    the streaming push), with the midpoint fields it gathers from (6 doubles or 8 floats per point) and the three
-    deposit planes."""
+    S = streaming particles, each read (ten doubles and two ints, 88 B) in every pass of a half-cell and written (seven
+    doubles, 56 B) in its last one, with the midpoint fields it gathers from (6 doubles or 8 floats per point) and the
+    three deposit planes. A launch that differs between the passes counts their mean. On the free-hand y grid the mixed
+    form's FP32 parts are the streaming current and the midpoint fields alone."""
     ns = cfg.nzeta - 1
     nk = cfg.nx * cfg.ny
     G = ns * nk
@@ -134,24 +135,30 @@ def algorithmic_bytes(name, cfg, mixed=False, S=0):
     Gc = (ns + 1) * cfg.ny * (cfg.nx // 2 + 1)      # current planes carry one more half-cell
     P = cfg.particles
     nkh = cfg.ny * (cfg.nx // 2 + 1)
-    cz = 8 if mixed else 16                          # bytes of a stored spectrum value other than R
-    cr = 4 if mixed else 8                           # bytes of a raw current value
+    cr = 4 if mixed else 8                           # bytes of a streaming current value
     fm = 32 if mixed else 48                         # bytes of the midpoint fields per point
+    fourier = cfg.ynode is None
+    mixed = mixed and fourier
+    cz = 8 if mixed else 16                          # bytes of a stored spectrum value other than R
+    plasma_cfg = dict({"iterations": 2, "predictor_extrapolate": 1}, **(cfg.plasma or {}))
+    passes = max(1, int(plasma_cfg["iterations"]))
+    ext = 1 if plasma_cfg["predictor_extrapolate"] else 0
+    # k_pass_cols, per mode: the half rows, R, E_z, B_z of slice n, all six of slice n + 1, j0 (2 half-cells), jk (3 + 2),
+    # js0 (2) and, extrapolating, js0 and dl (2 + 2) read, six field columns written; in the last pass pin (2; and js0
+    # without extrapolation) read, the slice, R of slice n + 1, jk (2), js0 (3), dl and pin (2 + 2) written
+    pass_cols = 48 + (2 + 2 + 2) * 16 + ext * 64 + 15 * cz + 6 * cz
+    pass_cols_last = 32 + (1 - ext) * 32 + 64 + 4 * cz + 2 * cz + 48 + 64
     march_slice = (4 * 16 + 10 * cz + 6 * cz) * nkh + (2 * 16 + 4 * cz) * nkh
     # jsn, sin, js0 (2), dl, pin read; jk (2 half-cells) read and written; sin, pin written (3 components each)
     replace_pred = (6 * 48 + 2 * 3 * cz) * nkh + (2 * 3 * cz + 2 * 48) * nkh
     slice_prologue = (48 + 96 + 48 + 2 * 3 * cz + 48 + 32 + 2 * cz + 64) * nkh
     correct = (48 + 32 + 32 + 48 + 32 + 48 + 48) * nkh  # jsn, si0, R, js0 read; R, dl, js0 written
     plasma = {
-        "stream": 144 * S + fm * nk + 3 * cr * nk,
+        "stream": 88 * S + 56 * S // passes + fm * nk + 3 * cr * nk,
         # Fourier y: the rows alone: the deposit planes read and cleared (FP32: (jx, jy, jz, 0) per point), three
-        # complex128 half rows written
-        "stream_spectra": 2 * (16 if mixed else 24) * nk + 48 * nkh,
-        # the fused column work of a pass: the half rows read, jsn written, the replace and march of the slice
-        # (less its read of jsn), the six column transforms of the slice's fields written (their inputs stay in
-        # shared memory); the correction and the next half-cell's prologue on the last of a half-cell's passes
-        "pass_cols": 48 * nkh + 48 * nkh + replace_pred + march_slice - 48 * nkh + 6 * cz * nkh
-        + (correct + slice_prologue) // max(1, int((cfg.plasma or {}).get("iterations", 1))),
+        # complex128 half rows written; free-hand y: the lines' filters too
+        "stream_spectra": (2 * (16 if mixed else 24) * nk if fourier else 6 * cr * nk + 96 * nkh) + 48 * nkh,
+        "pass_cols": (pass_cols + pass_cols_last // passes) * nkh,
         "march_slice": march_slice,
         "real_cols_slice": (2 * 16 + 4 * cz + 6 * cz) * nkh,
         # six column transforms read, F written; the other F plane read and the midpoint fields written
