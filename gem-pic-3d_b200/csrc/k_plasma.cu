@@ -662,7 +662,7 @@ __device__ __forceinline__ void sdeposit_warp_fh(const StreamArgs& c, const DepR
 constexpr int ST_NT = 128;
 // Resident CTAs per SM the register budget of the plain variant is sized for, by form: the mixed form 6 (80 registers; 38.6 us
 // per launch against 41.8 at 5), the FP64 form 5 (96 registers; 57.5 us against 58.1 at 4), the events' ~5 us included
-// (256 x 256 laser-plasma case, 540,000 particles, all builds in one call).
+// (256 x 256 laser-plasma case, 540,000 particles, all builds in one call; with gamma_root since 38.9 and 58.9 us on another box).
 // What bounds the push is latency and instructions, not bytes: a warp's chain is the particle state, the gather, two Boris
 // pushes and the deposit, at 20 to 24 resident warps. So the code on that chain is kept short: one root and one quotient
 // where a textbook form has two or three of each, no integer remainder, no product formed twice, the deposit handed on
@@ -925,8 +925,9 @@ __global__ void k_front(PlasmaPtrs p, Geo g, cpx* __restrict__ Rx, cpx* __restri
 // what is left now, and one launch more.
 // Bound by latency (one CTA of NY threads per SM): the loads of 34 values a thread, whose 16-byte (8-byte) accesses use
 // half (a quarter) of a 32-byte sector, then two transforms and the march one after the other. The transforms run on
-// FftShape<NY>::T threads a line, each line in one warp, with the twiddles in shared memory; the three current lines on
-// three of them, the six field lines on six (two lines each where a column has too few threads). Per launch with the
+// FftShape<NY>::T threads a line, with the twiddles in shared memory: a line lies in one warp and its passes meet at warp
+// barriers, but for NY = 512 (64 threads a line, barriers of the CTA); the three current lines on three such groups, the six field
+// lines on six (two lines each where a column has too few threads). Per launch with the
 // events' ~5 us: 256 x 256 mixed 19.5 -> 15.7 us, FP64 20.5 -> 15.6 us, 64 x 64 FP64 11.6 -> 8.4 us; the correction's
 // launch, 8.5 to 9.6 us per half-cell, is gone.
 template <int NY, class T, class WT, bool LAST>
@@ -1268,8 +1269,9 @@ void launch_stream(Ctx& c, const StreamArgs& a) {
     PlasmaState& P = *c.pl;
     if (P.s.cap <= 0) return;
     const int tok = c.prof_begin("stream");
-    const unsigned blocks = 148 * 16;             // fixed (the kernel strides over the count on the device), so
-                                                  // that the graph of the slice loop does not depend on the list
+    const unsigned blocks = 148 * 16;             // fixed: the kernel strides over the count on the device, which freed
+                                                  // electrons raise in the march, and a graph of the slice loop
+                                                  // (GRAPH_POINTS_*) must not depend on the list
     if (c.f32s) stream_launch<true>(c, a, blocks);
     else stream_launch<false>(c, a, blocks);
     c.check_launch("k_stream");
